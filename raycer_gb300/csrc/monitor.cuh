@@ -97,11 +97,13 @@ static __device__ __noinline__ int poll_render(RenderMonitor* mon, unsigned long
 // polls (then it just stops watching). The other warps' work loop carries no poll at all.
 // publish: kPublishNone, kPublishProgress, or kPublishEstimate (the pixels of
 // the items taken before those the other warps may hold, at most `pixels`).
+// finished: where an item is long (a whole path), the count of warps that
+// have left the kernel's loop; the watch then goes on until all have.
 constexpr unsigned kWatchPolls = 1u << 24;
 
 static __device__ __forceinline__ void watch_queue(RenderMonitor* mon, unsigned long long budgetNs, DevControl* ctl,
                                          unsigned* head, unsigned long long items, unsigned long long publish,
-                                         unsigned long long pixels)
+                                         unsigned long long pixels, const unsigned* finished = nullptr)
 {
     if ((threadIdx.x & 31u) != 0u)
         return;
@@ -118,7 +120,8 @@ static __device__ __forceinline__ void watch_queue(RenderMonitor* mon, unsigned 
         }
         // polled once before the head is looked at: a kernel whose items
         // were all taken at once is still checked (a budget of 0 stops it)
-        if (poll_render(mon, budgetNs, ctl, head, true, pub) || h >= items)
+        if (poll_render(mon, budgetNs, ctl, head, true, pub) ||
+            (h >= items && (!finished || *reinterpret_cast<const volatile unsigned*>(finished) >= workers)))
             return;
         __nanosleep(2000);
     }

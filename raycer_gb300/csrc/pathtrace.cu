@@ -28,6 +28,7 @@
 // Queue counts live on the device, so a pass is a fixed launch sequence the
 // host never waits on (and can be captured in a CUDA graph).
 
+#include <algorithm>
 #include <cfloat>
 #include <cstdlib>
 
@@ -501,13 +502,22 @@ __device__ __forceinline__ void nrc_end(const NrcPass& n, uint32_t g, float r, f
 // terminal radiance, and other paths end at the hit of segment termSegment
 // with a cache lookup (res gets thr * cache after the last segment).
 // Returns whether the path goes on (the slot joins the next segment's
-// queue); a cache lookup sets `lookup` and `lrec`. With OD the caller passes
-// the slot's ray (o, d) it already holds, else they are read from the path
-// state.
-template <bool NRC, bool OD>
-__device__ __forceinline__ bool shade_slot(const PassParams& p, int segment, int s, int4 h, float4 o, float4 d,
+// queue); a cache lookup sets `lookup` and `lrec`. RAY says where the slot's
+// ray is: kRayInMemory reads it from the path state and stores the next one
+// there, kRayPassed takes (o, d) from the caller and stores the next one,
+// kRayKept takes it and returns the next one in (o, d).
+enum ShadeRay
+{
+    kRayInMemory,
+    kRayPassed,
+    kRayKept
+};
+
+template <bool NRC, int RAY>
+__device__ __forceinline__ bool shade_slot(const PassParams& p, int segment, int s, int4 h, float4& o, float4& d,
                                            bool& lookup, NrcRecord& lrec)
 {
+    constexpr bool OD = RAY != kRayInMemory;
     bool cont = false;
     // a one-scene pass has one chunk: no dependent load of the slot's chunk
     const PathChunk& ch = p.chunks[p.singleScene && p.numChunks == 1 ? 0 : p.chunkOf[s]];
@@ -620,10 +630,6 @@ __device__ __forceinline__ bool shade_slot(const PassParams& p, int segment, int
                     thr.y = __fmul_rn(thr.y, fg);
                     thr.z = __fmul_rn(thr.z, fb);
                 }
-                V3 no = vfma(dir, scn.rayStartOffset, ip);
-                p.o[s] = make_float4(no.x, no.y, no.z, __int_as_float(h.x));
-                p.d[s] = make_float4(dir.x, dir.y, dir.z, __int_as_float(inst));
-                p.thr[s] = thr;
                 cont = true;
                 if (train)
                 {
@@ -632,6 +638,20 @@ __device__ __forceinline__ bool shade_slot(const PassParams& p, int segment, int
                     if (dielectric)
                         rec.c.y = -1.0f;
                     p.nrc.vtx[size_t(segment) * size_t(p.nrc.groups) + g] = rec;
+                }
+                V3 no = vfma(dir, scn.rayStartOffset, ip);
+                const float4 o2 = make_float4(no.x, no.y, no.z, __int_as_float(h.x));
+                const float4 d2 = make_float4(dir.x, dir.y, dir.z, __int_as_float(inst));
+                p.thr[s] = thr;
+                if (RAY == kRayKept)
+                {
+                    o = o2;
+                    d = d2;
+                }
+                else
+                {
+                    p.o[s] = o2;
+                    p.d[s] = d2;
                 }
             }
             else if (train)
@@ -716,8 +736,8 @@ __global__ void __launch_bounds__(BLOCK) k_shade(PassParams p, int segment)
         if (q < total)
         {
             s = qin[q];
-            cont = shade_slot<NRC, false>(p, segment, s, p.hit[s], make_float4(0.0f, 0.0f, 0.0f, 0.0f),
-                                          make_float4(0.0f, 0.0f, 0.0f, 0.0f), lookup, lrec);
+            float4 o, d;  // read from the path state where they are needed
+            cont = shade_slot<NRC, kRayInMemory>(p, segment, s, p.hit[s], o, d, lookup, lrec);
         }
         enqueue_continuing(cont, s, outCount, qout);
         if (NRC)
@@ -766,13 +786,13 @@ __global__ void __launch_bounds__(BLOCK,
         {
             s = queue[q];
             const DevScene sc = scene_of_slot(p, s);
-            const float4 o = p.o[s];
-            const float4 d = p.d[s];
+            float4 o = p.o[s];
+            float4 d = p.d[s];
             RayF ray = make_ray(v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), 0.0f, FLT_MAX);
             HitF h{ -1, FLT_MAX, 0.0f, 0.0f, -1 };
             const bool found = traverse_wide(sc, ray, h, err, __float_as_int(o.w));
             done++;
-            cont = shade_slot<NRC, true>(p, segment, s, make_int4(found ? h.slot : -1, __float_as_int(h.t), 0, -1),
+            cont = shade_slot<NRC, kRayPassed>(p, segment, s, make_int4(found ? h.slot : -1, __float_as_int(h.t), 0, -1),
                                          o, d, lookup, lrec);
         }
         enqueue_continuing(cont, s, outCount, qout);
@@ -780,6 +800,93 @@ __global__ void __launch_bounds__(BLOCK,
             enqueue_lookup(lookup, lrec, p);
     }
     flush_extend_counts(p, done, TravCount{ 0, 0 }, err);
+}
+
+// Every segment from `first` on in one kernel: a lane takes a path from the
+// queue of segment `first` and traces and shades it, segment after segment
+// with its ray in registers, until the path ends; before each segment the
+// lanes whose path has ended take new ones (one atomic per warp). A launch
+// lasts as long as its longest warp, and one launch per segment paid that
+// tail once per segment (160-200 us for each of the nine segments that only
+// the training paths of a 5M-triangle cache frame reach); here the walks of
+// all segments overlap and the tail is paid once per pass. Frames, render
+// and image: that cache frame 6.21 -> 5.35 ms, the 1080p heightfield of depth
+// 4 1.879 -> 1.780 ms, a 64x48 preview 294 -> 179 us; the room at 16 samples
+// per pixel and dense rooms, whose segments are long, are level. The camera
+// rays keep their own launch: walked in the same warps as bounce rays they
+// lose their coherence (room 2.53 -> 2.71 ms, heightfield 1.78 -> 1.85 ms).
+template <int BLOCK, bool NRC>
+__global__ void __launch_bounds__(BLOCK,
+                                  ((NRC ? RC_EXTEND_SHADE_NRC_MIN_BLOCKS : RC_EXTEND_WIDE_MIN_BLOCKS) * 128) / BLOCK)
+    k_bounce_paths(PassParams p, int first)
+{
+    const unsigned total = *reinterpret_cast<volatile unsigned*>(&p.counts[first * 4 + 0]);
+    const int* __restrict__ queue = (first & 1) ? p.qb : p.qa;
+    unsigned* head = &p.counts[first * 4 + 1];
+    unsigned* finished = &p.counts[first * 4 + 2];  // warps that have no more work
+    if (pass_stopped(p))
+        return;
+    if (is_watch_warp(p.monitor, p.budgetNs))
+    {
+        watch_queue(p.monitor, p.budgetNs, p.ctl, head, total, kPublishProgress, 0, finished);
+        return;
+    }
+    const bool watched = monitored(p.monitor, p.budgetNs);
+    // Lanes of this warp that take paths: all of them, or fewer where the
+    // queue would leave other warps without work.
+    const unsigned warps = gridDim.x * (BLOCK / 32);
+    const unsigned quota = min(32u, (total + warps - 1u) / warps);
+    int err = 0;
+    unsigned long long done = 0;
+    bool drained = total == 0u;  // warp-uniform
+    int s = -1;                  // this lane's path, -1 = none
+    int seg = first;
+    float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f), d = o;
+    while (true)
+    {
+        const unsigned idle = __ballot_sync(0xffffffffu, s < 0 && lane_id() < quota);
+        if (idle && !drained)
+        {
+            const unsigned n = unsigned(__popc(idle));
+            const unsigned base = warp_fetch(head, n);
+            drained = base + n >= total;
+            if ((idle >> lane_id()) & 1u)
+            {
+                const unsigned q = base + unsigned(__popc(idle & ((1u << lane_id()) - 1u)));
+                if (q < total)
+                {
+                    s = queue[q];
+                    o = p.o[s];
+                    d = p.d[s];
+                    seg = first;
+                }
+            }
+        }
+        // one decision per warp (lane 0's view of the stop bit)
+        const bool stop = watched && __shfl_sync(0xffffffffu, int(render_stopped(p.ctl)), 0) != 0;
+        if (stop || __ballot_sync(0xffffffffu, s >= 0) == 0u)
+            break;
+        bool lookup = false;
+        NrcRecord lrec;
+        if (s >= 0)
+        {
+            const DevScene sc = scene_of_slot(p, s);
+            RayF ray = make_ray(v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), 0.0f, FLT_MAX);
+            HitF h{ -1, FLT_MAX, 0.0f, 0.0f, -1 };
+            const bool found = traverse_wide(sc, ray, h, err, __float_as_int(o.w));
+            done++;
+            const bool cont = shade_slot<NRC, kRayKept>(
+                p, seg, s, make_int4(found ? h.slot : -1, __float_as_int(h.t), 0, -1), o, d, lookup, lrec);
+            seg++;
+            if (!cont)
+                s = -1;
+        }
+        if (NRC)
+            enqueue_lookup(lookup, lrec, p);
+    }
+    flush_extend_counts(p, done, TravCount{ 0, 0 }, err);
+    if (watched && lane_id() == 0)
+        atomicAdd(finished, 1u);
 }
 
 __global__ void __launch_bounds__(256) k_accumulate(PassParams p)
@@ -895,6 +1002,26 @@ cudaError_t extend_shade_b(const PassParams& p, int segment, cudaStream_t stream
     return cudaGetLastError();
 }
 
+template <int BLOCK, bool NRC>
+cudaError_t bounce_paths_b(const PassParams& p, int first, cudaStream_t stream, int numSMs)
+{
+    auto k = k_bounce_paths<BLOCK, NRC>;
+    static OccupancyCache occ;
+    k<<<persistent_blocks(k, BLOCK, numSMs, occ), BLOCK, 0, stream>>>(p, first);
+    return cudaGetLastError();
+}
+
+cudaError_t bounce_paths_t(const PassParams& p, int first, int block, cudaStream_t stream, int numSMs)
+{
+    if (p.nrc.query)
+        return bounce_paths_b<128, true>(p, first, stream, numSMs);
+    if (block == 64)
+        return bounce_paths_b<64, false>(p, first, stream, numSMs);
+    if (block == 256)
+        return bounce_paths_b<256, false>(p, first, stream, numSMs);
+    return bounce_paths_b<128, false>(p, first, stream, numSMs);
+}
+
 // The block sizes of the kernels it replaces: the autotuned extend block for
 // plain passes, 128 threads for cache passes.
 cudaError_t extend_shade_t(const PassParams& p, int segment, int block, cudaStream_t stream, int numSMs)
@@ -982,7 +1109,19 @@ __global__ void __launch_bounds__(256) k_nrc_targets(PassParams p)
     }
 }
 
+// Uncounted nearest-first passes over a 4-wide tree trace and shade in one
+// kernel: one launch for the camera rays, one for all later segments.
+bool fused_pass(const PassParams& p, int order, int counting)
+{
+    return !p.instanced && order == ORDER_NEAREST && !counting && p.wide && !extend_refill() && extend_shade_fused();
+}
+
 }  // namespace
+
+int path_extend_launches(const PassParams& p, int order, int counting)
+{
+    return fused_pass(p, order, counting) ? std::min(p.segments, 2) : p.segments;
+}
 
 cudaError_t launch_path_segments(const PassParams& p, int order, int counting, const PassShape& shape,
                                  cudaStream_t stream, int numSMs, const cudaEvent_t* extendEvents)
@@ -991,16 +1130,17 @@ cudaError_t launch_path_segments(const PassParams& p, int order, int counting, c
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
         return e;
-    // uncounted nearest-first passes over a 4-wide tree: one kernel per segment
-    const bool fused = !p.instanced && order == ORDER_NEAREST && !counting && p.wide && !extend_refill() &&
-                       extend_shade_fused();
-    for (int seg = 0; seg < p.segments; ++seg)
+    const bool fused = fused_pass(p, order, counting);
+    const int launches = path_extend_launches(p, order, counting);
+    for (int seg = 0; seg < launches; ++seg)
     {
         if (extendEvents && (e = cudaEventRecord(extendEvents[2 * seg], stream)) != cudaSuccess)
             return e;
         if (fused)
         {
-            if ((e = extend_shade_t(p, seg, shape.extendBlock, stream, numSMs)) != cudaSuccess)
+            e = seg == 0 ? extend_shade_t(p, seg, shape.extendBlock, stream, numSMs)
+                         : bounce_paths_t(p, seg, shape.extendBlock, stream, numSMs);
+            if (e != cudaSuccess)
                 return e;
             if (extendEvents && (e = cudaEventRecord(extendEvents[2 * seg + 1], stream)) != cudaSuccess)
                 return e;

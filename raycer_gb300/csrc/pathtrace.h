@@ -123,8 +123,11 @@ struct PassShape
     int shadeBlock = 128;
 };
 
-// Launch the kernels of one pass (generate, segments x (extend, shade),
-// accumulate) on `stream`. extendEvents: 2 * segments events recorded around
+// Extend launches of a pass: one per segment, or, where extend and shade run
+// as one kernel, one for the camera rays and one for all later segments.
+int path_extend_launches(const PassParams& p, int order, int counting);
+// Launch the kernels of one pass (generate, the segments, accumulate) on
+// `stream`. extendEvents: 2 * path_extend_launches() events recorded around
 // each extend launch, or nullptr. Graph-capturable (no host reads).
 cudaError_t launch_path_pass(const PassParams& p, int order, int counting, const PassShape& shape,
                              cudaStream_t stream, int numSMs, const cudaEvent_t* extendEvents);

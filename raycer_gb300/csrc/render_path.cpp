@@ -263,16 +263,6 @@ rc_status render_path(rc_tracer* h, uint64_t pixelStart, uint64_t count, RenderW
     const PathScene* dScene = static_cast<const PathScene*>(h->dTables);
     const PathChunk* dChunks = reinterpret_cast<const PathChunk*>(static_cast<char*>(h->dTables) + sizeof(PathScene));
 
-    // Events around every extend launch of every pass (stage 0 timing).
-    const size_t needEvents = size_t(passes) * size_t(2 * std::max(g.max_path_length, 0));
-    const bool timeStages = needEvents <= 4096;
-    while (timeStages && h->evPool.size() < needEvents)
-    {
-        cudaEvent_t e;
-        RC_CUDA_TRY(h, cudaEventCreate(&e), "create event");
-        h->evPool.push_back(e);
-    }
-
     PassParams pp = pass_params(h->dPath, h->pathSlots, h->dCounts, h->dCtl);
     pp.scenes = dScene;
     pp.numChunks = 1;
@@ -285,6 +275,16 @@ rc_status render_path(rc_tracer* h, uint64_t pixelStart, uint64_t count, RenderW
     {
         pp.monitor = watch->dev;
         pp.budgetNs = watch->budgetNs;
+    }
+    // Events around every extend launch of every pass (stage 0 timing).
+    const size_t passEvents = size_t(2 * path_extend_launches(pp, h->order, h->counting));
+    const size_t needEvents = size_t(passes) * passEvents;
+    const bool timeStages = needEvents <= 4096;
+    while (timeStages && h->evPool.size() < needEvents)
+    {
+        cudaEvent_t e;
+        RC_CUDA_TRY(h, cudaEventCreate(&e), "create event");
+        h->evPool.push_back(e);
     }
     PassShape shape;
     const bool nrc = nrc_active(h);
@@ -317,7 +317,7 @@ rc_status render_path(rc_tracer* h, uint64_t pixelStart, uint64_t count, RenderW
         pp.npixels = int(chunks[pass].pixels);
         pp.nslots = int(uint64_t(chunks[pass].pixels) * spp);
         RC_CUDA_TRY(h, cudaMemsetAsync(h->dCounts, 0, countsBytes, h->stream), "reset queue counters");
-        const cudaEvent_t* ev = timeStages ? h->evPool.data() + pass * size_t(2 * g.max_path_length) : nullptr;
+        const cudaEvent_t* ev = timeStages ? h->evPool.data() + pass * passEvents : nullptr;
         if (!nrc)
         {
             RC_CUDA_TRY(h, launch_path_pass(pp, h->order, h->counting, shape, h->stream, h->numSMs, ev),
