@@ -137,7 +137,7 @@ struct DevScene
     int rootLink;  // >= 0: inner node 0; < 0: the root is a leaf (~leaf code)
     int numTris;
     int numMats;
-    int pad;
+    int depth;     // levels of the BVH (a depth-first walk stacks no more entries)
     const DevNode* tlas;
     const DevInstance* instances;
     int tlasRoot;

@@ -110,7 +110,7 @@ extern "C" rc_status rc_cast_with_shadow_device_noalloc(rc_tracer* h, const rc_r
     sc.rootLink = h->rootLink;
     sc.numTris = int(h->nTris);
     sc.numMats = int(h->nMats);
-    sc.pad = 0;
+    sc.depth = int(h->bvhDepth);
     sc.ropes = h->dRopes;  // built by an earlier call, if any (nothing is allocated here)
     sc.ropeCount = int(h->ropeCount);
     rcx::DevCamera cam{};

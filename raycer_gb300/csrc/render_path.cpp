@@ -154,6 +154,7 @@ PathScene path_scene(const rc_tracer* h, uint64_t pixelStart)
     ps.sc.rootLink = h->rootLink;
     ps.sc.numTris = int(h->nTris);
     ps.sc.numMats = int(h->nMats);
+    ps.sc.depth = int(h->bvhDepth);
     ps.sc.tlas = h->dTlas;
     ps.sc.instances = h->dInstances;
     ps.sc.tlasRoot = h->tlasRoot;

@@ -374,12 +374,164 @@ __global__ void __launch_bounds__(kBlock, RC_TRACE_MIN_BLOCKS) k_raycast_shadow(
     flush_counts(ctl, 1, done, cnt, err);
 }
 
+// The same queries and frames with a group of G lanes per ray (traverse_group),
+// for calls with few rays; 32 / G rays per warp fetch. What bounds them is the
+// rounds of dependent fetches of the longest ray, about a twentieth of its
+// node count. 8 blocks of 16 KB of stacks leave the SM half its L1. 777 random
+// rays in 1M triangles 131 -> 26 us, 100,000 215 -> 170 us; RAY frames of 260k
+// triangles at 160x90 226 -> 58 us, at 320x180 199 -> 101 us, in the
+// reference's order 791 -> 60 and 482 -> 124 us.
+template <bool ANY, int ORDER>
+__global__ void __launch_bounds__(kBlock, 8) k_cast_group(DevScene sc, const rc_ray* __restrict__ rays, int n,
+                                                       rc_hit* __restrict__ hits, DevControl* ctl, unsigned G,
+                                                       int reserve)
+{
+    __shared__ int2 stacks[kWarpsPerBlock][kGroupEntries];
+    const unsigned take = 32u / G;
+    const unsigned group = lane_id() / G;
+    const int capacity = kGroupEntries / int(take);
+    int2* stack = stacks[threadIdx.x >> 5] + int(group) * capacity;
+    unsigned long long done = 0;
+    while (true)
+    {
+        const unsigned base = warp_fetch(&ctl->head[0], take);
+        if (base >= unsigned(n))
+            break;
+        const bool active = base + group < unsigned(n);
+        const int i = active ? int(base + group) : int(base);
+        const float4* rp = reinterpret_cast<const float4*>(rays + i);
+        const float4 r0 = __ldg(rp);
+        const float4 r1 = __ldg(rp + 1);
+        const RayF ray = make_ray(v3(r0.x, r0.y, r0.z), v3(r1.x, r1.y, r1.z), r0.w, r1.w);
+        HitF h{ -1, FLT_MAX, 0.0f, 0.0f, -1 };
+        const bool found = traverse_group<ANY, ORDER>(sc, ray, h, -1, active, G, stack, capacity, reserve);
+        if (active && lane_id() % G == 0)
+        {
+            int4 out;
+            out.x = found ? caller_index(sc, h.slot) : -1;
+            out.y = __float_as_int(found ? h.t : -1.0f);
+            out.z = __float_as_int(found ? h.u : 0.0f);
+            out.w = __float_as_int(found ? h.v : 0.0f);
+            reinterpret_cast<int4*>(hits)[i] = out;
+            done++;
+        }
+    }
+    flush_counts(ctl, 0, done, TravCount{ 0, 0 }, 0);
+}
+
+// The one-kernel RAY frame (primary ray, then the hit's shadow ray).
+template <int ORDER>
+__global__ void __launch_bounds__(kBlock, 8) k_raycast_group(DevScene sc, DevCamera cam, const rc_ray* __restrict__ rays,
+                                                          uint64_t pixelStart, int64_t count, int64_t width,
+                                                          int64_t height, int64_t tilesX, int castShadow,
+                                                          rc_cast_pixel* __restrict__ out, DevControl* ctl, float3 L,
+                                                          float rayStartOffset, unsigned G, int reserve)
+{
+    __shared__ int2 stacks[kWarpsPerBlock][kGroupEntries];
+    const unsigned take = 32u / G;
+    const unsigned group = lane_id() / G;
+    const int capacity = kGroupEntries / int(take);
+    int2* stack = stacks[threadIdx.x >> 5] + int(group) * capacity;
+    unsigned long long done = 0, done1 = 0;
+    const int64_t items = tilesX > 0 ? tilesX * ((height + 3) / 4) * 32 : count;
+    if (is_watch_warp(sc.monitor, sc.budgetNs))
+    {
+        watch_queue(sc.monitor, sc.budgetNs, ctl, &ctl->head[0], static_cast<unsigned long long>(items),
+                    kPublishEstimate, static_cast<unsigned long long>(count));
+        return;
+    }
+    while (true)
+    {
+        const unsigned base = warp_fetch(&ctl->head[0], take);
+        if (int64_t(base) >= items)
+            break;
+        int64_t i = int64_t(base) + group;
+        bool valid = i < items;
+        if (tilesX > 0 && valid)
+        {
+            const int64_t tile = i >> 5;
+            const int64_t px = (tile % tilesX) * 8 + (i & 7);
+            const int64_t py = (tile / tilesX) * 4 + ((i >> 3) & 3);
+            valid = px < width && py < height;
+            i = py * width + px;
+        }
+        const RayF ray = primary_ray(cam, rays, valid ? pixelStart + uint64_t(i) : pixelStart, valid ? i : 0, width);
+        HitF h{ -1, FLT_MAX, 0.0f, 0.0f, -1 };
+        const bool found = traverse_group<false, ORDER>(sc, ray, h, -1, valid, G, stack, capacity, reserve);
+        int4 o;
+        o.x = found ? caller_index(sc, h.slot) : -1;
+        o.y = __float_as_int(found ? h.t : -1.0f);
+        o.z = -1;
+        o.w = found ? 1 : 0;
+        if (castShadow)
+        {
+            // shadow_of's ray
+            const V3 dl = v3(L.x, L.y, L.z);
+            const RayF sr = make_ray(vfma(dl, rayStartOffset, vfma(ray.d, h.t, ray.o)), dl, 0.0f, FLT_MAX);
+            HitF s{ -1, FLT_MAX, 0.0f, 0.0f, -1 };
+            const bool occ = traverse_group<true, ORDER_REF>(sc, sr, s, h.slot, valid && found, G, stack, capacity, reserve);
+            if (found)
+            {
+                o.z = occ ? caller_index(sc, s.slot) : -1;
+                o.w = 1 | 2 | (occ ? 4 : 0);
+            }
+        }
+        if (valid && lane_id() % G == 0)
+        {
+            reinterpret_cast<int4*>(out)[i] = o;
+            done++;
+            done1 += found && castShadow ? 1 : 0;
+        }
+    }
+    flush_counts(ctl, 0, done, TravCount{ 0, 0 }, 0);
+    flush_counts(ctl, 1, done1, TravCount{ 0, 0 }, 0);
+}
+
 // Persistent grid of a ray kernel: resident blocks per SM (cached per
 // device) x the launching handle's SMs.
 template <typename K>
 int persistent_blocks(K kernel, int numSMs, OccupancyCache& cache)
 {
     return blocks_per_sm(kernel, kBlock, 0, cache) * numSMs;
+}
+
+// Lanes per ray of an uncounted call with n rays on a single-level scene, or 0
+// for one ray per lane: the largest group (32, 16, 8, 4) whose `rounds` rounds
+// of one ray per group cover the rays (twice as many rounds for groups of 4,
+// whose alternative is one ray per lane). Each larger group shortens a ray's
+// chain of fetches but gives the warp fewer rays, so the lines lie where a
+// call stops being bound by latency. Measured (device times; 1M-triangle
+// terrain for casts, 260k for frames; group of 32 / 16 / 8 / 4 / none):
+//   25,000 random rays    80 /  66 /  67 /  91 / 159 us   (lines for 4 rounds)
+//   100,000                - /   - / 146 / 170 / 214 us
+//   400,000                - /   - /   - / 458 / 360 us
+//   160x90 frame          86 /  58 /  60 /   - / 226 us   (2 rounds: a tile's
+//   320x180                - / 150 / 101 / 103 / 199 us    neighbouring rays share
+//   480x270                - /   - / 186 / 153 / 194 us    fetches in a full warp)
+//   640x360                - /   - /   - / 225 / 186 us
+// A tree too deep for the group's stack is walked one ray per lane.
+unsigned group_lanes(const DevScene& sc, int64_t n, int blocks, int rounds)
+{
+    const int64_t lanes = int64_t(blocks) * kBlock;
+    for (unsigned G = 32u; G >= 4u; G /= 2u)
+        if (n * int64_t(G) <= lanes * rounds * (G == 4u ? 2 : 1))
+            return int(G) * kGroupEntries / 32 >= sc.depth + 2 * int(G) ? G : 0u;
+    return 0u;
+}
+
+template <bool ANY, int ORDER>
+cudaError_t cast_group(const LaunchInfo& li, const DevScene& sc, const rc_ray* rays, int64_t n, rc_hit* hits,
+                       DevControl* ctl, bool& taken)
+{
+    auto k = k_cast_group<ANY, ORDER>;
+    static OccupancyCache occ;
+    const int blocks = persistent_blocks(k, li.numSMs, occ);
+    const unsigned G = group_lanes(sc, n, blocks, 4);
+    taken = G != 0u;
+    if (!taken)
+        return cudaSuccess;
+    k<<<blocks, kBlock, 0, li.stream>>>(sc, rays, int(n), hits, ctl, G, sc.depth);
+    return cudaGetLastError();
 }
 
 template <bool ANY, int ORDER, bool COUNT, bool SL = false>
@@ -512,6 +664,25 @@ bool fused_frames()
     return on;
 }
 
+template <int ORDER>
+cudaError_t raycast_group(const LaunchInfo& li, const DevScene& sc, const DevCamera& cam, const rc_ray* rays,
+                          uint64_t pixelStart, int64_t count, int64_t width, int castShadow, float3 L, float off,
+                          rc_cast_pixel* out, DevControl* ctl, bool& taken)
+{
+    auto k = k_raycast_group<ORDER>;
+    static OccupancyCache occ;
+    const int blocks = persistent_blocks(k, li.numSMs, occ);
+    const unsigned G = group_lanes(sc, count, blocks, 2);
+    taken = G != 0u;
+    if (!taken)
+        return cudaSuccess;
+    const int64_t height = width > 0 ? count / width : 0;
+    const int64_t tilesX = whole_frame(pixelStart, count, width) ? (width + 7) / 8 : 0;
+    k<<<blocks, kBlock, 0, li.stream>>>(sc, cam, rays, pixelStart, count, width, height, tilesX, castShadow, out, ctl, L,
+                                        off, G, sc.depth);
+    return cudaGetLastError();
+}
+
 // Uncounted frames: the fused or the two-kernel form.
 template <int ORDER, bool PACKET, bool INST, bool SL = false>
 cudaError_t raycast_u(const LaunchInfo& li, const DevScene& sc, const DevCamera& cam, const rc_ray* rays,
@@ -547,6 +718,16 @@ cudaError_t launch_cast(const LaunchInfo& li, const DevScene& sc, const rc_ray* 
     if (n <= 0)
         return cudaSuccess;
     const bool sl = !li.counting && sc.numInstances == 0 && sc.ropes && stackless_walk();
+    if (!li.counting && sc.numInstances == 0 && !sl)
+    {
+        bool taken = false;
+        const cudaError_t e =
+            anyHit                   ? cast_group<true, ORDER_REF>(li, sc, rays, n, hits, ctl, taken)
+            : order == ORDER_NEAREST ? cast_group<false, ORDER_NEAREST>(li, sc, rays, n, hits, ctl, taken)
+                                     : cast_group<false, ORDER_REF>(li, sc, rays, n, hits, ctl, taken);
+        if (taken)
+            return e;
+    }
     if (anyHit)
         return li.counting ? cast_t<true, ORDER_REF, true>(li, sc, rays, n, hits, ctl)
                : sl        ? cast_t<true, ORDER_REF, false, true>(li, sc, rays, n, hits, ctl)
@@ -579,6 +760,21 @@ cudaError_t launch_raycast(const LaunchInfo& li, const DevScene& sc, const DevCa
     if (li.counting)
         return order == ORDER_NEAREST ? raycast_t<ORDER_NEAREST, true, false, false>(RC_RAYCAST_ARGS)
                                       : raycast_t<ORDER_REF, true, false, false>(RC_RAYCAST_ARGS);
+    if (fused_frames() && !(stackless_walk() && sc.ropes))
+    {
+        bool taken = false;
+        const cudaError_t e =
+            order == ORDER_NEAREST
+                ? raycast_group<ORDER_NEAREST>(li, sc, cam, rays, pixelStart, count, width, castShadow, dirToLight,
+                                               rayStartOffset, out, ctl, taken)
+                : raycast_group<ORDER_REF>(li, sc, cam, rays, pixelStart, count, width, castShadow, dirToLight,
+                                           rayStartOffset, out, ctl, taken);
+        if (taken)
+        {
+            *kernels = 1;
+            return e;
+        }
+    }
     const int packets = trace_packets();
     const bool packet = whole_frame(pixelStart, count, width) && (packets == 2 || (packets == 1 && !rays));
     if (stackless_walk() && sc.ropes)

@@ -438,7 +438,7 @@ DevScene dev_scene(const rc_tracer* h)
     s.rootLink = h->rootLink;
     s.numTris = int(h->nTris);
     s.numMats = int(h->nMats);
-    s.pad = 0;
+    s.depth = int(h->bvhDepth);
     s.tlas = h->dTlas;
     s.instances = h->dInstances;
     s.tlasRoot = h->tlasRoot;

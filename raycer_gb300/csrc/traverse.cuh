@@ -624,6 +624,214 @@ __device__ __forceinline__ bool traverse_packet(const DevScene& sc, const RayF& 
     }
 }
 
+// One ray walked by a group of G lanes (a power of two, 4..32): calls with
+// fewer rays than the GPU has lanes are bound by the latency of one ray's
+// walk, a chain of dependent node fetches (a grazing ray over 1M triangles
+// visits hundreds), while most lanes have no ray. The group's lanes pop up to
+// G entries of one shared stack at a time, so that many nodes and leaves of
+// the ray are in flight together. All 32 lanes of a warp call this together,
+// the lanes of a group with the same ray; `active`: the group has a ray.
+// `stack`: the group's entries (link, entry distance) in shared memory,
+// `capacity` of them. A pop of G entries can push 2 G; once fewer than
+// `reserve` (at least the tree's depth) + G would be left, the group goes on
+// one entry at a time, depth first, which needs no more than the reserve.
+// The result (in every lane of the group) is the one-lane walk's:
+//   any-hit       the reference's first occluder is the one in the smallest
+//                 slot (the reference order meets leaves in slot order);
+//   closest hit   the minimum t, ties to the larger slot, does not depend on
+//                 the order the boxes are met in, with two exceptions, which
+//                 the group's first lane walks again alone. ORDER_REF takes
+//                 every NaN distance it meets (rays or vertices with NaN, or
+//                 so large that products overflow). ORDER_NEAREST skips a box
+//                 entered beyond the current hit, and rounding can put a
+//                 box's entry behind a hit inside it (overlapping coplanar
+//                 triangles): if the winner lies before its own leaf's entry,
+//                 the order may have decided; if not, no walk can have skipped
+//                 it (entries grow downward, hits only come nearer). The
+//                 group itself skips boxes only past kGroupCull times the
+//                 current hit, so that it meets such winners.
+constexpr float kGroupCull = 1.01f;
+
+template <int ORDER>
+static __device__ __noinline__ bool traverse_alone(const DevScene& sc, const RayF& ray, HitF& hit, int skip)
+{
+    TravCount none{ 0, 0 };
+    int err = 0;  // the tree's depth is within the stack (checked at upload)
+    hit = HitF{ -1, FLT_MAX, 0.0f, 0.0f, -1 };
+    return traverse<false, ORDER, false>(sc, ray, hit, none, err, skip);
+}
+
+template <bool ANY_HIT, int ORDER>
+__device__ __forceinline__ bool traverse_group(const DevScene& sc, const RayF& ray, HitF& hit, int skip, bool active,
+                                               unsigned G, int2* __restrict__ stack, int capacity, int reserve)
+{
+    constexpr unsigned kAll = 0xffffffffu;
+    constexpr bool CULL = !ANY_HIT && ORDER == ORDER_NEAREST;
+    const unsigned lane = threadIdx.x & 31u;
+    const unsigned gl = lane & (G - 1u);           // lane within the group
+    const unsigned shift = lane & ~(G - 1u);       // first lane of the group
+    const unsigned gmask = kAll >> (32u - G);      // the group's lanes, shifted down
+    const unsigned below = (1u << gl) - 1u;
+    const int limit = capacity - reserve - int(G); // most entries before a pop of G
+    float cull = __int_as_float(0x7f800000);       // boxes entered beyond this are skipped
+    int count = 0;
+    float he = 0.0f;                               // entry distance of the hit's leaf
+    bool odd = false;                              // reference order: a NaN distance was met
+    bool found = false;
+    if (active)
+    {
+        count = 1;
+        if (gl == 0)
+            stack[0] = make_int2(sc.rootLink, 0);
+    }
+    __syncwarp();
+    while (__ballot_sync(kAll, count > 0))
+    {
+        const int pops = count > limit ? min(count, 1) : min(count, int(G));
+        bool mine = int(gl) < pops;
+        int2 e = make_int2(0, 0);
+        if (mine)
+            e = stack[count - 1 - int(gl)];
+        count -= pops;
+        __syncwarp();  // every lane has read its entry before the pushes below
+        if (CULL && __int_as_float(e.y) > cull)
+            mine = false;
+        bool hNear = false, hFar = false;
+        int nearC = 0, farC = 0;
+        float nearD = 0.0f, farD = 0.0f;
+        bool leafHit = false;
+        if (mine && e.x >= 0)
+        {
+            float4 a, b, c;
+            int4 l;
+            load_node(sc.nodes, e.x, a, b, c, l);
+            float e0, e1;
+            bool h0, h1;
+            if (ray.finite)
+            {
+                h0 = slab_finite(ray, a.x, a.y, a.z, a.w, c.x, c.y, e0);
+                h1 = slab_finite(ray, b.x, b.y, b.z, b.w, c.z, c.w, e1);
+            }
+            else
+            {
+                h0 = slab(ray, a.x, a.y, a.z, a.w, c.x, c.y, e0);
+                h1 = slab(ray, b.x, b.y, b.z, b.w, c.z, c.w, e1);
+            }
+            if (CULL)
+            {
+                h0 = h0 && !(e0 > cull);
+                h1 = h1 && !(e1 > cull);
+            }
+            const bool swap = !ANY_HIT && e1 < e0;
+            hNear = swap ? h1 : h0;
+            hFar = swap ? h0 : h1;
+            nearC = swap ? l.y : l.x;
+            farC = swap ? l.x : l.y;
+            nearD = swap ? e1 : e0;
+            farD = swap ? e0 : e1;
+        }
+        else if (mine)
+        {
+            const int leaf = ~e.x;
+            const int start = leaf >> kLeafCountBits;
+            const int n = leaf & ((1 << kLeafCountBits) - 1);
+            // two triangles fetched per step, as in traverse()
+            for (int i = 0; i < n; i += 2)
+            {
+                if (ANY_HIT && found && start + i >= hit.slot)
+                    break;  // a smaller slot already occludes
+                float4 f[2][3];
+#pragma unroll
+                for (int k = 0; k < 2; ++k)
+                {
+                    const float4* tp = reinterpret_cast<const float4*>(sc.tris + start + min(i + k, n - 1));
+                    f[k][0] = __ldg(tp + 0);
+                    f[k][1] = __ldg(tp + 1);
+                    f[k][2] = __ldg(tp + 2);
+                }
+#pragma unroll
+                for (int k = 0; k < 2; ++k)
+                {
+                    const int slot = start + i + k;
+                    const float4 ta = f[k][0], tb = f[k][1], tc = f[k][2];
+                    float t, u, v;
+                    if (i + k >= n || slot == skip || (ANY_HIT && found && slot >= hit.slot) ||
+                        (ANY_HIT && (__float_as_uint(tc.y) & kMetaNonShadowing)) ||
+                        !tri_hit(ray, v3(ta.x, ta.y, ta.z), v3(ta.w, tb.x, tb.y), v3(tb.z, tb.w, tc.x), t, u, v))
+                        continue;
+                    if (!ANY_HIT && ORDER == ORDER_REF && !(t == t))
+                        odd = true;
+                    if (ANY_HIT || t < hit.t || (t == hit.t && slot > hit.slot))
+                    {
+                        hit.slot = slot;
+                        hit.t = t;
+                        hit.u = u;
+                        hit.v = v;
+                        he = __int_as_float(e.y);
+                        found = true;
+                    }
+                }
+            }
+            leafHit = CULL && found;
+        }
+        // far children first, the near ones above them
+        const unsigned mFar = (__ballot_sync(kAll, hFar) >> shift) & gmask;
+        const unsigned mNear = (__ballot_sync(kAll, hNear) >> shift) & gmask;
+        if (hFar)
+            stack[count + __popc(mFar & below)] = make_int2(farC, __float_as_int(farD));
+        if (hNear)
+            stack[count + __popc(mFar) + __popc(mNear & below)] = make_int2(nearC, __float_as_int(nearD));
+        count += __popc(mFar) + __popc(mNear);
+        if (CULL && __ballot_sync(kAll, leafHit))
+        {
+            float tb = hit.t;
+            for (unsigned o = 1; o < G; o <<= 1)
+                tb = fminf(tb, __shfl_xor_sync(kAll, tb, o));
+            cull = tb * kGroupCull;
+        }
+        __syncwarp();
+    }
+    for (unsigned o = 1; o < G; o <<= 1)
+    {
+        HitF h2;
+        const bool f2 = __shfl_xor_sync(kAll, int(found), o) != 0;
+        h2.slot = __shfl_xor_sync(kAll, hit.slot, o);
+        h2.t = __shfl_xor_sync(kAll, hit.t, o);
+        h2.u = __shfl_xor_sync(kAll, hit.u, o);
+        h2.v = __shfl_xor_sync(kAll, hit.v, o);
+        const float he2 = CULL ? __shfl_xor_sync(kAll, he, o) : 0.0f;
+        const bool better = ANY_HIT ? h2.slot < hit.slot : (h2.t < hit.t || (h2.t == hit.t && h2.slot > hit.slot));
+        if (f2 && (!found || better))
+        {
+            hit.slot = h2.slot;
+            hit.t = h2.t;
+            hit.u = h2.u;
+            hit.v = h2.v;
+            he = he2;
+            found = true;
+        }
+    }
+    if (!ANY_HIT)
+    {
+        const unsigned again = __ballot_sync(kAll, CULL ? found && he > hit.t : odd);
+        if (again)
+        {
+            if (gl == 0 && ((again >> shift) & gmask))
+                found = traverse_alone<ORDER>(sc, ray, hit, skip);
+            __syncwarp();
+            found = __shfl_sync(kAll, int(found), int(shift)) != 0;
+            hit.slot = __shfl_sync(kAll, hit.slot, int(shift));
+            hit.t = __shfl_sync(kAll, hit.t, int(shift));
+            hit.u = __shfl_sync(kAll, hit.u, int(shift));
+            hit.v = __shfl_sync(kAll, hit.v, int(shift));
+        }
+    }
+    return found;
+}
+
+// Shared-memory stack entries of a warp's groups together (4 KB).
+constexpr int kGroupEntries = 512;
+
 // Ray in an instance's object space: o' = A o + b, d' = A d. d' is not
 // renormalised, so a hit's parameter t is the same in both spaces and the
 // levels share one closest distance. (The reference's Instance normalises
