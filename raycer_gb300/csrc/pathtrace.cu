@@ -889,6 +889,92 @@ __global__ void __launch_bounds__(BLOCK,
         atomicAdd(finished, 1u);
 }
 
+// A small pass in one kernel: a group of G lanes per path (traverse_group)
+// from the camera ray to the path's end; the group's first lane shades. With
+// fewer paths than lanes a pass is bound by the latency of one path's walks,
+// each a chain of dependent fetches that the group's lanes share. Room of
+// 2,012 triangles, depth 4, one path per pixel, device time with one lane per
+// path -> with groups: 64x48 220 -> 95 us, 128x96 308 -> 126, 256x192
+// 424 -> 256, 400x300 533 -> 472.
+template <bool NRC>
+__global__ void __launch_bounds__(128, 8) k_path_group(PassParams p, unsigned G)
+{
+    __shared__ int2 stacks[4][kGroupEntries];
+    const unsigned total = *reinterpret_cast<volatile unsigned*>(&p.counts[0]);
+    unsigned* head = &p.counts[1];
+    unsigned* finished = &p.counts[2];  // warps that have no more work
+    if (pass_stopped(p))
+        return;
+    if (is_watch_warp(p.monitor, p.budgetNs))
+    {
+        watch_queue(p.monitor, p.budgetNs, p.ctl, head, total, kPublishProgress, 0, finished);
+        return;
+    }
+    const bool watched = monitored(p.monitor, p.budgetNs);
+    const unsigned take = 32u / G;
+    const int capacity = kGroupEntries / int(take);
+    int2* stack = stacks[threadIdx.x >> 5] + int(lane_id() / G) * capacity;
+    const int first = int(lane_id() & ~(G - 1u));  // the group's first lane
+    const bool leader = int(lane_id()) == first;
+    unsigned long long done = 0;
+    bool drained = false;  // warp-uniform
+    int s = -1;            // the group's path, -1 = none
+    int seg = 0;
+    float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f), d = o;
+    while (true)
+    {
+        const unsigned idle = __ballot_sync(0xffffffffu, leader && s < 0);
+        if (idle && !drained)
+        {
+            const unsigned n = unsigned(__popc(idle));
+            const unsigned base = warp_fetch(head, n);
+            drained = base + n >= total;
+            if (s < 0)
+            {
+                const unsigned q = base + unsigned(__popc(idle & ((1u << first) - 1u)));
+                if (q < total)
+                {
+                    s = p.qa[q];
+                    o = p.o[s];
+                    d = p.d[s];
+                    seg = 0;
+                }
+            }
+        }
+        // one decision per warp (lane 0's view of the stop bit)
+        const bool stop = watched && __shfl_sync(0xffffffffu, int(render_stopped(p.ctl)), 0) != 0;
+        if (stop || __ballot_sync(0xffffffffu, s >= 0) == 0u)
+            break;
+        const RayF ray = make_ray(v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), 0.0f, FLT_MAX);
+        HitF h{ -1, FLT_MAX, 0.0f, 0.0f, -1 };
+        const bool found = traverse_group<false, ORDER_NEAREST>(p.scene0, ray, h, __float_as_int(o.w), s >= 0, G, stack,
+                                                                capacity, p.scene0.depth);
+        bool lookup = false, cont = false;
+        NrcRecord lrec;
+        if (leader && s >= 0)
+        {
+            done++;
+            cont = shade_slot<NRC, kRayKept>(p, seg, s, make_int4(found ? h.slot : -1, __float_as_int(h.t), 0, -1), o, d,
+                                             lookup, lrec);
+        }
+        if (NRC)
+            enqueue_lookup(lookup, lrec, p);
+        seg++;
+        if (!__shfl_sync(0xffffffffu, int(cont), first))
+            s = -1;
+        o.x = __shfl_sync(0xffffffffu, o.x, first);
+        o.y = __shfl_sync(0xffffffffu, o.y, first);
+        o.z = __shfl_sync(0xffffffffu, o.z, first);
+        o.w = __shfl_sync(0xffffffffu, o.w, first);
+        d.x = __shfl_sync(0xffffffffu, d.x, first);
+        d.y = __shfl_sync(0xffffffffu, d.y, first);
+        d.z = __shfl_sync(0xffffffffu, d.z, first);
+    }
+    flush_extend_counts(p, done, TravCount{ 0, 0 }, 0);
+    if (watched && lane_id() == 0)
+        atomicAdd(finished, 1u);
+}
+
 __global__ void __launch_bounds__(256) k_accumulate(PassParams p)
 {
     int pix = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1116,6 +1202,34 @@ bool fused_pass(const PassParams& p, int order, int counting)
     return !p.instanced && order == ORDER_NEAREST && !counting && p.wide && !extend_refill() && extend_shade_fused();
 }
 
+// Lanes per path of a one-scene pass, or 0 for one path per lane: the largest
+// group whose two rounds of one path per group (four for groups of 4) cover
+// the pass. Measured on the room above (group of 32 / 16 / 8 / 4 / none):
+// 128x96 169 / 126 / 137 / - / 308 us, 192x144 309 / 208 / 181 / 216 / 360,
+// 320x240 - / - / 363 / 342 / 473, 480x360 - / - / - / 641 / 585. A tree too
+// deep for the group's stack is walked one path per lane.
+unsigned path_group_lanes(const PassParams& p, int order, int counting, int numSMs)
+{
+    constexpr int rounds = 2;
+    if (!p.singleScene || !fused_pass(p, order, counting) || p.segments < 1)
+        return 0u;
+    static OccupancyCache occ;
+    const int64_t lanes = int64_t(persistent_blocks(k_path_group<true>, 128, numSMs, occ)) * 128;
+    for (unsigned G = 32u; G >= 4u; G /= 2u)
+        if (int64_t(p.nslots) * int64_t(G) <= lanes * rounds * (G == 4u ? 2 : 1))
+            return int(G) * kGroupEntries / 32 >= p.scene0.depth + 2 * int(G) ? G : 0u;
+    return 0u;
+}
+
+template <bool NRC>
+cudaError_t path_group_b(const PassParams& p, unsigned G, cudaStream_t stream, int numSMs)
+{
+    auto k = k_path_group<NRC>;
+    static OccupancyCache occ;
+    k<<<persistent_blocks(k, 128, numSMs, occ), 128, 0, stream>>>(p, G);
+    return cudaGetLastError();
+}
+
 }  // namespace
 
 int path_extend_launches(const PassParams& p, int order, int counting)
@@ -1132,6 +1246,20 @@ cudaError_t launch_path_segments(const PassParams& p, int order, int counting, c
         return e;
     const bool fused = fused_pass(p, order, counting);
     const int launches = path_extend_launches(p, order, counting);
+    const unsigned G = path_group_lanes(p, order, counting, numSMs);
+    if (G)
+    {
+        if (extendEvents && (e = cudaEventRecord(extendEvents[0], stream)) != cudaSuccess)
+            return e;
+        if ((e = p.nrc.query ? path_group_b<true>(p, G, stream, numSMs) : path_group_b<false>(p, G, stream, numSMs)) !=
+            cudaSuccess)
+            return e;
+        // every event of the pass is recorded
+        for (int i = 1; extendEvents && i < 2 * launches; ++i)
+            if ((e = cudaEventRecord(extendEvents[i], stream)) != cudaSuccess)
+                return e;
+        return cudaSuccess;
+    }
     for (int seg = 0; seg < launches; ++seg)
     {
         if (extendEvents && (e = cudaEventRecord(extendEvents[2 * seg], stream)) != cudaSuccess)

@@ -1,7 +1,7 @@
-"""The path tracer's bounce kernel (all segments after the camera rays in one
-launch) at the sizes where its work distribution changes: fewer paths than
-warps, a partial warp, about one path per resident warp, more than one; one
-segment (no bounce launch), two, and many, with and without Russian
+"""Passes at the sizes where the path tracer's work distribution changes: a
+group of 32, 16, 8 or 4 lanes per path (small passes, one kernel), one path
+per lane (camera rays, then all later segments in one launch), partial warps;
+one segment (no bounce launch), two, and many, with and without Russian
 roulette. Films equal the float32 oracle's bit for bit."""
 
 from __future__ import annotations
@@ -18,7 +18,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("width,height,depth,rr", [(2, 2, 4, 0), (3, 11, 2, 0), (3, 11, 1, 0), (62, 89, 6, 3),
-                                                   (97, 113, 12, 2)])
+                                                   (97, 113, 12, 2), (139, 141, 5, 0), (200, 195, 4, 3),
+                                                   (400, 390, 1, 0), (400, 390, 2, 0), (400, 390, 7, 3)])
 def test_film_matches_oracle(width, height, depth, rr):
     sc = small_room(width=width, height=height)
     sc.settings.update(multi_sample_count_sqrt=1, path_sample_count=1, max_path_length=depth,
