@@ -515,9 +515,10 @@ rc_status rc_batch_render(rc_batch* b, double* scene_done_ms)
         return fail(b, RC_NOT_READY, "batch_render: no scenes");
     cudaSetDevice(b->device);
     rc_status s;
-    if (!b->graphValid && (s = capture(b)) != RC_OK)
-        return s;
+    // before the capture: it builds the scenes' 4-wide trees, which decide the passes' kernels
     if ((s = upload_scene_table(b)) != RC_OK)
+        return s;
+    if (!b->graphValid && (s = capture(b)) != RC_OK)
         return s;
     RB_TRY(b, cudaGraphLaunch(b->exec, b->stream), "launch batch graph");
     DevControl ctl;
