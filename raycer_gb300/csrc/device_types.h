@@ -57,7 +57,7 @@ struct __align__(32) DevRope
     int miss;
 };
 
-struct __align__(16) DevNode4
+struct __align__(32) DevNode4
 {
     float4 lox, hix, loy, hiy, loz, hiz;  // child k's box in component k
     int4 link;   // child k: >= 0 DevNode4 index, < 0 leaf code ~((start << 4) | count)

@@ -59,6 +59,10 @@ namespace
 #ifndef RC_EXTEND_WIDE_MIN_BLOCKS
 #define RC_EXTEND_WIDE_MIN_BLOCKS 9
 #endif
+// The same for the plain bounce kernel.
+#ifndef RC_BOUNCE_MIN_BLOCKS
+#define RC_BOUNCE_MIN_BLOCKS 8
+#endif
 // The same for the extend + shade kernel of radiance-cache passes, whose
 // shading also writes training vertices and lookups: at 9 blocks it spilled
 // 96 bytes, at 8 (64 registers) 52, and cache frames ran 1 % faster.
@@ -295,8 +299,7 @@ __global__ void __launch_bounds__(BLOCK, (RC_EXTEND_REFILL_MIN_BLOCKS * 128) / B
         return;
     int err = 0;
     unsigned long long done = 0;
-    int stack[kMaxStack];
-    float sdist[kMaxStack];
+    int2 stack[kMaxStack];
     int s = -1;  // this lane's path slot, -1 = idle
     RayF ray;
     HitF h{ -1, FLT_MAX, 0.0f, 0.0f, -1 };
@@ -347,7 +350,7 @@ __global__ void __launch_bounds__(BLOCK, (RC_EXTEND_REFILL_MIN_BLOCKS * 128) / B
                 break;
             continue;
         }
-        if (s >= 0 && wide_step(wide, tris, ray, h, w, stack, sdist, skip, err))
+        if (s >= 0 && wide_step(wide, tris, ray, h, w, stack, skip, err))
         {
             p.hit[s] = make_int4(w.found ? h.slot : -1, __float_as_int(h.t), __float_as_int(h.u), __float_as_int(h.v));
             done++;
@@ -802,22 +805,36 @@ __global__ void __launch_bounds__(BLOCK,
     flush_extend_counts(p, done, TravCount{ 0, 0 }, err);
 }
 
-// Every segment from `first` on in one kernel: a lane takes a path from the
-// queue of segment `first` and traces and shades it, segment after segment
-// with its ray in registers, until the path ends; before each segment the
-// lanes whose path has ended take new ones (one atomic per warp). A launch
-// lasts as long as its longest warp, and one launch per segment paid that
-// tail once per segment (160-200 us for each of the nine segments that only
-// the training paths of a 5M-triangle cache frame reach); here the walks of
-// all segments overlap and the tail is paid once per pass. Frames, render
-// and image: that cache frame 6.21 -> 5.35 ms, the 1080p heightfield of depth
-// 4 1.879 -> 1.780 ms, a 64x48 preview 294 -> 179 us; the room at 16 samples
-// per pixel and dense rooms, whose segments are long, are level. The camera
-// rays keep their own launch: walked in the same warps as bounce rays they
-// lose their coherence (room 2.53 -> 2.71 ms, heightfield 1.78 -> 1.85 ms).
-template <int BLOCK, bool NRC>
+// Every segment from `first` on in one kernel, in warp-wide phases. A lane
+// holds one path: a walk in progress (at a node or at a leaf) or one that is
+// over. Each turn the warp takes one phase for the lanes that wait for it: a
+// node step or a leaf step of two triangles, whichever more lanes wait for,
+// or, once kShadeLanes lanes have finished their walks (or none walks any
+// more), shading: those lanes shade their hits and start the next segment's
+// walk, and the lanes whose path has ended take new ones from the queue.
+//
+// Why one launch: a launch lasts as long as its longest warp, and one launch
+// per segment paid that tail once per segment (160-200 us for each of the
+// nine segments that only the training paths of a 5M-triangle cache frame
+// reach). Why phases: in a loop where each lane steps its own walk until the
+// warp's longest ray is done, 6-7 of 32 lanes worked per instruction; here
+// 14.5-16 do, for 28 % fewer warp instructions in the room of 2,012
+// triangles. What binds it: L1 requests of the divergent node and triangle
+// fetches (L1 75 % busy; one 32-byte load per lane instead of two of 16 took
+// the room from 2.13 to 1.92 ms), issue 52-61 %, ALU 50 %. Device time per
+// frame, a launch per segment -> one launch -> phases and 32-byte loads: room
+// at 16 samples per pixel 2.47 -> 2.35 -> 1.92 ms, 1080p heightfield of depth
+// 4 1.61 -> 1.45 -> 1.29, cache frame 5.88 -> 4.75 -> 4.38.
+//
+// The camera rays keep their own launch: among bounce rays they lose their
+// coherence (room 2.41 ms, heightfield 1.55). Shading at 6 / 10 / 16 / 20 /
+// 24 / 28 finished lanes: room 2.26 / 2.18 / 2.12 / 2.11 / 2.13 / 2.19 ms
+// (with 16-byte loads); 7, 8 and 9 blocks per SM: 2.25 / 2.18 / 2.30.
+constexpr int kShadeLanes = 16;
+
+template <int BLOCK, bool NRC, bool MULTI>
 __global__ void __launch_bounds__(BLOCK,
-                                  ((NRC ? RC_EXTEND_SHADE_NRC_MIN_BLOCKS : RC_EXTEND_WIDE_MIN_BLOCKS) * 128) / BLOCK)
+                                  ((NRC ? RC_EXTEND_SHADE_NRC_MIN_BLOCKS : RC_BOUNCE_MIN_BLOCKS) * 128) / BLOCK)
     k_bounce_paths(PassParams p, int first)
 {
     const unsigned total = *reinterpret_cast<volatile unsigned*>(&p.counts[first * 4 + 0]);
@@ -836,53 +853,86 @@ __global__ void __launch_bounds__(BLOCK,
     // queue would leave other warps without work.
     const unsigned warps = gridDim.x * (BLOCK / 32);
     const unsigned quota = min(32u, (total + warps - 1u) / warps);
+    constexpr unsigned kAll = 0xffffffffu;
     int err = 0;
     unsigned long long done = 0;
     bool drained = total == 0u;  // warp-uniform
     int s = -1;                  // this lane's path, -1 = none
     int seg = first;
     float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f), d = o;
+    RayF ray = make_ray(v3(0.0f, 0.0f, 0.0f), v3(1.0f, 1.0f, 1.0f), 0.0f, FLT_MAX);
+    HitF h{ -1, FLT_MAX, 0.0f, 0.0f, -1 };
+    WideWalk w{ kWalkDone, 0, false };
+    const DevNode4* wide = p.scene0.wide;
+    const DevTri* tris = p.scene0.tris;
+    int2 stack[kMaxStack];
     while (true)
     {
-        const unsigned idle = __ballot_sync(0xffffffffu, s < 0 && lane_id() < quota);
-        if (idle && !drained)
+        const unsigned atNode = __ballot_sync(kAll, w.cur >= 0);
+        const unsigned atLeaf = __ballot_sync(kAll, w.cur < 0 && w.cur != kWalkDone);
+        const unsigned walking = atNode | atLeaf;
+        const unsigned waiting = __ballot_sync(kAll, w.cur == kWalkDone && (s >= 0 || (!drained && lane_id() < quota)));
+        if (waiting && (walking == 0u || __popc(waiting) >= kShadeLanes))
         {
-            const unsigned n = unsigned(__popc(idle));
-            const unsigned base = warp_fetch(head, n);
-            drained = base + n >= total;
-            if ((idle >> lane_id()) & 1u)
+            bool lookup = false;
+            NrcRecord lrec;
+            bool start = false;
+            if (s >= 0 && w.cur == kWalkDone)
             {
+                done++;
+                start = shade_slot<NRC, kRayKept>(
+                    p, seg, s, make_int4(w.found ? h.slot : -1, __float_as_int(h.t), 0, -1), o, d, lookup, lrec);
+                seg++;
+                if (!start)
+                    s = -1;
+            }
+            if (NRC)
+                enqueue_lookup(lookup, lrec, p);
+            const unsigned idle = __ballot_sync(kAll, s < 0 && lane_id() < quota);
+            if (idle && !drained)
+            {
+                const unsigned n = unsigned(__popc(idle));
+                const unsigned base = warp_fetch(head, n);
+                drained = base + n >= total;
                 const unsigned q = base + unsigned(__popc(idle & ((1u << lane_id()) - 1u)));
-                if (q < total)
+                if (((idle >> lane_id()) & 1u) && q < total)
                 {
                     s = queue[q];
                     o = p.o[s];
                     d = p.d[s];
                     seg = first;
+                    start = true;
                 }
             }
+            if (start)
+            {
+                ray = make_ray(v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), 0.0f, FLT_MAX);
+                h = HitF{ -1, FLT_MAX, 0.0f, 0.0f, -1 };
+                w = WideWalk{ p.scene0.wideRoot, 0, false };
+                if (MULTI)
+                {
+                    const DevScene& sc = p.scenes[p.chunks[p.chunkOf[s]].scene].sc;
+                    wide = sc.wide;
+                    tris = sc.tris;
+                    w.cur = sc.wideRoot;
+                }
+            }
+            // one decision per warp (lane 0's view of the stop bit)
+            if (watched && __shfl_sync(kAll, int(render_stopped(p.ctl)), 0) != 0)
+                break;
+            if (__ballot_sync(kAll, s >= 0) == 0u)
+                break;
+            continue;
         }
-        // one decision per warp (lane 0's view of the stop bit)
-        const bool stop = watched && __shfl_sync(0xffffffffu, int(render_stopped(p.ctl)), 0) != 0;
-        if (stop || __ballot_sync(0xffffffffu, s >= 0) == 0u)
+        if (walking == 0u)
             break;
-        bool lookup = false;
-        NrcRecord lrec;
-        if (s >= 0)
+        if (__popc(atLeaf) > __popc(atNode))
         {
-            const DevScene sc = scene_of_slot(p, s);
-            RayF ray = make_ray(v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), 0.0f, FLT_MAX);
-            HitF h{ -1, FLT_MAX, 0.0f, 0.0f, -1 };
-            const bool found = traverse_wide(sc, ray, h, err, __float_as_int(o.w));
-            done++;
-            const bool cont = shade_slot<NRC, kRayKept>(
-                p, seg, s, make_int4(found ? h.slot : -1, __float_as_int(h.t), 0, -1), o, d, lookup, lrec);
-            seg++;
-            if (!cont)
-                s = -1;
+            if (w.cur < 0 && w.cur != kWalkDone)
+                wide_leaf_step(tris, ray, h, w, stack, __float_as_int(o.w));
         }
-        if (NRC)
-            enqueue_lookup(lookup, lrec, p);
+        else if (w.cur >= 0)
+            wide_node_step(wide, ray, h, w, stack, err);
     }
     flush_extend_counts(p, done, TravCount{ 0, 0 }, err);
     if (watched && lane_id() == 0)
@@ -1088,10 +1138,10 @@ cudaError_t extend_shade_b(const PassParams& p, int segment, cudaStream_t stream
     return cudaGetLastError();
 }
 
-template <int BLOCK, bool NRC>
+template <int BLOCK, bool NRC, bool MULTI>
 cudaError_t bounce_paths_b(const PassParams& p, int first, cudaStream_t stream, int numSMs)
 {
-    auto k = k_bounce_paths<BLOCK, NRC>;
+    auto k = k_bounce_paths<BLOCK, NRC, MULTI>;
     static OccupancyCache occ;
     k<<<persistent_blocks(k, BLOCK, numSMs, occ), BLOCK, 0, stream>>>(p, first);
     return cudaGetLastError();
@@ -1099,13 +1149,15 @@ cudaError_t bounce_paths_b(const PassParams& p, int first, cudaStream_t stream, 
 
 cudaError_t bounce_paths_t(const PassParams& p, int first, int block, cudaStream_t stream, int numSMs)
 {
-    if (p.nrc.query)
-        return bounce_paths_b<128, true>(p, first, stream, numSMs);
+    if (p.nrc.query)  // one-scene renders only
+        return bounce_paths_b<128, true, false>(p, first, stream, numSMs);
+    if (p.singleScene)
+        return bounce_paths_b<128, false, false>(p, first, stream, numSMs);
     if (block == 64)
-        return bounce_paths_b<64, false>(p, first, stream, numSMs);
+        return bounce_paths_b<64, false, true>(p, first, stream, numSMs);
     if (block == 256)
-        return bounce_paths_b<256, false>(p, first, stream, numSMs);
-    return bounce_paths_b<128, false>(p, first, stream, numSMs);
+        return bounce_paths_b<256, false, true>(p, first, stream, numSMs);
+    return bounce_paths_b<128, false, true>(p, first, stream, numSMs);
 }
 
 // The block sizes of the kernels it replaces: the autotuned extend block for

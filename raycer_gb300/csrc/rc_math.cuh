@@ -138,6 +138,60 @@ __device__ __forceinline__ bool slab_oct(const RayF& r, float lox, float hix, fl
     return !(tmax < entry);
 }
 
+// Two floats per 64-bit register pair: add, multiply and fused multiply-add of
+// both halves as one instruction, each half rounded as the scalar operation.
+struct F2
+{
+    unsigned long long v;
+};
+
+__device__ __forceinline__ F2 f2(float lo, float hi)
+{
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float f2_lo(F2 a)
+{
+    return __uint_as_float(uint32_t(a.v));
+}
+__device__ __forceinline__ float f2_hi(F2 a)
+{
+    return __uint_as_float(uint32_t(a.v >> 32));
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b)
+{
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b)
+{
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c)
+{
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+
+// Minimum and maximum of three (fminf / fmaxf of the nested pair).
+__device__ __forceinline__ float fmin3(float a, float b, float c)
+{
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float fmax3(float a, float b, float c)
+{
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
 // Sign octant of a ray's inverse direction (slab_oct's OCT), or -1 when a
 // component is not finite (slab_oct does not apply).
 __device__ __forceinline__ int ray_octant(const RayF& r)

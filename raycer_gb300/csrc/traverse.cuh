@@ -68,6 +68,15 @@ __device__ __forceinline__ void load_node(const DevNode* __restrict__ nodes, int
     l = __ldg(reinterpret_cast<const int4*>(p + 3));
 }
 
+// 32 bytes of read-only memory (32-byte aligned) as one load: an L1 request
+// per lane instead of two.
+__device__ __forceinline__ void ldg32(const void* p, float4& a, float4& b)
+{
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(p));
+}
+
 // The test of one leaf triangle in traverse(): nonShadowing triangles are
 // skipped by any-hit rays (Triangle.cpp:55); returns true when an any-hit
 // ray has found its occluder (the walk ends), else updates the closest hit
@@ -318,14 +327,34 @@ __device__ __forceinline__ bool traverse_stackless(const DevScene& sc, const Ray
 }
 
 // Entry distance of one child box of a wide node, or +inf when the ray misses
-// it or enters it beyond `limit` (the current closest hit).
+// it or enters it beyond `limit` (the current closest hit); any ray.
 __device__ __forceinline__ float wide_entry(const RayF& ray, float lox, float hix, float loy, float hiy, float loz,
                                             float hiz, float limit)
 {
     float e;
-    const bool h = ray.finite ? slab_finite(ray, lox, hix, loy, hiy, loz, hiz, e)
-                              : slab(ray, lox, hix, loy, hiy, loz, hiz, e);
+    const bool h = slab(ray, lox, hix, loy, hiy, loz, hiz, e);
     return h && !(e > limit) ? e : __int_as_float(0x7f800000);
+}
+
+// The plane distances of two children on one axis, (plane - o) * inv in
+// slab_finite's arithmetic (subtract, then multiply, each rounded), for both
+// children at once.
+struct AxisF2
+{
+    F2 no;   // -o, -o
+    F2 inv;  // inv, inv
+};
+
+__device__ __forceinline__ F2 plane2(float a, float b, const AxisF2& x) { return mul2(add2(f2(a, b), x.no), x.inv); }
+
+// Entry from the plane distances, as wide_entry for a ray whose inverse
+// direction is finite: entered at the largest near distance (at least 0),
+// left at the smallest far one, both within `limit`.
+__device__ __forceinline__ float wide_entry_of(float x0, float x1, float y0, float y1, float z0, float z1, float limit)
+{
+    const float e = fmaxf(fmax3(fminf(x0, x1), fminf(y0, y1), fminf(z0, z1)), 0.0f);
+    const float f = fminf(fmin3(fmaxf(x0, x1), fmaxf(y0, y1), fmaxf(z0, z1)), limit);
+    return e <= f ? e : __int_as_float(0x7f800000);
 }
 
 // Orders two (distance, link) pairs by distance.
@@ -376,109 +405,140 @@ __device__ __forceinline__ void wide_leaf_test(const RayF& ray, HitF& hit, WideW
     }
 }
 
-// One step of the 4-wide walk: a node fetch (entering its nearest child hit
-// within the current closest distance, the others pushed) or a leaf's
-// triangle tests; where no child is entered, the pop of the next stack entry
-// still in range. Returns true when the walk is over (stack empty, or
-// overflow: err = 1).
-__device__ __forceinline__ bool wide_step(const DevNode4* __restrict__ wide, const DevTri* __restrict__ tris,
-                                          const RayF& ray, HitF& hit, WideWalk& w, int* stack, float* sdist,
-                                          int skip, int& err)
+// A walk that is over (no leaf code has this value: a leaf's last triangle
+// lies below 2^27).
+constexpr int kWalkDone = -0x7fffffff - 1;
+
+// Pops the next stack entry still within the current hit, or ends the walk.
+__device__ __forceinline__ void wide_pop(const HitF& hit, WideWalk& w, const int2* stack)
+{
+    while (w.sp > 0)
+    {
+        const int2 e = stack[--w.sp];
+        w.cur = e.x;
+        if (!(__int_as_float(e.y) > hit.t))
+            return;
+    }
+    w.cur = kWalkDone;
+}
+
+// Node step of the 4-wide walk (w.cur >= 0): enters the nearest child hit
+// within the current closest distance and pushes the others; with none hit,
+// pops. On stack overflow err = 1 and the walk is over.
+__device__ __forceinline__ void wide_node_step(const DevNode4* __restrict__ wide, const RayF& ray, HitF& hit,
+                                               WideWalk& w, int2* stack, int& err)
 {
     const float kInf = __int_as_float(0x7f800000);
-    if (w.cur >= 0)
+    const float4* p = reinterpret_cast<const float4*>(wide + w.cur);
+    float4 lox, hix, loy, hiy, loz, hiz, lf, mf;
+    ldg32(p + 0, lox, hix);
+    ldg32(p + 2, loy, hiy);
+    ldg32(p + 4, loz, hiz);
+    ldg32(p + 6, lf, mf);
+    const int4 l = make_int4(__float_as_int(lf.x), __float_as_int(lf.y), __float_as_int(lf.z), __float_as_int(lf.w));
+    const int nc = __float_as_int(mf.x);
+    float d0, d1, d2, d3;
+    if (ray.finite)
     {
-        const float4* p = reinterpret_cast<const float4*>(wide + w.cur);
-        const float4 lox = __ldg(p + 0), hix = __ldg(p + 1), loy = __ldg(p + 2), hiy = __ldg(p + 3);
-        const float4 loz = __ldg(p + 4), hiz = __ldg(p + 5);
-        const int4 l = __ldg(reinterpret_cast<const int4*>(p + 6));
-        const int nc = __ldg(reinterpret_cast<const int*>(p + 7));
-        float d0 = wide_entry(ray, lox.x, hix.x, loy.x, hiy.x, loz.x, hiz.x, hit.t);
-        float d1 = wide_entry(ray, lox.y, hix.y, loy.y, hiy.y, loz.y, hiz.y, hit.t);
-        float d2 = nc > 2 ? wide_entry(ray, lox.z, hix.z, loy.z, hiy.z, loz.z, hiz.z, hit.t) : kInf;
-        float d3 = nc > 3 ? wide_entry(ray, lox.w, hix.w, loy.w, hiy.w, loz.w, hiz.w, hit.t) : kInf;
-        int l0 = l.x, l1 = l.y, l2 = l.z, l3 = l.w;
-        const int hits = (d0 < kInf ? 1 : 0) + (d1 < kInf ? 1 : 0) + (d2 < kInf ? 1 : 0) + (d3 < kInf ? 1 : 0);
-        if (hits == 1)
+        const AxisF2 X{ f2(-ray.o.x, -ray.o.x), f2(ray.inv.x, ray.inv.x) };
+        const AxisF2 Y{ f2(-ray.o.y, -ray.o.y), f2(ray.inv.y, ray.inv.y) };
+        const AxisF2 Z{ f2(-ray.o.z, -ray.o.z), f2(ray.inv.z, ray.inv.z) };
         {
-            w.cur = d0 < kInf ? l0 : (d1 < kInf ? l1 : (d2 < kInf ? l2 : l3));
-            return false;
+            const F2 x0 = plane2(lox.x, lox.y, X), x1 = plane2(hix.x, hix.y, X);
+            const F2 y0 = plane2(loy.x, loy.y, Y), y1 = plane2(hiy.x, hiy.y, Y);
+            const F2 z0 = plane2(loz.x, loz.y, Z), z1 = plane2(hiz.x, hiz.y, Z);
+            d0 = wide_entry_of(f2_lo(x0), f2_lo(x1), f2_lo(y0), f2_lo(y1), f2_lo(z0), f2_lo(z1), hit.t);
+            d1 = wide_entry_of(f2_hi(x0), f2_hi(x1), f2_hi(y0), f2_hi(y1), f2_hi(z0), f2_hi(z1), hit.t);
         }
-        if (hits > 1)
         {
-            wide_cswap(d0, l0, d1, l1);
-            wide_cswap(d2, l2, d3, l3);
-            wide_cswap(d0, l0, d2, l2);
-            wide_cswap(d1, l1, d3, l3);
-            wide_cswap(d1, l1, d2, l2);
-            if (w.sp + hits - 1 > kMaxStack)
-            {
-                err = 1;
-                return true;
-            }
-            if (d3 < kInf)
-            {
-                stack[w.sp] = l3;
-                sdist[w.sp] = d3;
-                w.sp++;
-            }
-            if (d2 < kInf)
-            {
-                stack[w.sp] = l2;
-                sdist[w.sp] = d2;
-                w.sp++;
-            }
-            if (d1 < kInf)
-            {
-                stack[w.sp] = l1;
-                sdist[w.sp] = d1;
-                w.sp++;
-            }
-            w.cur = l0;
-            return false;
+            const F2 x0 = plane2(lox.z, lox.w, X), x1 = plane2(hix.z, hix.w, X);
+            const F2 y0 = plane2(loy.z, loy.w, Y), y1 = plane2(hiy.z, hiy.w, Y);
+            const F2 z0 = plane2(loz.z, loz.w, Z), z1 = plane2(hiz.z, hiz.w, Z);
+            d2 = wide_entry_of(f2_lo(x0), f2_lo(x1), f2_lo(y0), f2_lo(y1), f2_lo(z0), f2_lo(z1), hit.t);
+            d3 = wide_entry_of(f2_hi(x0), f2_hi(x1), f2_hi(y0), f2_hi(y1), f2_hi(z0), f2_hi(z1), hit.t);
         }
     }
     else
     {
-        const int leaf = ~w.cur;
-        const int start = leaf >> kLeafCountBits;
-        const int count = leaf & ((1 << kLeafCountBits) - 1);
-        // Two triangles per iteration, both fetched before either is tested
-        // (the second index clamped to the leaf: an odd leaf fetches its last
-        // triangle twice and tests it once), so a leaf's fetches overlap.
-        // The accepted hit does not depend on the order of the tests.
-        for (int i = 0; i < count; i += 2)
-        {
-            const int s0 = start + i;
-            const int s1 = start + min(i + 1, count - 1);
-            const float4* p0 = reinterpret_cast<const float4*>(tris + s0);
-            const float4* p1 = reinterpret_cast<const float4*>(tris + s1);
-            const float4 a0 = __ldg(p0 + 0), b0 = __ldg(p0 + 1), c0 = __ldg(p0 + 2);
-            const float4 a1 = __ldg(p1 + 0), b1 = __ldg(p1 + 1), c1 = __ldg(p1 + 2);
-            wide_leaf_test(ray, hit, w, s0, skip, a0, b0, c0);
-            if (i + 1 < count)
-                wide_leaf_test(ray, hit, w, s1, skip, a1, b1, c1);
-        }
+        d0 = wide_entry(ray, lox.x, hix.x, loy.x, hiy.x, loz.x, hiz.x, hit.t);
+        d1 = wide_entry(ray, lox.y, hix.y, loy.y, hiy.y, loz.y, hiz.y, hit.t);
+        d2 = wide_entry(ray, lox.z, hix.z, loy.z, hiy.z, loz.z, hiz.z, hit.t);
+        d3 = wide_entry(ray, lox.w, hix.w, loy.w, hiy.w, loz.w, hiz.w, hit.t);
     }
-    // pop
-    while (true)
+    if (nc < 3)
+        d2 = kInf;
+    if (nc < 4)
+        d3 = kInf;
+    int l0 = l.x, l1 = l.y, l2 = l.z, l3 = l.w;
+    wide_cswap(d0, l0, d1, l1);
+    wide_cswap(d2, l2, d3, l3);
+    wide_cswap(d0, l0, d2, l2);
+    wide_cswap(d1, l1, d3, l3);
+    wide_cswap(d1, l1, d2, l2);
+    if (d0 < kInf)
     {
-        if (w.sp == 0)
-            return true;
-        w.sp--;
-        w.cur = stack[w.sp];
-        if (sdist[w.sp] > hit.t)
-            continue;
-        return false;
+        if (w.sp > kMaxStack - 3 &&
+            w.sp + (d1 < kInf ? 1 : 0) + (d2 < kInf ? 1 : 0) + (d3 < kInf ? 1 : 0) > kMaxStack)
+        {
+            err = 1;
+            w.sp = 0;
+            w.cur = kWalkDone;
+            return;
+        }
+        if (d3 < kInf)
+            stack[w.sp++] = make_int2(l3, __float_as_int(d3));
+        if (d2 < kInf)
+            stack[w.sp++] = make_int2(l2, __float_as_int(d2));
+        if (d1 < kInf)
+            stack[w.sp++] = make_int2(l1, __float_as_int(d1));
+        w.cur = l0;
+        return;
     }
+    wide_pop(hit, w, stack);
+}
+
+// Leaf step (w.cur < 0): two of the leaf's triangles, both fetched before
+// either is tested (the second index clamped to the leaf: an odd leaf fetches
+// its last triangle twice and tests it once), then the rest of the leaf as
+// the next link, or the pop. The accepted hit does not depend on the order
+// of the tests.
+__device__ __forceinline__ void wide_leaf_step(const DevTri* __restrict__ tris, const RayF& ray, HitF& hit, WideWalk& w,
+                                               const int2* stack, int skip)
+{
+    const int leaf = ~w.cur;
+    const int s0 = leaf >> kLeafCountBits;
+    const int count = leaf & ((1 << kLeafCountBits) - 1);
+    const int s1 = s0 + min(1, count - 1);
+    const float4* p0 = reinterpret_cast<const float4*>(tris + s0);
+    const float4* p1 = reinterpret_cast<const float4*>(tris + s1);
+    const float4 a0 = __ldg(p0 + 0), b0 = __ldg(p0 + 1), c0 = __ldg(p0 + 2);
+    const float4 a1 = __ldg(p1 + 0), b1 = __ldg(p1 + 1), c1 = __ldg(p1 + 2);
+    wide_leaf_test(ray, hit, w, s0, skip, a0, b0, c0);
+    if (count > 1)
+        wide_leaf_test(ray, hit, w, s1, skip, a1, b1, c1);
+    if (count > 2)
+        w.cur = ~(((s0 + 2) << kLeafCountBits) | (count - 2));
+    else
+        wide_pop(hit, w, stack);
+}
+
+// One step of the 4-wide walk, a node's or a leaf's. Returns true when the
+// walk is over.
+__device__ __forceinline__ bool wide_step(const DevNode4* __restrict__ wide, const DevTri* __restrict__ tris,
+                                          const RayF& ray, HitF& hit, WideWalk& w, int2* stack, int skip, int& err)
+{
+    if (w.cur >= 0)
+        wide_node_step(wide, ray, hit, w, stack, err);
+    else
+        wide_leaf_step(tris, ray, hit, w, stack, skip);
+    return w.cur == kWalkDone;
 }
 
 __device__ __forceinline__ bool traverse_wide(const DevScene& sc, const RayF& ray, HitF& hit, int& err, int skip)
 {
-    int stack[kMaxStack];
-    float sdist[kMaxStack];
+    int2 stack[kMaxStack];
     WideWalk w{ sc.wideRoot, 0, false };
-    while (!wide_step(sc.wide, sc.tris, ray, hit, w, stack, sdist, skip, err))
+    while (!wide_step(sc.wide, sc.tris, ray, hit, w, stack, skip, err))
     {
     }
     return w.found;
