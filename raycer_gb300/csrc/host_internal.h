@@ -114,9 +114,9 @@ struct rc_tracer
     int32_t tlasRoot = 0;
     std::vector<rcx::InstancedMesh> instMeshes;  // two-level scene: its meshes
     std::vector<rc_instance> instDescs;          //   and instances, for rc_save_scene
-    // 4-wide BVH of a single-level scene (wide_bvh.cpp), or none.
+    // 4-wide BVH of a single-level scene (wide_build.cu), or none.
     rcx::DevNode4* dWide = nullptr;
-    size_t wideCount = 0;
+    size_t wideCount = 0;              // allocated nodes
     int32_t wideRoot = 0;
     bool wideTried = false;  // ensure_wide ran for the current scene
     // Rope records of a single-level scene for the stackless walk (wide_bvh.cpp), or none.
@@ -232,13 +232,10 @@ void build_host_scene(const double* v, const uint32_t* matIdx, int64_t n, const 
                       std::vector<BuildNode>&& nodes, std::vector<uint32_t>&& order, uint32_t depth, HostScene& hs);
 rc_status upload_host_scene(rc_tracer* h, HostScene&& hs);
 void release_scene_data(rc_tracer* h);
-// Collapses the binary device nodes (root `rootLink`) into the 4-wide BVH and
-// uploads it (h->dWide); leaves it out where its stack need exceeds the
-// traversal stack. Failure to allocate is an error.
-rc_status upload_wide(rc_tracer* h, const std::vector<DevNode>& nodes, int32_t rootLink);
-// Builds the 4-wide BVH of the handle's single-level scene on first use (the
-// first PATH or batch render of a scene): downloads the binary nodes once,
-// collapses and uploads them. Uploads and RAY frames do not pay for it.
+// Collapses the binary device nodes of the handle's single-level scene into
+// the 4-wide BVH on first use (the first PATH or batch render of a scene);
+// leaves it out where its stack need exceeds the traversal stack. Failure to
+// allocate is an error. Uploads and RAY frames do not pay for it.
 rc_status ensure_wide(rc_tracer* h);
 // Builds the rope records of the handle's single-level scene on first use
 // (the first RAY frame or rc_cast while the stackless walk is on): one

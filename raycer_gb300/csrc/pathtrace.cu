@@ -299,11 +299,12 @@ __global__ void __launch_bounds__(BLOCK, (RC_EXTEND_REFILL_MIN_BLOCKS * 128) / B
         return;
     int err = 0;
     unsigned long long done = 0;
-    int2 stack[kMaxStack];
+    int2 entries[kMaxStack];
+    LocalStack stack{ entries };
     int s = -1;  // this lane's path slot, -1 = idle
     RayF ray;
     HitF h{ -1, FLT_MAX, 0.0f, 0.0f, -1 };
-    WideWalk w{ 0, 0, false };
+    WideWalk w{ 0, 0 };
     int skip = -1;
     const DevNode4* wide = nullptr;
     const DevTri* tris = nullptr;
@@ -337,7 +338,7 @@ __global__ void __launch_bounds__(BLOCK, (RC_EXTEND_REFILL_MIN_BLOCKS * 128) / B
                     const float4 d = p.d[s];
                     ray = make_ray(v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), 0.0f, FLT_MAX);
                     h = HitF{ -1, FLT_MAX, 0.0f, 0.0f, -1 };
-                    w = WideWalk{ sc.wideRoot, 0, false };
+                    w = WideWalk{ sc.wideRoot, 0 };
                     skip = __float_as_int(o.w);
                     wide = sc.wide;
                     tris = sc.tris;
@@ -352,7 +353,7 @@ __global__ void __launch_bounds__(BLOCK, (RC_EXTEND_REFILL_MIN_BLOCKS * 128) / B
         }
         if (s >= 0 && wide_step(wide, tris, ray, h, w, stack, skip, err))
         {
-            p.hit[s] = make_int4(w.found ? h.slot : -1, __float_as_int(h.t), __float_as_int(h.u), __float_as_int(h.v));
+            p.hit[s] = make_int4(h.slot, __float_as_int(h.t), __float_as_int(h.u), __float_as_int(h.v));
             done++;
             s = -1;
         }
@@ -820,22 +821,38 @@ __global__ void __launch_bounds__(BLOCK,
 // warp's longest ray is done, 6-7 of 32 lanes worked per instruction; here
 // 14.5-16 do, for 28 % fewer warp instructions in the room of 2,012
 // triangles. What binds it: L1 requests of the divergent node and triangle
-// fetches (L1 75 % busy; one 32-byte load per lane instead of two of 16 took
-// the room from 2.13 to 1.92 ms), issue 52-61 %, ALU 50 %. Device time per
+// fetches, one wavefront per lane and load (76 % of the L1's wavefronts; one
+// 32-byte load per lane instead of two of 16 took the room from 2.13 to
+// 1.92 ms), issue 56-63 %, ALU 53 %. Device time per
 // frame, a launch per segment -> one launch -> phases and 32-byte loads: room
 // at 16 samples per pixel 2.47 -> 2.35 -> 1.92 ms, 1080p heightfield of depth
-// 4 1.61 -> 1.45 -> 1.29, cache frame 5.88 -> 4.75 -> 4.38.
+// 4 1.61 -> 1.45 -> 1.28, cache frame 5.88 -> 4.75 -> 4.31.
 //
-// The camera rays keep their own launch: among bounce rays they lose their
-// coherence (room 2.41 ms, heightfield 1.55). Shading at 6 / 10 / 16 / 20 /
+// The camera rays keep their own launch and k_extend_shade's loop: among
+// bounce rays they lose their coherence (room 2.41 ms, heightfield 1.55), and
+// in phases of their own they gain less than the turns cost (room 1.98,
+// heightfield 1.37). Shading at 6 / 10 / 16 / 20 /
 // 24 / 28 finished lanes: room 2.26 / 2.18 / 2.12 / 2.11 / 2.13 / 2.19 ms
 // (with 16-byte loads); 7, 8 and 9 blocks per SM: 2.25 / 2.18 / 2.30.
 constexpr int kShadeLanes = 16;
+// The walks' first stack entries are in shared memory (SharedStack): in local
+// memory each divergent push and pop was an L1 request per lane. 8 / 12 / 16
+// entries: cache frame 4.41 / 4.37 / 4.41 ms, dense rooms 45.0 / 43.5 / 43.4.
+constexpr int kNearEntries = 12;
+
+// The bounce kernel's shading, out of line: inlined, its registers made the
+// walk loop spill.
+template <bool NRC>
+static __device__ __noinline__ bool shade_kept(const PassParams& p, int segment, int s, int slot, float t, float4& o,
+                                               float4& d, bool& lookup, NrcRecord& lrec)
+{
+    return shade_slot<NRC, kRayKept>(p, segment, s, make_int4(slot, __float_as_int(t), 0, -1), o, d, lookup, lrec);
+}
 
 template <int BLOCK, bool NRC, bool MULTI>
 __global__ void __launch_bounds__(BLOCK,
                                   ((NRC ? RC_EXTEND_SHADE_NRC_MIN_BLOCKS : RC_BOUNCE_MIN_BLOCKS) * 128) / BLOCK)
-    k_bounce_paths(PassParams p, int first)
+    k_bounce_paths(const __grid_constant__ PassParams p, int first)
 {
     const unsigned total = *reinterpret_cast<volatile unsigned*>(&p.counts[first * 4 + 0]);
     const int* __restrict__ queue = (first & 1) ? p.qb : p.qa;
@@ -854,41 +871,47 @@ __global__ void __launch_bounds__(BLOCK,
     const unsigned warps = gridDim.x * (BLOCK / 32);
     const unsigned quota = min(32u, (total + warps - 1u) / warps);
     constexpr unsigned kAll = 0xffffffffu;
-    int err = 0;
-    unsigned long long done = 0;
+    // this lane's path and its segment: touched by shading only, so they
+    // leave the walk its registers
+    __shared__ int2 paths[BLOCK];
+    unsigned done = 0;           // warp-uniform
     bool drained = total == 0u;  // warp-uniform
-    int s = -1;                  // this lane's path, -1 = none
-    int seg = first;
+    int err = 0;
     float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f), d = o;
     RayF ray = make_ray(v3(0.0f, 0.0f, 0.0f), v3(1.0f, 1.0f, 1.0f), 0.0f, FLT_MAX);
     HitF h{ -1, FLT_MAX, 0.0f, 0.0f, -1 };
-    WideWalk w{ kWalkDone, 0, false };
+    WideWalk w{ kWalkNone, 0 };
     const DevNode4* wide = p.scene0.wide;
     const DevTri* tris = p.scene0.tris;
-    int2 stack[kMaxStack];
+    __shared__ int2 nearEntries[kNearEntries][BLOCK];
+    int2 farEntries[kMaxStack - kNearEntries];
+    SharedStack<kNearEntries, BLOCK> stack{ &nearEntries[0][threadIdx.x], farEntries };
     while (true)
     {
         const unsigned atNode = __ballot_sync(kAll, w.cur >= 0);
-        const unsigned atLeaf = __ballot_sync(kAll, w.cur < 0 && w.cur != kWalkDone);
+        const unsigned atLeaf = __ballot_sync(kAll, w.cur < 0 && w.cur > kWalkNone);
         const unsigned walking = atNode | atLeaf;
-        const unsigned waiting = __ballot_sync(kAll, w.cur == kWalkDone && (s >= 0 || (!drained && lane_id() < quota)));
+        const unsigned waiting =
+            __ballot_sync(kAll, w.cur == kWalkDone || (w.cur == kWalkNone && !drained && lane_id() < quota));
         if (waiting && (walking == 0u || __popc(waiting) >= kShadeLanes))
         {
             bool lookup = false;
             NrcRecord lrec;
             bool start = false;
-            if (s >= 0 && w.cur == kWalkDone)
+            done += unsigned(__popc(__ballot_sync(kAll, w.cur == kWalkDone)));
+            if (w.cur == kWalkDone)
             {
-                done++;
-                start = shade_slot<NRC, kRayKept>(
-                    p, seg, s, make_int4(w.found ? h.slot : -1, __float_as_int(h.t), 0, -1), o, d, lookup, lrec);
-                seg++;
-                if (!start)
-                    s = -1;
+                const int2 path = paths[threadIdx.x];
+                float4 o2 = o, d2 = d;
+                start = shade_kept<NRC>(p, path.y, path.x, h.slot, h.t, o2, d2, lookup, lrec);
+                paths[threadIdx.x].y = path.y + 1;
+                o = o2;
+                d = d2;
+                w.cur = kWalkNone;
             }
             if (NRC)
                 enqueue_lookup(lookup, lrec, p);
-            const unsigned idle = __ballot_sync(kAll, s < 0 && lane_id() < quota);
+            const unsigned idle = __ballot_sync(kAll, w.cur == kWalkNone && !start && lane_id() < quota);
             if (idle && !drained)
             {
                 const unsigned n = unsigned(__popc(idle));
@@ -897,10 +920,10 @@ __global__ void __launch_bounds__(BLOCK,
                 const unsigned q = base + unsigned(__popc(idle & ((1u << lane_id()) - 1u)));
                 if (((idle >> lane_id()) & 1u) && q < total)
                 {
-                    s = queue[q];
+                    const int s = queue[q];
+                    paths[threadIdx.x] = make_int2(s, first);
                     o = p.o[s];
                     d = p.d[s];
-                    seg = first;
                     start = true;
                 }
             }
@@ -908,10 +931,10 @@ __global__ void __launch_bounds__(BLOCK,
             {
                 ray = make_ray(v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), 0.0f, FLT_MAX);
                 h = HitF{ -1, FLT_MAX, 0.0f, 0.0f, -1 };
-                w = WideWalk{ p.scene0.wideRoot, 0, false };
+                w = WideWalk{ p.scene0.wideRoot, 0 };
                 if (MULTI)
                 {
-                    const DevScene& sc = p.scenes[p.chunks[p.chunkOf[s]].scene].sc;
+                    const DevScene& sc = p.scenes[p.chunks[p.chunkOf[paths[threadIdx.x].x]].scene].sc;
                     wide = sc.wide;
                     tris = sc.tris;
                     w.cur = sc.wideRoot;
@@ -920,7 +943,7 @@ __global__ void __launch_bounds__(BLOCK,
             // one decision per warp (lane 0's view of the stop bit)
             if (watched && __shfl_sync(kAll, int(render_stopped(p.ctl)), 0) != 0)
                 break;
-            if (__ballot_sync(kAll, s >= 0) == 0u)
+            if (__ballot_sync(kAll, w.cur > kWalkNone) == 0u)
                 break;
             continue;
         }
@@ -928,13 +951,13 @@ __global__ void __launch_bounds__(BLOCK,
             break;
         if (__popc(atLeaf) > __popc(atNode))
         {
-            if (w.cur < 0 && w.cur != kWalkDone)
+            if (w.cur < 0 && w.cur > kWalkNone)
                 wide_leaf_step(tris, ray, h, w, stack, __float_as_int(o.w));
         }
         else if (w.cur >= 0)
             wide_node_step(wide, ray, h, w, stack, err);
     }
-    flush_extend_counts(p, done, TravCount{ 0, 0 }, err);
+    flush_extend_counts(p, lane_id() == 0 ? done : 0u, TravCount{ 0, 0 }, err);
     if (watched && lane_id() == 0)
         atomicAdd(finished, 1u);
 }

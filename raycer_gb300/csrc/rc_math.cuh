@@ -138,8 +138,8 @@ __device__ __forceinline__ bool slab_oct(const RayF& r, float lox, float hix, fl
     return !(tmax < entry);
 }
 
-// Two floats per 64-bit register pair: add, multiply and fused multiply-add of
-// both halves as one instruction, each half rounded as the scalar operation.
+// Two floats per 64-bit register pair: add and multiply of both halves as one
+// instruction, each half rounded as the scalar operation.
 struct F2
 {
     unsigned long long v;
@@ -171,13 +171,6 @@ __device__ __forceinline__ F2 mul2(F2 a, F2 b)
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
     return r;
 }
-__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c)
-{
-    F2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-    return r;
-}
-
 // Minimum and maximum of three (fminf / fmaxf of the nested pair).
 __device__ __forceinline__ float fmin3(float a, float b, float c)
 {

@@ -384,37 +384,48 @@ struct WideWalk
 {
     int cur;
     int sp;
-    bool found;
 };
-
-// The closest-hit test of one leaf triangle in the 4-wide walk.
-__device__ __forceinline__ void wide_leaf_test(const RayF& ray, HitF& hit, WideWalk& w, int slot, int skip,
-                                               const float4& ta, const float4& tb, const float4& tc)
-{
-    if (slot == skip)
-        return;
-    float t, u, v;
-    if (tri_hit(ray, v3(ta.x, ta.y, ta.z), v3(ta.w, tb.x, tb.y), v3(tb.z, tb.w, tc.x), t, u, v) &&
-        (t < hit.t || (t == hit.t && slot > hit.slot)))
-    {
-        hit.slot = slot;
-        hit.t = t;
-        hit.u = u;
-        hit.v = v;
-        w.found = true;
-    }
-}
 
 // A walk that is over (no leaf code has this value: a leaf's last triangle
 // lies below 2^27).
 constexpr int kWalkDone = -0x7fffffff - 1;
+// A lane without a walk (no leaf code either: its 14 triangles would start
+// at slot 2^27 - 1, the last one).
+constexpr int kWalkNone = -0x7fffffff;
+
+// A walk's stack in local memory.
+struct LocalStack
+{
+    int2* e;
+    __device__ __forceinline__ void put(int i, int2 v) { e[i] = v; }
+    __device__ __forceinline__ int2 get(int i) const { return e[i]; }
+};
+
+// A walk's stack with its first D entries in shared memory, entry i of the
+// block's threads side by side (a warp's accesses meet no bank twice, whatever
+// the depths), the rest in local memory.
+template <int D, int THREADS>
+struct SharedStack
+{
+    int2* near;  // this thread's entry 0
+    int2* far;
+    __device__ __forceinline__ void put(int i, int2 v)
+    {
+        if (i < D)
+            near[i * THREADS] = v;
+        else
+            far[i - D] = v;
+    }
+    __device__ __forceinline__ int2 get(int i) const { return i < D ? near[i * THREADS] : far[i - D]; }
+};
 
 // Pops the next stack entry still within the current hit, or ends the walk.
-__device__ __forceinline__ void wide_pop(const HitF& hit, WideWalk& w, const int2* stack)
+template <typename Stack>
+__device__ __forceinline__ void wide_pop(const HitF& hit, WideWalk& w, const Stack& stack)
 {
     while (w.sp > 0)
     {
-        const int2 e = stack[--w.sp];
+        const int2 e = stack.get(--w.sp);
         w.cur = e.x;
         if (!(__int_as_float(e.y) > hit.t))
             return;
@@ -425,8 +436,9 @@ __device__ __forceinline__ void wide_pop(const HitF& hit, WideWalk& w, const int
 // Node step of the 4-wide walk (w.cur >= 0): enters the nearest child hit
 // within the current closest distance and pushes the others; with none hit,
 // pops. On stack overflow err = 1 and the walk is over.
+template <typename Stack>
 __device__ __forceinline__ void wide_node_step(const DevNode4* __restrict__ wide, const RayF& ray, HitF& hit,
-                                               WideWalk& w, int2* stack, int& err)
+                                               WideWalk& w, Stack& stack, int& err)
 {
     const float kInf = __int_as_float(0x7f800000);
     const float4* p = reinterpret_cast<const float4*>(wide + w.cur);
@@ -486,24 +498,44 @@ __device__ __forceinline__ void wide_node_step(const DevNode4* __restrict__ wide
             return;
         }
         if (d3 < kInf)
-            stack[w.sp++] = make_int2(l3, __float_as_int(d3));
+            stack.put(w.sp++, make_int2(l3, __float_as_int(d3)));
         if (d2 < kInf)
-            stack[w.sp++] = make_int2(l2, __float_as_int(d2));
+            stack.put(w.sp++, make_int2(l2, __float_as_int(d2)));
         if (d1 < kInf)
-            stack[w.sp++] = make_int2(l1, __float_as_int(d1));
+            stack.put(w.sp++, make_int2(l1, __float_as_int(d1)));
         w.cur = l0;
         return;
     }
     wide_pop(hit, w, stack);
 }
 
+// The closest-hit test of one leaf triangle in the 4-wide walk.
+__device__ __forceinline__ void wide_leaf_test(const RayF& ray, HitF& hit, int slot, int skip, const float4& ta,
+                                               const float4& tb, const float4& tc)
+{
+    if (slot == skip)
+        return;
+    float t, u, v;
+    if (tri_hit(ray, v3(ta.x, ta.y, ta.z), v3(ta.w, tb.x, tb.y), v3(tb.z, tb.w, tc.x), t, u, v) &&
+        (t < hit.t || (t == hit.t && slot > hit.slot)))
+    {
+        hit.slot = slot;
+        hit.t = t;
+        hit.u = u;
+        hit.v = v;
+    }
+}
+
 // Leaf step (w.cur < 0): two of the leaf's triangles, both fetched before
 // either is tested (the second index clamped to the leaf: an odd leaf fetches
 // its last triangle twice and tests it once), then the rest of the leaf as
 // the next link, or the pop. The accepted hit does not depend on the order
-// of the tests.
+// of the tests. (Both triangles at once in two-wide arithmetic, from records
+// of interleaved pairs: no faster, for 8 more registers and 60 MB per 1M
+// triangles.)
+template <typename Stack>
 __device__ __forceinline__ void wide_leaf_step(const DevTri* __restrict__ tris, const RayF& ray, HitF& hit, WideWalk& w,
-                                               const int2* stack, int skip)
+                                               const Stack& stack, int skip)
 {
     const int leaf = ~w.cur;
     const int s0 = leaf >> kLeafCountBits;
@@ -513,9 +545,9 @@ __device__ __forceinline__ void wide_leaf_step(const DevTri* __restrict__ tris, 
     const float4* p1 = reinterpret_cast<const float4*>(tris + s1);
     const float4 a0 = __ldg(p0 + 0), b0 = __ldg(p0 + 1), c0 = __ldg(p0 + 2);
     const float4 a1 = __ldg(p1 + 0), b1 = __ldg(p1 + 1), c1 = __ldg(p1 + 2);
-    wide_leaf_test(ray, hit, w, s0, skip, a0, b0, c0);
+    wide_leaf_test(ray, hit, s0, skip, a0, b0, c0);
     if (count > 1)
-        wide_leaf_test(ray, hit, w, s1, skip, a1, b1, c1);
+        wide_leaf_test(ray, hit, s1, skip, a1, b1, c1);
     if (count > 2)
         w.cur = ~(((s0 + 2) << kLeafCountBits) | (count - 2));
     else
@@ -524,8 +556,9 @@ __device__ __forceinline__ void wide_leaf_step(const DevTri* __restrict__ tris, 
 
 // One step of the 4-wide walk, a node's or a leaf's. Returns true when the
 // walk is over.
+template <typename Stack>
 __device__ __forceinline__ bool wide_step(const DevNode4* __restrict__ wide, const DevTri* __restrict__ tris,
-                                          const RayF& ray, HitF& hit, WideWalk& w, int2* stack, int skip, int& err)
+                                          const RayF& ray, HitF& hit, WideWalk& w, Stack& stack, int skip, int& err)
 {
     if (w.cur >= 0)
         wide_node_step(wide, ray, hit, w, stack, err);
@@ -536,12 +569,13 @@ __device__ __forceinline__ bool wide_step(const DevNode4* __restrict__ wide, con
 
 __device__ __forceinline__ bool traverse_wide(const DevScene& sc, const RayF& ray, HitF& hit, int& err, int skip)
 {
-    int2 stack[kMaxStack];
-    WideWalk w{ sc.wideRoot, 0, false };
+    int2 entries[kMaxStack];
+    LocalStack stack{ entries };
+    WideWalk w{ sc.wideRoot, 0 };
     while (!wide_step(sc.wide, sc.tris, ray, hit, w, stack, skip, err))
     {
     }
-    return w.found;
+    return hit.slot >= 0;
 }
 
 // One stack entry of the warp-wide traversal: a node link and the lanes
