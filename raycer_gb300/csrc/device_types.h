@@ -95,6 +95,7 @@ constexpr uint32_t kMatDielectric = 8u;  // DevMat.diffuse.w = index of refracti
 
 constexpr int kLeafCountBits = 4;
 constexpr int kMaxStack = 64;
+constexpr int kTwoLevelStack = 96;  // entries of a two-level scene's 4-wide walk, both levels
 
 // One placed copy of a mesh (two-level scenes): world -> object rows
 // (object = A world + b; r_i = (A_i0, A_i1, A_i2, b_i)), the mesh's BVH
@@ -144,6 +145,11 @@ struct DevScene
     int numInstances;  // 0: single-level scene
     const DevNode4* wide;  // 4-wide BVH of a single-level scene, or null
     int wideRoot;          // >= 0: DevNode4 0; < 0: the root is a leaf
+    // two-level scenes: the meshes' 4-wide trees are in `wide`; the instances'
+    // top-level one, and each instance's mesh root in `wide` (or leaf code)
+    const DevNode4* wideTlas;
+    const int* instWide;
+    int wideTlasRoot;
     int ropeCount;         // records in `ropes`
     const DevRope* ropes;  // the stackless walk's records of a single-level scene, or null
     RenderMonitor* monitor = nullptr;          // rc_render with a cancel flag or progress counter, else null

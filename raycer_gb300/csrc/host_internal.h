@@ -118,6 +118,14 @@ struct rc_tracer
     rcx::DevNode4* dWide = nullptr;
     size_t wideCount = 0;              // allocated nodes
     int32_t wideRoot = 0;
+    // Two-level scene: its instances' mesh roots (binary links, in top-level
+    // order), the 4-wide top-level tree and each instance's 4-wide mesh root.
+    std::vector<int32_t> instRoots;
+    rcx::DevNode4* dWideTlas = nullptr;
+    size_t wideTlasCount = 0;
+    int32_t wideTlasRoot = 0;
+    int32_t* dInstWide = nullptr;
+    bool wideInstanced = false;  // the three above and dWide are built
     bool wideTried = false;  // ensure_wide ran for the current scene
     // Rope records of a single-level scene for the stackless walk (wide_bvh.cpp), or none.
     rcx::DevRope* dRopes = nullptr;

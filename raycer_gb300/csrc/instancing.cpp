@@ -476,6 +476,9 @@ rc_status upload_instanced_scenes(rc_tracer* h, std::vector<HostScene>&& meshSce
     h->tlasCount = tn.size();
     h->nInstances = ni;
     h->tlasRoot = troot;
+    h->instRoots.clear();
+    for (const DevInstance& in : ordered)
+        h->instRoots.push_back(in.rootLink);
     h->rootLink = meshRoot[0];
     uint32_t depth = 0;
     for (uint32_t d : meshDepth)

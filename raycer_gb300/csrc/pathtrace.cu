@@ -24,7 +24,8 @@
 //              Film.cpp:54-59). One thread owns one pixel: deterministic.
 // Uncounted nearest-first passes over the 4-wide BVH run extend and shade of
 // a segment as one kernel (k_extend_shade); the hit record is then never
-// written.
+// written. All segments after the first run as one kernel (k_bounce_paths,
+// k_bounce_instanced); small passes run whole in one (k_path_group).
 // Queue counts live on the device, so a pass is a fixed launch sequence the
 // host never waits on (and can be captured in a CUDA graph).
 
@@ -843,10 +844,10 @@ constexpr int kNearEntries = 12;
 // The bounce kernel's shading, out of line: inlined, its registers made the
 // walk loop spill.
 template <bool NRC>
-static __device__ __noinline__ bool shade_kept(const PassParams& p, int segment, int s, int slot, float t, float4& o,
-                                               float4& d, bool& lookup, NrcRecord& lrec)
+static __device__ __noinline__ bool shade_kept(const PassParams& p, int segment, int s, int slot, float t, int inst,
+                                               float4& o, float4& d, bool& lookup, NrcRecord& lrec)
 {
-    return shade_slot<NRC, kRayKept>(p, segment, s, make_int4(slot, __float_as_int(t), 0, -1), o, d, lookup, lrec);
+    return shade_slot<NRC, kRayKept>(p, segment, s, make_int4(slot, __float_as_int(t), 0, inst), o, d, lookup, lrec);
 }
 
 template <int BLOCK, bool NRC, bool MULTI>
@@ -903,7 +904,7 @@ __global__ void __launch_bounds__(BLOCK,
             {
                 const int2 path = paths[threadIdx.x];
                 float4 o2 = o, d2 = d;
-                start = shade_kept<NRC>(p, path.y, path.x, h.slot, h.t, o2, d2, lookup, lrec);
+                start = shade_kept<NRC>(p, path.y, path.x, h.slot, h.t, -1, o2, d2, lookup, lrec);
                 paths[threadIdx.x].y = path.y + 1;
                 o = o2;
                 d = d2;
@@ -956,6 +957,162 @@ __global__ void __launch_bounds__(BLOCK,
         }
         else if (w.cur >= 0)
             wide_node_step(wide, ray, h, w, stack, err);
+    }
+    flush_extend_counts(p, lane_id() == 0 ? done : 0u, TravCount{ 0, 0 }, err);
+    if (watched && lane_id() == 0)
+        atomicAdd(finished, 1u);
+}
+
+// The bounce kernel for two-level scenes: one walk over both levels
+// (TwoLevelWalk, 4-wide trees), with one more phase, which takes lanes into an
+// instance (its ray transformed) or back out of it. Nested loops, as in
+// traverse_instanced, held a warp in step instance by instance: a segment's
+// launch took 600 us however few paths it had. 1080p, heightfield + 200
+// blobs of 20,480 triangles, 30 % glass, depth 12: 11.1 -> 5.8 ms of device
+// time. Bound by ALU (58 %) and issue (63 %) at 14.6 lanes per instruction.
+// The camera rays stay with k_extend_instanced and k_shade, whose coherent
+// warps lose nothing to the nesting (1.10 ms; 1.34 in phases). 6, 7 and 8
+// blocks per SM: 6.10 / 5.85 / 6.37 (72 registers; 8 blocks spill).
+#ifndef RC_INST_MIN_BLOCKS
+#define RC_INST_MIN_BLOCKS 7
+#endif
+template <bool NRC>
+__global__ void __launch_bounds__(128, RC_INST_MIN_BLOCKS)
+    k_bounce_instanced(const __grid_constant__ PassParams p, int first)
+{
+    constexpr int BLOCK = 128;
+    const unsigned total = *reinterpret_cast<volatile unsigned*>(&p.counts[first * 4 + 0]);
+    const int* __restrict__ queue = (first & 1) ? p.qb : p.qa;
+    unsigned* head = &p.counts[first * 4 + 1];
+    unsigned* finished = &p.counts[first * 4 + 2];  // warps that have no more work
+    if (pass_stopped(p))
+        return;
+    if (is_watch_warp(p.monitor, p.budgetNs))
+    {
+        watch_queue(p.monitor, p.budgetNs, p.ctl, head, total, kPublishProgress, 0, finished);
+        return;
+    }
+    const bool watched = monitored(p.monitor, p.budgetNs);
+    const unsigned warps = gridDim.x * (BLOCK / 32);
+    const unsigned quota = min(32u, (total + warps - 1u) / warps);
+    constexpr unsigned kAll = 0xffffffffu;
+    __shared__ int2 paths[BLOCK];    // this lane's path and its segment
+    __shared__ float4 worldO[BLOCK];  // its ray in world space (w: the triangle and instance it leaves)
+    __shared__ float4 worldD[BLOCK];
+    __shared__ int skips[BLOCK];      // the triangle the walk skips in its instance
+    __shared__ int hitInst[BLOCK];    // the closest hit's instance
+    __shared__ int2 nearEntries[kNearEntries][BLOCK];
+    int2 farEntries[kTwoLevelStack - kNearEntries];
+    SharedStack<kNearEntries, BLOCK, kTwoLevelStack> stack{ &nearEntries[0][threadIdx.x], farEntries };
+    unsigned done = 0;           // warp-uniform
+    bool drained = total == 0u;  // warp-uniform
+    int err = 0;
+    RayF ray = make_ray(v3(0.0f, 0.0f, 0.0f), v3(1.0f, 1.0f, 1.0f), 0.0f, FLT_MAX);
+    HitF h{ -1, FLT_MAX, 0.0f, 0.0f, -1 };
+    TwoLevelWalk w{ kWalkNone, 0, 0, -1 };
+    while (true)
+    {
+        const unsigned atNode = __ballot_sync(kAll, w.cur >= 0);
+        const bool leaf = w.cur < 0 && w.cur > kWalkReturn;
+        const unsigned atLeaf = __ballot_sync(kAll, leaf && w.inst >= 0);
+        const unsigned atSwitch = __ballot_sync(kAll, w.cur == kWalkReturn || (leaf && w.inst < 0));
+        const unsigned walking = atNode | atLeaf | atSwitch;
+        const unsigned waiting =
+            __ballot_sync(kAll, w.cur == kWalkDone || (w.cur == kWalkNone && !drained && lane_id() < quota));
+        if (waiting && (walking == 0u || __popc(waiting) >= kShadeLanes))
+        {
+            bool lookup = false;
+            NrcRecord lrec;
+            bool start = false;
+            done += unsigned(__popc(__ballot_sync(kAll, w.cur == kWalkDone)));
+            float4 o, d;
+            if (w.cur == kWalkDone)
+            {
+                const int2 path = paths[threadIdx.x];
+                o = worldO[threadIdx.x];
+                d = worldD[threadIdx.x];
+                start = shade_kept<NRC>(p, path.y, path.x, h.slot, h.t, hitInst[threadIdx.x], o, d, lookup, lrec);
+                paths[threadIdx.x].y = path.y + 1;
+                w.cur = kWalkNone;
+            }
+            if (NRC)
+                enqueue_lookup(lookup, lrec, p);
+            const unsigned idle = __ballot_sync(kAll, w.cur == kWalkNone && !start && lane_id() < quota);
+            if (idle && !drained)
+            {
+                const unsigned n = unsigned(__popc(idle));
+                const unsigned base = warp_fetch(head, n);
+                drained = base + n >= total;
+                const unsigned q = base + unsigned(__popc(idle & ((1u << lane_id()) - 1u)));
+                if (((idle >> lane_id()) & 1u) && q < total)
+                {
+                    const int s = queue[q];
+                    paths[threadIdx.x] = make_int2(s, first);
+                    o = p.o[s];
+                    d = p.d[s];
+                    start = true;
+                }
+            }
+            if (start)
+            {
+                worldO[threadIdx.x] = o;
+                worldD[threadIdx.x] = d;
+                ray = make_ray(v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), 0.0f, FLT_MAX);
+                h = HitF{ -1, FLT_MAX, 0.0f, 0.0f, -1 };
+                hitInst[threadIdx.x] = -1;
+                w = TwoLevelWalk{ p.scene0.wideTlasRoot, 0, 0, -1 };
+            }
+            // one decision per warp (lane 0's view of the stop bit)
+            if (watched && __shfl_sync(kAll, int(render_stopped(p.ctl)), 0) != 0)
+                break;
+            if (__ballot_sync(kAll, w.cur > kWalkReturn) == 0u)
+                break;
+            continue;
+        }
+        if (walking == 0u)
+            break;
+        const int nNode = __popc(atNode), nLeaf = __popc(atLeaf), nSwitch = __popc(atSwitch);
+        if (nSwitch >= nNode && nSwitch >= nLeaf)
+        {
+            if ((atSwitch >> lane_id()) & 1u)
+            {
+                const float4 o = worldO[threadIdx.x], d = worldD[threadIdx.x];
+                ray = make_ray(v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), 0.0f, FLT_MAX);
+                if (w.cur == kWalkReturn)
+                {
+                    w.base = 0;
+                    w.inst = -1;
+                    wide_pop(h, w, stack);
+                }
+                if (w.cur < 0 && w.cur > kWalkReturn)
+                {
+                    // the first instance of the leaf; the others wait on the stack
+                    const int code = ~w.cur;
+                    const int k = code >> kLeafCountBits;
+                    const int count = code & ((1 << kLeafCountBits) - 1);
+                    if (count > 1)
+                        stack.put(w.sp++, make_int2(~(((k + 1) << kLeafCountBits) | (count - 1)), 0));
+                    w.base = w.sp;
+                    w.inst = k;
+                    skips[threadIdx.x] = __float_as_int(d.w) == k ? __float_as_int(o.w) : -1;
+                    ray = instance_ray(load_instance(p.scene0.instances, k), ray);
+                    w.cur = __ldg(p.scene0.instWide + k);
+                }
+            }
+        }
+        else if (nLeaf > nNode)
+        {
+            if ((atLeaf >> lane_id()) & 1u)
+            {
+                const float t0 = h.t;
+                const int s0 = h.slot;
+                wide_leaf_step(p.scene0.tris, ray, h, w, stack, skips[threadIdx.x]);
+                if (h.t != t0 || h.slot != s0)
+                    hitInst[threadIdx.x] = w.inst;
+            }
+        }
+        else if (w.cur >= 0)
+            wide_node_step(w.inst >= 0 ? p.scene0.wide : p.scene0.wideTlas, ray, h, w, stack, err);
     }
     flush_extend_counts(p, lane_id() == 0 ? done : 0u, TravCount{ 0, 0 }, err);
     if (watched && lane_id() == 0)
@@ -1183,6 +1340,20 @@ cudaError_t bounce_paths_t(const PassParams& p, int first, int block, cudaStream
     return bounce_paths_b<128, false, true>(p, first, stream, numSMs);
 }
 
+template <bool NRC>
+cudaError_t bounce_inst_b(const PassParams& p, int first, cudaStream_t stream, int numSMs)
+{
+    auto k = k_bounce_instanced<NRC>;
+    static OccupancyCache occ;
+    k<<<persistent_blocks(k, 128, numSMs, occ), 128, 0, stream>>>(p, first);
+    return cudaGetLastError();
+}
+
+cudaError_t bounce_inst(const PassParams& p, int first, cudaStream_t stream, int numSMs)
+{
+    return p.nrc.query ? bounce_inst_b<true>(p, first, stream, numSMs) : bounce_inst_b<false>(p, first, stream, numSMs);
+}
+
 // The block sizes of the kernels it replaces: the autotuned extend block for
 // plain passes, 128 threads for cache passes.
 cudaError_t extend_shade_t(const PassParams& p, int segment, int block, cudaStream_t stream, int numSMs)
@@ -1270,11 +1441,11 @@ __global__ void __launch_bounds__(256) k_nrc_targets(PassParams p)
     }
 }
 
-// Uncounted nearest-first passes over a 4-wide tree trace and shade in one
-// kernel: one launch for the camera rays, one for all later segments.
+// Uncounted nearest-first passes over 4-wide trees: one launch for the camera
+// rays (two-level scenes: extend and shade apart), one for all later segments.
 bool fused_pass(const PassParams& p, int order, int counting)
 {
-    return !p.instanced && order == ORDER_NEAREST && !counting && p.wide && !extend_refill() && extend_shade_fused();
+    return order == ORDER_NEAREST && !counting && p.wide && !extend_refill() && extend_shade_fused();
 }
 
 // Lanes per path of a one-scene pass, or 0 for one path per lane: the largest
@@ -1286,7 +1457,7 @@ bool fused_pass(const PassParams& p, int order, int counting)
 unsigned path_group_lanes(const PassParams& p, int order, int counting, int numSMs)
 {
     constexpr int rounds = 2;
-    if (!p.singleScene || !fused_pass(p, order, counting) || p.segments < 1)
+    if (!p.singleScene || p.instanced || !fused_pass(p, order, counting) || p.segments < 1)
         return 0u;
     static OccupancyCache occ;
     const int64_t lanes = int64_t(persistent_blocks(k_path_group<true>, 128, numSMs, occ)) * 128;
@@ -1341,8 +1512,13 @@ cudaError_t launch_path_segments(const PassParams& p, int order, int counting, c
             return e;
         if (fused)
         {
-            e = seg == 0 ? extend_shade_t(p, seg, shape.extendBlock, stream, numSMs)
-                         : bounce_paths_t(p, seg, shape.extendBlock, stream, numSMs);
+            if (seg > 0)
+                e = p.instanced ? bounce_inst(p, seg, stream, numSMs)
+                                : bounce_paths_t(p, seg, shape.extendBlock, stream, numSMs);
+            else if (!p.instanced)
+                e = extend_shade_t(p, seg, shape.extendBlock, stream, numSMs);
+            else if ((e = extend_inst<false>(p, seg, stream, numSMs)) == cudaSuccess)
+                e = shade_t(p, seg, shape.shadeBlock, stream, numSMs);
             if (e != cudaSuccess)
                 return e;
             if (extendEvents && (e = cudaEventRecord(extendEvents[2 * seg + 1], stream)) != cudaSuccess)

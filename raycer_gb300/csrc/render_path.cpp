@@ -160,6 +160,9 @@ PathScene path_scene(const rc_tracer* h, uint64_t pixelStart)
     ps.sc.tlasRoot = h->tlasRoot;
     ps.sc.numInstances = int(h->nInstances);
     ps.sc.wide = h->dWide;
+    ps.sc.wideTlas = h->dWideTlas;
+    ps.sc.instWide = h->dInstWide;
+    ps.sc.wideTlasRoot = h->wideTlasRoot;
     ps.sc.wideRoot = h->wideRoot;
     for (int k = 0; k < 3; ++k)
     {
@@ -269,7 +272,7 @@ rc_status render_path(rc_tracer* h, uint64_t pixelStart, uint64_t count, RenderW
     pp.numChunks = 1;
     pp.segments = g.max_path_length;
     pp.instanced = h->nInstances > 0 ? 1 : 0;
-    pp.wide = h->dWide != nullptr && h->nInstances == 0 ? 1 : 0;
+    pp.wide = h->nInstances > 0 ? (h->wideInstanced ? 1 : 0) : (h->dWide != nullptr ? 1 : 0);
     pp.singleScene = 1;
     pp.scene0 = ps.sc;
     if (watch)

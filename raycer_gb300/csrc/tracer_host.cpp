@@ -115,6 +115,11 @@ void release_scene(rc_tracer* h)
     dev_free(h, &h->dInstances, size_t(h->nInstances));
     dev_free(h, &h->dWide, h->wideCount);
     h->wideCount = 0;
+    dev_free(h, &h->dWideTlas, h->wideTlasCount);
+    h->wideTlasCount = 0;
+    dev_free(h, &h->dInstWide, h->instRoots.size());
+    h->instRoots.clear();
+    h->wideInstanced = false;
     h->wideRoot = 0;
     h->wideTried = false;
     dev_free(h, &h->dRopes, h->ropeCount);

@@ -384,6 +384,7 @@ struct WideWalk
 {
     int cur;
     int sp;
+    __device__ __forceinline__ void abandon();
 };
 
 // A walk that is over (no leaf code has this value: a leaf's last triangle
@@ -396,7 +397,10 @@ constexpr int kWalkNone = -0x7fffffff;
 // A walk's stack in local memory.
 struct LocalStack
 {
+    static constexpr int kEntries = kMaxStack;
     int2* e;
+    static constexpr int kNear = kMaxStack;
+    __device__ __forceinline__ void putNear(int i, int2 v) { e[i] = v; }
     __device__ __forceinline__ void put(int i, int2 v) { e[i] = v; }
     __device__ __forceinline__ int2 get(int i) const { return e[i]; }
 };
@@ -404,9 +408,12 @@ struct LocalStack
 // A walk's stack with its first D entries in shared memory, entry i of the
 // block's threads side by side (a warp's accesses meet no bank twice, whatever
 // the depths), the rest in local memory.
-template <int D, int THREADS>
+template <int D, int THREADS, int ENTRIES = kMaxStack>
 struct SharedStack
 {
+    static constexpr int kEntries = ENTRIES;
+    static constexpr int kNear = D;
+    __device__ __forceinline__ void putNear(int i, int2 v) { near[i * THREADS] = v; }
     int2* near;  // this thread's entry 0
     int2* far;
     __device__ __forceinline__ void put(int i, int2 v)
@@ -418,6 +425,12 @@ struct SharedStack
     }
     __device__ __forceinline__ int2 get(int i) const { return i < D ? near[i * THREADS] : far[i - D]; }
 };
+
+__device__ __forceinline__ void WideWalk::abandon()
+{
+    sp = 0;
+    cur = kWalkDone;
+}
 
 // Pops the next stack entry still within the current hit, or ends the walk.
 template <typename Stack>
@@ -436,9 +449,9 @@ __device__ __forceinline__ void wide_pop(const HitF& hit, WideWalk& w, const Sta
 // Node step of the 4-wide walk (w.cur >= 0): enters the nearest child hit
 // within the current closest distance and pushes the others; with none hit,
 // pops. On stack overflow err = 1 and the walk is over.
-template <typename Stack>
-__device__ __forceinline__ void wide_node_step(const DevNode4* __restrict__ wide, const RayF& ray, HitF& hit,
-                                               WideWalk& w, Stack& stack, int& err)
+template <typename Walk, typename Stack>
+__device__ __forceinline__ void wide_node_step(const DevNode4* __restrict__ wide, const RayF& ray, HitF& hit, Walk& w,
+                                               Stack& stack, int& err)
 {
     const float kInf = __int_as_float(0x7f800000);
     const float4* p = reinterpret_cast<const float4*>(wide + w.cur);
@@ -489,12 +502,23 @@ __device__ __forceinline__ void wide_node_step(const DevNode4* __restrict__ wide
     wide_cswap(d1, l1, d2, l2);
     if (d0 < kInf)
     {
-        if (w.sp > kMaxStack - 3 &&
-            w.sp + (d1 < kInf ? 1 : 0) + (d2 < kInf ? 1 : 0) + (d3 < kInf ? 1 : 0) > kMaxStack)
+        // room for three in the near entries: no test per entry
+        if (w.sp <= Stack::kNear - 3)
+        {
+            if (d3 < kInf)
+                stack.putNear(w.sp++, make_int2(l3, __float_as_int(d3)));
+            if (d2 < kInf)
+                stack.putNear(w.sp++, make_int2(l2, __float_as_int(d2)));
+            if (d1 < kInf)
+                stack.putNear(w.sp++, make_int2(l1, __float_as_int(d1)));
+            w.cur = l0;
+            return;
+        }
+        if (w.sp > Stack::kEntries - 3 &&
+            w.sp + (d1 < kInf ? 1 : 0) + (d2 < kInf ? 1 : 0) + (d3 < kInf ? 1 : 0) > Stack::kEntries)
         {
             err = 1;
-            w.sp = 0;
-            w.cur = kWalkDone;
+            w.abandon();
             return;
         }
         if (d3 < kInf)
@@ -533,8 +557,8 @@ __device__ __forceinline__ void wide_leaf_test(const RayF& ray, HitF& hit, int s
 // of the tests. (Both triangles at once in two-wide arithmetic, from records
 // of interleaved pairs: no faster, for 8 more registers and 60 MB per 1M
 // triangles.)
-template <typename Stack>
-__device__ __forceinline__ void wide_leaf_step(const DevTri* __restrict__ tris, const RayF& ray, HitF& hit, WideWalk& w,
+template <typename Walk, typename Stack>
+__device__ __forceinline__ void wide_leaf_step(const DevTri* __restrict__ tris, const RayF& ray, HitF& hit, Walk& w,
                                                const Stack& stack, int skip)
 {
     const int leaf = ~w.cur;
@@ -552,6 +576,38 @@ __device__ __forceinline__ void wide_leaf_step(const DevTri* __restrict__ tris, 
         w.cur = ~(((s0 + 2) << kLeafCountBits) | (count - 2));
     else
         wide_pop(hit, w, stack);
+}
+
+// A walk of a two-level scene: the top-level tree over the instances (inst =
+// -1) or an instance's mesh, whose entries lie above `base` of one stack. At
+// the top level a leaf code names instances.
+constexpr int kWalkReturn = -0x7ffffffe;  // the mesh is done (no leaf code: 13 triangles would start at the last slot)
+
+struct TwoLevelWalk
+{
+    int cur;
+    int sp;
+    int base;
+    int inst;
+    __device__ __forceinline__ void abandon()
+    {
+        sp = base = 0;
+        inst = -1;
+        cur = kWalkDone;
+    }
+};
+
+template <typename Stack>
+__device__ __forceinline__ void wide_pop(const HitF& hit, TwoLevelWalk& w, const Stack& stack)
+{
+    while (w.sp > w.base)
+    {
+        const int2 e = stack.get(--w.sp);
+        w.cur = e.x;
+        if (!(__int_as_float(e.y) > hit.t))
+            return;
+    }
+    w.cur = w.inst >= 0 ? kWalkReturn : kWalkDone;
 }
 
 // One step of the 4-wide walk, a node's or a leaf's. Returns true when the

@@ -1,5 +1,6 @@
-// 4-wide BVH of a single-level scene, collapsed on the device from its binary
-// nodes at the scene's first use by a kernel that walks it.
+// 4-wide BVHs, collapsed on the device from a scene's binary nodes at its
+// first use by a kernel that walks them: the tree of a single-level scene, or
+// the trees of a two-level scene's meshes and the one over its instances.
 //
 // Each wide node starts from one binary node's two children and repeatedly
 // replaces its inner child of largest surface area by that child's two
@@ -28,6 +29,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <string>
+#include <vector>
 
 #include "host_internal.h"
 
@@ -158,53 +160,42 @@ __global__ void __launch_bounds__(kBlock) k_collapse(const DevNode* __restrict__
     }
 }
 
-// Level 0: the root. A later call closes the level just taken.
-__global__ void k_collapse_level(WideItem* items, WideCounters* c, int root, int level)
-{
-    if (level == 0)
-    {
-        items[0] = WideItem{ root, 0 };
-        c->nodes = 1;
-        c->bound[0] = 0;
-    }
-    c->bound[level + 1] = c->nodes;
-}
+// Closes the level just taken.
+__global__ void k_collapse_level(WideCounters* c, int level) { c->bound[level + 1] = c->nodes; }
 
-}  // namespace
-
-rc_status ensure_wide(rc_tracer* h)
+// Collapses the trees of `roots` (inner links into nodes[0, count)) into one
+// array of 4-wide nodes, root i at index i. *out stays null where the stack
+// need (*need) is above `maxNeed`.
+rc_status collapse(rc_tracer* h, const DevNode* nodes, size_t count, const std::vector<int32_t>& roots, int levels,
+                   int maxNeed, DevNode4** out, int* need)
 {
-    if (h->wideTried || !h->sceneReady || h->nInstances > 0)
-        return RC_OK;
-    h->wideTried = true;
-    h->wideRoot = h->rootLink;
-    static const bool enabled = [] {
-        const char* v = std::getenv("RC_WIDE_BVH");
-        return !(v && v[0] == '0');
-    }();
-    if (h->rootLink < 0 || !enabled)
-        return RC_OK;  // a leaf root (nothing to collapse) or switched off: binary traversal
-    const size_t maxNodes = h->innerCount;  // a wide node stands for one binary inner node
+    *out = nullptr;
     WideItem* items = nullptr;
     WideCounters* counters = nullptr;
     WideCounters got{};
-    cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&h->dWide), maxNodes * sizeof(DevNode4));
+    std::vector<WideItem> first(roots.size());
+    for (size_t i = 0; i < roots.size(); ++i)
+        first[i] = WideItem{ roots[i], 0 };
+    got.nodes = int(roots.size());
+    // a wide node stands for one binary inner node
+    cudaError_t e = cudaMalloc(reinterpret_cast<void**>(out), count * sizeof(DevNode4));
     if (e == cudaSuccess)
-        e = cudaMalloc(reinterpret_cast<void**>(&items), maxNodes * sizeof(WideItem) + sizeof(WideCounters));
+        e = cudaMalloc(reinterpret_cast<void**>(&items), count * sizeof(WideItem) + sizeof(WideCounters));
     if (e == cudaSuccess)
     {
-        counters = reinterpret_cast<WideCounters*>(items + maxNodes);
-        e = cudaMemsetAsync(counters, 0, sizeof(WideCounters), h->stream);
+        counters = reinterpret_cast<WideCounters*>(items + count);
+        e = cudaMemcpyAsync(counters, &got, sizeof(got), cudaMemcpyHostToDevice, h->stream);
     }
-    const int levels = int(std::min<uint64_t>(std::max<uint64_t>(h->bvhDepth, 1), kMaxStack));
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(items, first.data(), first.size() * sizeof(WideItem), cudaMemcpyHostToDevice, h->stream);
+    levels = std::min(std::max(levels, 1), kMaxStack);
     for (int level = 0; e == cudaSuccess && level < levels; ++level)
     {
-        k_collapse_level<<<1, 1, 0, h->stream>>>(items, counters, h->rootLink, level);
-        // at most 4^level nodes
-        const size_t most = level < 12 ? std::min(maxNodes, size_t(1) << (2 * level)) : maxNodes;
+        k_collapse_level<<<1, 1, 0, h->stream>>>(counters, level);
+        // at most 4^level nodes per root
+        const size_t most = level < 12 ? std::min(count, roots.size() << (2 * level)) : count;
         const unsigned blocks = unsigned(std::min<size_t>((most + kBlock - 1) / kBlock, size_t(h->numSMs) * 16));
-        k_collapse<<<blocks, kBlock, 0, h->stream>>>(h->dNodes, int(h->innerCount), items, h->dWide, counters,
-                                                     level);
+        k_collapse<<<blocks, kBlock, 0, h->stream>>>(nodes, int(count), items, *out, counters, level);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess)
@@ -212,26 +203,104 @@ rc_status ensure_wide(rc_tracer* h)
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(h->stream);
     cudaFree(items);
-    if (e != cudaSuccess || got.error || got.maxNeed > kMaxStack || got.nodes != got.bound[levels])
+    if (e == cudaSuccess && !got.error && got.maxNeed <= maxNeed && got.nodes == got.bound[levels])
+    {
+        *need = got.maxNeed;
+        return RC_OK;
+    }
+    cudaGetLastError();
+    cudaFree(*out);
+    *out = nullptr;
+    if (e != cudaSuccess)
+    {
+        h->err = std::string("wide BVH: ") + cudaGetErrorString(e);
+        return e == cudaErrorMemoryAllocation ? RC_OOM : RC_CUDA;
+    }
+    if (got.error)
+    {
+        h->err = "wide BVH: malformed binary node links";
+        return RC_DEVICE_ERROR;
+    }
+    return RC_OK;  // stays binary
+}
+
+// The meshes' trees, the top-level one and the instances' mesh roots.
+rc_status ensure_wide_instanced(rc_tracer* h)
+{
+    std::vector<int32_t> roots;  // inner mesh roots, each once
+    for (int32_t r : h->instRoots)
+        if (r >= 0)
+            roots.push_back(r);
+    std::sort(roots.begin(), roots.end());
+    roots.erase(std::unique(roots.begin(), roots.end()), roots.end());
+    std::vector<int32_t> wideRoots;
+    for (int32_t r : h->instRoots)
+        wideRoots.push_back(
+            r < 0 ? r : int32_t(std::lower_bound(roots.begin(), roots.end(), r) - roots.begin()));
+    const int levels = int(std::min<uint64_t>(h->bvhDepth, kMaxStack));
+    int needMesh = 0, needTop = 0;
+    rc_status s = RC_OK;
+    if (!roots.empty() &&
+        ((s = collapse(h, h->dNodes, h->innerCount, roots, levels, kTwoLevelStack, &h->dWide, &needMesh)) != RC_OK ||
+         !h->dWide))
+        return s;
+    h->wideCount = h->dWide ? h->innerCount : 0;
+    h->deviceBytes += h->wideCount * sizeof(DevNode4);
+    h->wideTlasRoot = h->tlasRoot;
+    if (h->tlasRoot >= 0)
+    {
+        s = collapse(h, h->dTlas, h->tlasCount, { h->tlasRoot }, levels, kTwoLevelStack, &h->dWideTlas, &needTop);
+        if (s != RC_OK || !h->dWideTlas)
+            return s;
+        h->wideTlasRoot = 0;
+        h->wideTlasCount = h->tlasCount;
+        h->deviceBytes += h->wideTlasCount * sizeof(DevNode4);
+    }
+    // a leaf of two instances stacks its second one
+    if (needMesh + needTop + 1 > kTwoLevelStack)
+        return RC_OK;  // stays binary
+    cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&h->dInstWide), wideRoots.size() * sizeof(int32_t));
+    if (e == cudaSuccess)
+    {
+        h->deviceBytes += wideRoots.size() * sizeof(int32_t);
+        e = cudaMemcpy(h->dInstWide, wideRoots.data(), wideRoots.size() * sizeof(int32_t), cudaMemcpyHostToDevice);
+    }
+    if (e != cudaSuccess)
     {
         cudaGetLastError();
-        cudaFree(h->dWide);
-        h->dWide = nullptr;
-        if (e != cudaSuccess)
-        {
-            h->err = std::string("wide BVH: ") + cudaGetErrorString(e);
-            return e == cudaErrorMemoryAllocation ? RC_OOM : RC_CUDA;
-        }
-        if (got.error)
-        {
-            h->err = "wide BVH: malformed binary node links";
-            return RC_DEVICE_ERROR;
-        }
-        return RC_OK;  // stays binary
+        h->err = std::string("wide BVH: ") + cudaGetErrorString(e);
+        return e == cudaErrorMemoryAllocation ? RC_OOM : RC_CUDA;
     }
-    h->wideCount = maxNodes;
+    h->wideInstanced = true;
+    return RC_OK;
+}
+
+}  // namespace
+
+rc_status ensure_wide(rc_tracer* h)
+{
+    if (h->wideTried || !h->sceneReady)
+        return RC_OK;
+    h->wideTried = true;
+    h->wideRoot = h->rootLink;
+    static const bool enabled = [] {
+        const char* v = std::getenv("RC_WIDE_BVH");
+        return !(v && v[0] == '0');
+    }();
+    if (!enabled)
+        return RC_OK;
+    if (h->nInstances > 0)
+        return ensure_wide_instanced(h);
+    if (h->rootLink < 0)
+        return RC_OK;  // a leaf root: nothing to collapse
+    int need = 0;
+    const rc_status s = collapse(h, h->dNodes, h->innerCount, { h->rootLink }, int(h->bvhDepth), kMaxStack, &h->dWide,
+                                 &need);
+    if (s != RC_OK || !h->dWide)
+        return s;
+    h->wideCount = h->innerCount;
     h->wideRoot = 0;
-    h->deviceBytes += maxNodes * sizeof(DevNode4);
+    h->deviceBytes += h->wideCount * sizeof(DevNode4);
     return RC_OK;
 }
 
