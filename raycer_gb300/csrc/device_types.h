@@ -35,7 +35,7 @@
 namespace rcx
 {
 
-struct __align__(16) DevNode
+struct __align__(32) DevNode
 {
     float4 xy0;  // child 0: lo.x, hi.x, lo.y, hi.y
     float4 xy1;  // child 1: lo.x, hi.x, lo.y, hi.y

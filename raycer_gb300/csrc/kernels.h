@@ -97,6 +97,10 @@ int blocks_per_sm(K kernel, int block, size_t smem, OccupancyCache& cache)
 // use while this is on).
 bool stackless_walk();
 
+// Whether launch_cast of this call walks the scene's 4-wide tree where there
+// is one (the host builds it on first use).
+bool cast_walks_wide(const LaunchInfo& li, const DevScene& sc, int64_t n, int anyHit, int order);
+
 // Generic ray queries (rc_ray -> rc_hit).
 cudaError_t launch_cast(const LaunchInfo& li, const DevScene& sc, const rc_ray* rays, int64_t n, int anyHit,
                         int order, rc_hit* hits, DevControl* ctl);

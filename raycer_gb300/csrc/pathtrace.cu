@@ -1443,10 +1443,12 @@ __global__ void __launch_bounds__(256) k_nrc_targets(PassParams p)
 
 // Uncounted nearest-first passes over 4-wide trees: one launch for the camera
 // rays (two-level scenes: extend and shade apart), one for all later segments.
-bool fused_pass(const PassParams& p, int order, int counting)
+bool one_kernel_pass(int order, int counting)
 {
-    return order == ORDER_NEAREST && !counting && p.wide && !extend_refill() && extend_shade_fused();
+    return order == ORDER_NEAREST && !counting && !extend_refill() && extend_shade_fused();
 }
+
+bool fused_pass(const PassParams& p, int order, int counting) { return one_kernel_pass(order, counting) && p.wide; }
 
 // Lanes per path of a one-scene pass, or 0 for one path per lane: the largest
 // group whose two rounds of one path per group (four for groups of 4) cover
@@ -1457,7 +1459,7 @@ bool fused_pass(const PassParams& p, int order, int counting)
 unsigned path_group_lanes(const PassParams& p, int order, int counting, int numSMs)
 {
     constexpr int rounds = 2;
-    if (!p.singleScene || p.instanced || !fused_pass(p, order, counting) || p.segments < 1)
+    if (!p.singleScene || p.instanced || !one_kernel_pass(order, counting) || p.segments < 1 || p.scene0.rootLink < 0)
         return 0u;
     static OccupancyCache occ;
     const int64_t lanes = int64_t(persistent_blocks(k_path_group<true>, 128, numSMs, occ)) * 128;
@@ -1478,9 +1480,14 @@ cudaError_t path_group_b(const PassParams& p, unsigned G, cudaStream_t stream, i
 
 }  // namespace
 
+bool path_walks_wide(const PassParams& p, int order, int counting, int numSMs)
+{
+    return path_group_lanes(p, order, counting, numSMs) == 0u;
+}
+
 int path_extend_launches(const PassParams& p, int order, int counting)
 {
-    return fused_pass(p, order, counting) ? std::min(p.segments, 2) : p.segments;
+    return std::min(p.segments, p.small ? 1 : fused_pass(p, order, counting) ? 2 : p.segments);
 }
 
 cudaError_t launch_path_segments(const PassParams& p, int order, int counting, const PassShape& shape,
@@ -1490,9 +1497,9 @@ cudaError_t launch_path_segments(const PassParams& p, int order, int counting, c
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
         return e;
+    const unsigned G = path_group_lanes(p, order, counting, numSMs);
     const bool fused = fused_pass(p, order, counting);
     const int launches = path_extend_launches(p, order, counting);
-    const unsigned G = path_group_lanes(p, order, counting, numSMs);
     if (G)
     {
         if (extendEvents && (e = cudaEventRecord(extendEvents[0], stream)) != cudaSuccess)

@@ -102,6 +102,7 @@ struct PassParams
     NrcPass nrc;
     int instanced;   // 1: the pass has two-level scenes (k_extend_instanced)
     int wide;        // 1: every scene of the pass has its 4-wide BVH (uncounted nearest-first extend uses it)
+    int small = 0;        // 1: the render's largest pass is walked by groups of lanes (path_walks_wide false)
     int singleScene = 0;  // 1: every slot of the pass is scene0's (a one-scene render), so the
                           // extend kernels read the scene record from the parameters, not the table
     DevScene scene0;
@@ -123,8 +124,12 @@ struct PassShape
     int shadeBlock = 128;
 };
 
+// Whether a pass (nslots, scene0 and the like set) walks the 4-wide trees
+// where there are any; a small one does not.
+bool path_walks_wide(const PassParams& p, int order, int counting, int numSMs);
 // Extend launches of a pass: one per segment, or, where extend and shade run
-// as one kernel, one for the camera rays and one for all later segments.
+// as one kernel, one for the camera rays and one for all later segments (a
+// render of small passes: one).
 int path_extend_launches(const PassParams& p, int order, int counting);
 // Launch the kernels of one pass (generate, the segments, accumulate) on
 // `stream`. extendEvents: 2 * path_extend_launches() events recorded around

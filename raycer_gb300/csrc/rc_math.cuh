@@ -185,6 +185,19 @@ __device__ __forceinline__ float fmax3(float a, float b, float c)
     return r;
 }
 
+// slab_finite with each axis's two planes in two-wide arithmetic and
+// three-input min/max: the same decision and entry distance.
+__device__ __forceinline__ bool slab_finite2(const RayF& r, float lox, float hix, float loy, float hiy, float loz,
+                                             float hiz, float& entry)
+{
+    const F2 x = mul2(add2(f2(lox, hix), f2(-r.o.x, -r.o.x)), f2(r.inv.x, r.inv.x));
+    const F2 y = mul2(add2(f2(loy, hiy), f2(-r.o.y, -r.o.y)), f2(r.inv.y, r.inv.y));
+    const F2 z = mul2(add2(f2(loz, hiz), f2(-r.o.z, -r.o.z)), f2(r.inv.z, r.inv.z));
+    entry = fmaxf(fmax3(fminf(f2_lo(x), f2_hi(x)), fminf(f2_lo(y), f2_hi(y)), fminf(f2_lo(z), f2_hi(z))), 0.0f);
+    const float tmax = fmin3(fmaxf(f2_lo(x), f2_hi(x)), fmaxf(f2_lo(y), f2_hi(y)), fmaxf(f2_lo(z), f2_hi(z)));
+    return !(tmax < entry);
+}
+
 // Sign octant of a ray's inverse direction (slab_oct's OCT), or -1 when a
 // component is not finite (slab_oct does not apply).
 __device__ __forceinline__ int ray_octant(const RayF& r)

@@ -216,11 +216,6 @@ rc_status render_path(rc_tracer* h, uint64_t pixelStart, uint64_t count, RenderW
 {
     const volatile int32_t* cancel = watch ? watch->cancel : nullptr;
     const rc_general& g = h->general;
-    {
-        rc_status ws = ensure_wide(h);
-        if (ws != RC_OK)
-            return ws;
-    }
     const uint64_t spp = uint64_t(g.multi_sample_count_sqrt) * uint64_t(g.multi_sample_count_sqrt) *
                          uint64_t(g.path_sample_count);
     if (spp > kTargetSlots)
@@ -228,6 +223,20 @@ rc_status render_path(rc_tracer* h, uint64_t pixelStart, uint64_t count, RenderW
     const uint64_t pixelsPerPass = std::max<uint64_t>(1, kTargetSlots / spp);
     const uint64_t slots = std::min<uint64_t>(pixelsPerPass, count) * spp;
     const uint64_t passes = (count + pixelsPerPass - 1) / pixelsPerPass;
+    bool small = false;
+    {
+        // the first pass is the largest
+        PassParams probe{};
+        probe.nslots = int(slots);
+        probe.segments = g.max_path_length;
+        probe.instanced = h->nInstances > 0 ? 1 : 0;
+        probe.singleScene = 1;
+        probe.scene0 = path_scene(h, pixelStart).sc;
+        small = !path_walks_wide(probe, h->order, h->counting, h->numSMs);
+        const rc_status ws = small ? RC_OK : ensure_wide(h);
+        if (ws != RC_OK)
+            return ws;
+    }
 
     if (h->pathSlots < slots)
     {
@@ -273,6 +282,7 @@ rc_status render_path(rc_tracer* h, uint64_t pixelStart, uint64_t count, RenderW
     pp.segments = g.max_path_length;
     pp.instanced = h->nInstances > 0 ? 1 : 0;
     pp.wide = h->nInstances > 0 ? (h->wideInstanced ? 1 : 0) : (h->dWide != nullptr ? 1 : 0);
+    pp.small = small ? 1 : 0;
     pp.singleScene = 1;
     pp.scene0 = ps.sc;
     if (watch)

@@ -1063,6 +1063,8 @@ rc_status rc_cast_device(rc_tracer* h, const rc_ray* d_rays, int64_t n, int32_t 
         return fail(h, RC_INVALID_ARG, "cast: invalid traversal order");
     cudaSetDevice(h->device);
     rc_status s = stackless_walk() ? ensure_ropes(h) : RC_OK;
+    if (s == RC_OK && cast_walks_wide(launch_info(h), dev_scene(h), n, any_hit, order))
+        s = ensure_wide(h);
     if (s != RC_OK)
         return s;
     s = begin_launch(h);

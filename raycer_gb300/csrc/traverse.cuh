@@ -385,6 +385,11 @@ struct WideWalk
     int cur;
     int sp;
     __device__ __forceinline__ void abandon();
+    // boxes entered beyond this are skipped
+    __device__ __forceinline__ float limit(const HitF& hit) const { return hit.t; }
+    // the box of `cur` was entered at e; the hit lies in it
+    __device__ __forceinline__ void entered(float) {}
+    __device__ __forceinline__ void accepted() {}
 };
 
 // A walk that is over (no leaf code has this value: a leaf's last triangle
@@ -408,22 +413,22 @@ struct LocalStack
 // A walk's stack with its first D entries in shared memory, entry i of the
 // block's threads side by side (a warp's accesses meet no bank twice, whatever
 // the depths), the rest in local memory.
-template <int D, int THREADS, int ENTRIES = kMaxStack>
+template <int D, int THREADS, int ENTRIES = kMaxStack, typename Entry = int2>
 struct SharedStack
 {
     static constexpr int kEntries = ENTRIES;
     static constexpr int kNear = D;
-    __device__ __forceinline__ void putNear(int i, int2 v) { near[i * THREADS] = v; }
-    int2* near;  // this thread's entry 0
-    int2* far;
-    __device__ __forceinline__ void put(int i, int2 v)
+    __device__ __forceinline__ void putNear(int i, Entry v) { near[i * THREADS] = v; }
+    Entry* near;  // this thread's entry 0
+    Entry* far;
+    __device__ __forceinline__ void put(int i, Entry v)
     {
         if (i < D)
             near[i * THREADS] = v;
         else
             far[i - D] = v;
     }
-    __device__ __forceinline__ int2 get(int i) const { return i < D ? near[i * THREADS] : far[i - D]; }
+    __device__ __forceinline__ Entry get(int i) const { return i < D ? near[i * THREADS] : far[i - D]; }
 };
 
 __device__ __forceinline__ void WideWalk::abandon()
@@ -432,16 +437,41 @@ __device__ __forceinline__ void WideWalk::abandon()
     cur = kWalkDone;
 }
 
+// How far past the current closest hit a walk goes that must meet every box
+// which could decide a tie (see traverse_group).
+constexpr float kTieCull = 1.01f;
+
+// A walk whose hit is reported (rc_cast): it keeps the entry distance of the
+// hit's leaf and skips boxes only past kTieCull times the hit.
+struct CastWalk
+{
+    int cur;
+    int sp;
+    float entry;     // of cur
+    float hitEntry;  // of the hit's leaf
+    __device__ __forceinline__ void abandon()
+    {
+        sp = 0;
+        cur = kWalkDone;
+    }
+    __device__ __forceinline__ float limit(const HitF& hit) const { return hit.t * kTieCull; }
+    __device__ __forceinline__ void entered(float e) { entry = e; }
+    __device__ __forceinline__ void accepted() { hitEntry = entry; }
+};
+
 // Pops the next stack entry still within the current hit, or ends the walk.
-template <typename Stack>
-__device__ __forceinline__ void wide_pop(const HitF& hit, WideWalk& w, const Stack& stack)
+template <typename Walk, typename Stack>
+__device__ __forceinline__ void wide_pop(const HitF& hit, Walk& w, const Stack& stack)
 {
     while (w.sp > 0)
     {
         const int2 e = stack.get(--w.sp);
         w.cur = e.x;
-        if (!(__int_as_float(e.y) > hit.t))
+        if (!(__int_as_float(e.y) > w.limit(hit)))
+        {
+            w.entered(__int_as_float(e.y));
             return;
+        }
     }
     w.cur = kWalkDone;
 }
@@ -462,6 +492,7 @@ __device__ __forceinline__ void wide_node_step(const DevNode4* __restrict__ wide
     ldg32(p + 6, lf, mf);
     const int4 l = make_int4(__float_as_int(lf.x), __float_as_int(lf.y), __float_as_int(lf.z), __float_as_int(lf.w));
     const int nc = __float_as_int(mf.x);
+    const float limit = w.limit(hit);
     float d0, d1, d2, d3;
     if (ray.finite)
     {
@@ -472,23 +503,23 @@ __device__ __forceinline__ void wide_node_step(const DevNode4* __restrict__ wide
             const F2 x0 = plane2(lox.x, lox.y, X), x1 = plane2(hix.x, hix.y, X);
             const F2 y0 = plane2(loy.x, loy.y, Y), y1 = plane2(hiy.x, hiy.y, Y);
             const F2 z0 = plane2(loz.x, loz.y, Z), z1 = plane2(hiz.x, hiz.y, Z);
-            d0 = wide_entry_of(f2_lo(x0), f2_lo(x1), f2_lo(y0), f2_lo(y1), f2_lo(z0), f2_lo(z1), hit.t);
-            d1 = wide_entry_of(f2_hi(x0), f2_hi(x1), f2_hi(y0), f2_hi(y1), f2_hi(z0), f2_hi(z1), hit.t);
+            d0 = wide_entry_of(f2_lo(x0), f2_lo(x1), f2_lo(y0), f2_lo(y1), f2_lo(z0), f2_lo(z1), limit);
+            d1 = wide_entry_of(f2_hi(x0), f2_hi(x1), f2_hi(y0), f2_hi(y1), f2_hi(z0), f2_hi(z1), limit);
         }
         {
             const F2 x0 = plane2(lox.z, lox.w, X), x1 = plane2(hix.z, hix.w, X);
             const F2 y0 = plane2(loy.z, loy.w, Y), y1 = plane2(hiy.z, hiy.w, Y);
             const F2 z0 = plane2(loz.z, loz.w, Z), z1 = plane2(hiz.z, hiz.w, Z);
-            d2 = wide_entry_of(f2_lo(x0), f2_lo(x1), f2_lo(y0), f2_lo(y1), f2_lo(z0), f2_lo(z1), hit.t);
-            d3 = wide_entry_of(f2_hi(x0), f2_hi(x1), f2_hi(y0), f2_hi(y1), f2_hi(z0), f2_hi(z1), hit.t);
+            d2 = wide_entry_of(f2_lo(x0), f2_lo(x1), f2_lo(y0), f2_lo(y1), f2_lo(z0), f2_lo(z1), limit);
+            d3 = wide_entry_of(f2_hi(x0), f2_hi(x1), f2_hi(y0), f2_hi(y1), f2_hi(z0), f2_hi(z1), limit);
         }
     }
     else
     {
-        d0 = wide_entry(ray, lox.x, hix.x, loy.x, hiy.x, loz.x, hiz.x, hit.t);
-        d1 = wide_entry(ray, lox.y, hix.y, loy.y, hiy.y, loz.y, hiz.y, hit.t);
-        d2 = wide_entry(ray, lox.z, hix.z, loy.z, hiy.z, loz.z, hiz.z, hit.t);
-        d3 = wide_entry(ray, lox.w, hix.w, loy.w, hiy.w, loz.w, hiz.w, hit.t);
+        d0 = wide_entry(ray, lox.x, hix.x, loy.x, hiy.x, loz.x, hiz.x, limit);
+        d1 = wide_entry(ray, lox.y, hix.y, loy.y, hiy.y, loz.y, hiz.y, limit);
+        d2 = wide_entry(ray, lox.z, hix.z, loy.z, hiy.z, loz.z, hiz.z, limit);
+        d3 = wide_entry(ray, lox.w, hix.w, loy.w, hiy.w, loz.w, hiz.w, limit);
     }
     if (nc < 3)
         d2 = kInf;
@@ -512,6 +543,7 @@ __device__ __forceinline__ void wide_node_step(const DevNode4* __restrict__ wide
             if (d1 < kInf)
                 stack.putNear(w.sp++, make_int2(l1, __float_as_int(d1)));
             w.cur = l0;
+            w.entered(d0);
             return;
         }
         if (w.sp > Stack::kEntries - 3 &&
@@ -528,14 +560,16 @@ __device__ __forceinline__ void wide_node_step(const DevNode4* __restrict__ wide
         if (d1 < kInf)
             stack.put(w.sp++, make_int2(l1, __float_as_int(d1)));
         w.cur = l0;
+        w.entered(d0);
         return;
     }
     wide_pop(hit, w, stack);
 }
 
 // The closest-hit test of one leaf triangle in the 4-wide walk.
-__device__ __forceinline__ void wide_leaf_test(const RayF& ray, HitF& hit, int slot, int skip, const float4& ta,
-                                               const float4& tb, const float4& tc)
+template <typename Walk>
+__device__ __forceinline__ void wide_leaf_test(const RayF& ray, HitF& hit, Walk& w, int slot, int skip,
+                                               const float4& ta, const float4& tb, const float4& tc)
 {
     if (slot == skip)
         return;
@@ -547,6 +581,7 @@ __device__ __forceinline__ void wide_leaf_test(const RayF& ray, HitF& hit, int s
         hit.t = t;
         hit.u = u;
         hit.v = v;
+        w.accepted();
     }
 }
 
@@ -569,9 +604,9 @@ __device__ __forceinline__ void wide_leaf_step(const DevTri* __restrict__ tris, 
     const float4* p1 = reinterpret_cast<const float4*>(tris + s1);
     const float4 a0 = __ldg(p0 + 0), b0 = __ldg(p0 + 1), c0 = __ldg(p0 + 2);
     const float4 a1 = __ldg(p1 + 0), b1 = __ldg(p1 + 1), c1 = __ldg(p1 + 2);
-    wide_leaf_test(ray, hit, s0, skip, a0, b0, c0);
+    wide_leaf_test(ray, hit, w, s0, skip, a0, b0, c0);
     if (count > 1)
-        wide_leaf_test(ray, hit, s1, skip, a1, b1, c1);
+        wide_leaf_test(ray, hit, w, s1, skip, a1, b1, c1);
     if (count > 2)
         w.cur = ~(((s0 + 2) << kLeafCountBits) | (count - 2));
     else
@@ -595,6 +630,9 @@ struct TwoLevelWalk
         inst = -1;
         cur = kWalkDone;
     }
+    __device__ __forceinline__ float limit(const HitF& hit) const { return hit.t; }
+    __device__ __forceinline__ void entered(float) {}
+    __device__ __forceinline__ void accepted() {}
 };
 
 template <typename Stack>
@@ -621,6 +659,73 @@ __device__ __forceinline__ bool wide_step(const DevNode4* __restrict__ wide, con
     else
         wide_leaf_step(tris, ray, hit, w, stack, skip);
     return w.cur == kWalkDone;
+}
+
+// Steps of the binary tree's walk in the reference's order, for warps that
+// take one phase at a time: the boxes and triangles of traverse<ANY_HIT,
+// ORDER_REF>, in its order. Stack entries are links.
+struct RefWalk
+{
+    int cur;
+    int sp;
+};
+
+template <typename Stack>
+__device__ __forceinline__ void ref_pop(RefWalk& w, const Stack& stack)
+{
+    w.cur = w.sp > 0 ? stack.get(--w.sp) : kWalkDone;
+}
+
+template <typename Stack>
+__device__ __forceinline__ void ref_node_step(const DevNode* __restrict__ nodes, const RayF& ray, RefWalk& w, Stack& stack)
+{
+    float4 a, b, c, lf;
+    ldg32(nodes + w.cur, a, b);
+    ldg32(reinterpret_cast<const float4*>(nodes + w.cur) + 2, c, lf);
+    const int l0 = __float_as_int(lf.x), l1 = __float_as_int(lf.y);
+    float e0, e1;
+    bool h0, h1;
+    if (ray.finite)
+    {
+        h0 = slab_finite2(ray, a.x, a.y, a.z, a.w, c.x, c.y, e0);
+        h1 = slab_finite2(ray, b.x, b.y, b.z, b.w, c.z, c.w, e1);
+    }
+    else
+    {
+        h0 = slab(ray, a.x, a.y, a.z, a.w, c.x, c.y, e0);
+        h1 = slab(ray, b.x, b.y, b.z, b.w, c.z, c.w, e1);
+    }
+    if (h0 && h1)
+        stack.put(w.sp++, l1);  // no deeper than the tree, which fits the stack (checked at upload)
+    if (h0 || h1)
+        w.cur = h0 ? l0 : l1;
+    else
+        ref_pop(w, stack);
+}
+
+template <bool ANY_HIT, typename Stack>
+__device__ __forceinline__ void ref_leaf_step(const DevTri* __restrict__ tris, const RayF& ray, HitF& hit, RefWalk& w,
+                                              const Stack& stack, int skip)
+{
+    const int leaf = ~w.cur;
+    const int s0 = leaf >> kLeafCountBits;
+    const int count = leaf & ((1 << kLeafCountBits) - 1);
+    const int s1 = s0 + min(1, count - 1);
+    const float4* p0 = reinterpret_cast<const float4*>(tris + s0);
+    const float4* p1 = reinterpret_cast<const float4*>(tris + s1);
+    const float4 a0 = __ldg(p0 + 0), b0 = __ldg(p0 + 1), c0 = __ldg(p0 + 2);
+    const float4 a1 = __ldg(p1 + 0), b1 = __ldg(p1 + 1), c1 = __ldg(p1 + 2);
+    TravCount none{ 0, 0 };
+    bool found = false;
+    bool over = leaf_test<ANY_HIT, ORDER_REF, false>(ray, hit, found, none, s0, skip, a0, b0, c0);
+    if (!over && count > 1)
+        over = leaf_test<ANY_HIT, ORDER_REF, false>(ray, hit, found, none, s1, skip, a1, b1, c1);
+    if (over)
+        w.cur = kWalkDone;
+    else if (count > 2)
+        w.cur = ~(((s0 + 2) << kLeafCountBits) | (count - 2));
+    else
+        ref_pop(w, stack);
 }
 
 __device__ __forceinline__ bool traverse_wide(const DevScene& sc, const RayF& ray, HitF& hit, int& err, int skip)
@@ -798,9 +903,8 @@ __device__ __forceinline__ bool traverse_packet(const DevScene& sc, const RayF& 
 //                 triangles): if the winner lies before its own leaf's entry,
 //                 the order may have decided; if not, no walk can have skipped
 //                 it (entries grow downward, hits only come nearer). The
-//                 group itself skips boxes only past kGroupCull times the
+//                 group itself skips boxes only past kTieCull times the
 //                 current hit, so that it meets such winners.
-constexpr float kGroupCull = 1.01f;
 
 template <int ORDER>
 static __device__ __noinline__ bool traverse_alone(const DevScene& sc, const RayF& ray, HitF& hit, int skip)
@@ -937,7 +1041,7 @@ __device__ __forceinline__ bool traverse_group(const DevScene& sc, const RayF& r
             float tb = hit.t;
             for (unsigned o = 1; o < G; o <<= 1)
                 tb = fminf(tb, __shfl_xor_sync(kAll, tb, o));
-            cull = tb * kGroupCull;
+            cull = tb * kTieCull;
         }
         __syncwarp();
     }

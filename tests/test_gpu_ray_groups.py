@@ -1,5 +1,6 @@
 """Calls with few rays walk each ray with a group of 32, 16, 8 or 4 lanes
-(traverse_group); the group follows from the number of rays. Casts and RAY
+(traverse_group); the group follows from the number of rays. Larger casts walk
+one ray per lane in warp-wide phases. Casts and RAY
 frames on both sides of every line, and with a partial last warp, equal the
 float32 oracle's bit for bit in both orders, as do overlapping coplanar
 triangles (where box rounding decides ties) and rays with NaN components."""
@@ -73,7 +74,7 @@ def test_frames(width, height, order):
     assert np.array_equal(tail, ref[n - part:])
 
 
-@pytest.mark.parametrize("n", [500, 30_000])
+@pytest.mark.parametrize("n", [500, 30_000, 330_000])
 @pytest.mark.parametrize("order", ORDERS)
 def test_coplanar(n, order):
     sc = degenerate_scene("coplanar", 4)
