@@ -58,6 +58,18 @@ struct TravCount
     uint32_t tris;   // triangle tests
 };
 
+// 32 bytes of read-only memory (32-byte aligned) as one load: an L1 request
+// per lane instead of two.
+__device__ __forceinline__ void ldg32(const void* p, float4& a, float4& b)
+{
+    unsigned long long x, y, z, w;
+    asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(x), "=l"(y), "=l"(z), "=l"(w) : "l"(p));
+    a = make_float4(__uint_as_float(uint32_t(x)), __uint_as_float(uint32_t(x >> 32)), __uint_as_float(uint32_t(y)),
+                    __uint_as_float(uint32_t(y >> 32)));
+    b = make_float4(__uint_as_float(uint32_t(z)), __uint_as_float(uint32_t(z >> 32)), __uint_as_float(uint32_t(w)),
+                    __uint_as_float(uint32_t(w >> 32)));
+}
+
 __device__ __forceinline__ void load_node(const DevNode* __restrict__ nodes, int i, float4& a, float4& b, float4& c,
                                           int4& l)
 {
@@ -66,15 +78,6 @@ __device__ __forceinline__ void load_node(const DevNode* __restrict__ nodes, int
     b = __ldg(p + 1);
     c = __ldg(p + 2);
     l = __ldg(reinterpret_cast<const int4*>(p + 3));
-}
-
-// 32 bytes of read-only memory (32-byte aligned) as one load: an L1 request
-// per lane instead of two.
-__device__ __forceinline__ void ldg32(const void* p, float4& a, float4& b)
-{
-    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
-        : "l"(p));
 }
 
 // The test of one leaf triangle in traverse(): nonShadowing triangles are
@@ -687,8 +690,8 @@ __device__ __forceinline__ void ref_node_step(const DevNode* __restrict__ nodes,
     bool h0, h1;
     if (ray.finite)
     {
-        h0 = slab_finite2(ray, a.x, a.y, a.z, a.w, c.x, c.y, e0);
-        h1 = slab_finite2(ray, b.x, b.y, b.z, b.w, c.z, c.w, e1);
+        h0 = slab_finite(ray, a.x, a.y, a.z, a.w, c.x, c.y, e0);
+        h1 = slab_finite(ray, b.x, b.y, b.z, b.w, c.z, c.w, e1);
     }
     else
     {
