@@ -70,6 +70,28 @@ __device__ __forceinline__ void ldg32(const void* p, float4& a, float4& b)
                     __uint_as_float(uint32_t(w >> 32)));
 }
 
+// Pixel that the q-th of n items of a row-major range takes when the items go
+// through the film in tiles of 8x4 pixels (`line` pixels per row, counted from
+// the range's first pixel): bands of four lines, in a band tiles of eight
+// columns. The last band has the lines that are left, its last tile the
+// columns; a rest of less than a line keeps its order. A permutation of 0..n-1,
+// so no item is lost or padded whatever the width.
+__device__ __forceinline__ unsigned tile_order(unsigned q, unsigned line, unsigned n)
+{
+    const unsigned lines = n / line;
+    const unsigned band = q / (4u * line);
+    const unsigned base = band * 4u * line;
+    const unsigned h = min(4u, lines - min(lines, 4u * band));
+    const unsigned r = q - base;
+    if (r >= h * line)
+        return q;
+    const unsigned x0 = r / (8u * h) * 8u;
+    const unsigned w = min(8u, line - x0);
+    const unsigned k = r - x0 * h;
+    const unsigned y = k / w;
+    return base + y * line + x0 + (k - y * w);
+}
+
 __device__ __forceinline__ void load_node(const DevNode* __restrict__ nodes, int i, float4& a, float4& b, float4& c,
                                           int4& l)
 {
