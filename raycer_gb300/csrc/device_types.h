@@ -125,6 +125,31 @@ struct RenderMonitor
 
 constexpr unsigned long long kNoBudget = ~0ull;
 
+// A range of a film's pixels in tiles of 8x4 pixels, one per warp: columns of
+// tiles (0: the range is taken in order), rows of tiles from the range's first
+// film row on, and the pixels of that row before the range.
+struct FilmTiles
+{
+    int columns = 0;
+    int rows = 0;
+    int64_t width = 0;
+    int64_t skip = 0;
+};
+
+// Tiles of `count` pixels from pixelStart on of a film `width` wide; none where
+// the range has no four lines or a line no tile.
+inline FilmTiles film_tiles(uint64_t pixelStart, int64_t count, int64_t width)
+{
+    FilmTiles t;
+    if (width < 8 || count / width < 4 || count >= (int64_t(1) << 30))
+        return t;
+    t.width = width;
+    t.skip = int64_t(pixelStart % uint64_t(width));
+    t.columns = int((width + 7) / 8);
+    t.rows = int(((t.skip + count + width - 1) / width + 3) / 4);
+    return t;
+}
+
 // Device scene handed to every kernel by value. Two-level scenes
 // (numInstances > 0) keep every mesh's BVH in `nodes` / `tris` / `shade`
 // (links already offset into the pools) and a top-level BVH over the

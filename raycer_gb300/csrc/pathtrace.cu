@@ -213,9 +213,12 @@ __global__ void __launch_bounds__(256) k_generate(PassParams p)
     p.d[s] = make_float4(d.x, d.y, d.z, __int_as_float(-1));  // w: instance the ray leaves from
     p.thr[s] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
     p.res[s] = make_float4(0.0f, 0.0f, 0.0f, w);
-    // the queue in tile order: warps of neighbouring pixels (1080p two-level
-    // frame 5.76 -> 5.61 ms)
-    p.qa[s] = int(p.tileLine ? tile_order(s, p.tileLine, uint32_t(p.nslots)) : s);
+    // the queue in tiles: warps of neighbouring pixels (1080p two-level frame
+    // 5.76 -> 5.61 ms); whole tiles only, the queue has no gaps
+    int64_t at = s;
+    if (p.tiles.columns > 0 && p.tiles.skip == 0 && p.tiles.width % 8 == 0 && p.nslots % (4 * p.tiles.width) == 0)
+        tile_pixel(p.tiles, p.nslots, s, at);
+    p.qa[s] = int(at);
 }
 
 __device__ __forceinline__ DevScene scene_of_slot(const PassParams& p, int s)
@@ -808,7 +811,7 @@ __global__ void __launch_bounds__(BLOCK) k_shade(PassParams p, int segment)
 // It runs the first segment, whose rays it makes itself (start_slot): generate
 // wrote 64 bytes of path state per slot for this kernel to read back (35 us of
 // a 1080p frame, and the loads here). With one path per pixel the warps take
-// 8x4-pixel tiles (tile_order) instead of 32 pixels of a row: nearer rays,
+// 8x4-pixel tiles (FilmTiles) instead of 32 pixels of a row: nearer rays,
 // here and in the bounce kernel, whose queue keeps the order. 1080p
 // heightfield of depth 4, device time: 1.27 ms with generate, 1.23 without,
 // 1.19 in tiles; cache frame 4.25 -> 4.21 -> 4.15. Several samples per pixel
@@ -818,7 +821,7 @@ __global__ void __launch_bounds__(BLOCK,
                                   ((NRC ? RC_EXTEND_SHADE_NRC_MIN_BLOCKS : RC_EXTEND_WIDE_MIN_BLOCKS) * 128) / BLOCK)
     k_extend_shade(PassParams p)
 {
-    const unsigned total = unsigned(p.nslots);
+    const unsigned total = unsigned(tile_items(p.tiles, p.nslots));
     unsigned* outCount = &p.counts[4];
     int err = 0;
     unsigned long long done = 0;
@@ -839,9 +842,10 @@ __global__ void __launch_bounds__(BLOCK,
         bool lookup = false;
         int s = -1;
         NrcRecord lrec;
-        if (q < total)
+        int64_t at;
+        if (tile_pixel(p.tiles, p.nslots, q, at))
         {
-            s = int(p.tileLine ? tile_order(q, p.tileLine, total) : q);
+            s = int(at);
             float4 o, d;
             start_slot<NRC, false>(p, unsigned(s), o, d);
             const DevScene sc = scene_of_slot(p, s);

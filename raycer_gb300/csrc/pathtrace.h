@@ -106,9 +106,10 @@ struct PassParams
     int singleScene = 0;  // 1: every slot of the pass is scene0's (a one-scene render), so the
                           // extend kernels read the scene record from the parameters, not the table
     DevScene scene0;
-    // Film width where the camera rays are taken in 8x4-pixel tiles (tile_order;
-    // one-scene passes with one path per pixel), 0 for slot order.
-    unsigned tileLine = 0;
+    // How the camera rays of a one-scene pass with one path per pixel are taken;
+    // two-level passes, whose tiles are the queue's order, only where every
+    // line is whole tiles.
+    FilmTiles tiles;
     RenderMonitor* monitor = nullptr;         // monitored render (rc_render): cancel word and progress, else null
     unsigned long long budgetNs = kNoBudget;  // the render's time budget (kNoBudget: none)
 };

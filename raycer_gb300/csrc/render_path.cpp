@@ -330,7 +330,8 @@ rc_status render_path(rc_tracer* h, uint64_t pixelStart, uint64_t count, RenderW
         pp.chunks = dChunks + pass;
         pp.npixels = int(chunks[pass].pixels);
         pp.nslots = int(uint64_t(chunks[pass].pixels) * spp);
-        pp.tileLine = spp == 1 && uint64_t(pp.npixels) / h->width >= 4 ? unsigned(h->width) : 0u;
+        pp.tiles = spp == 1 ? film_tiles(pixelStart + chunks[pass].pixelLocalBegin, pp.npixels, int64_t(h->width))
+                            : FilmTiles{};
         RC_CUDA_TRY(h, cudaMemsetAsync(h->dCounts, 0, countsBytes, h->stream), "reset queue counters");
         const cudaEvent_t* ev = timeStages ? h->evPool.data() + pass * passEvents : nullptr;
         if (!nrc)

@@ -70,26 +70,31 @@ __device__ __forceinline__ void ldg32(const void* p, float4& a, float4& b)
                     __uint_as_float(uint32_t(w >> 32)));
 }
 
-// Pixel that the q-th of n items of a row-major range takes when the items go
-// through the film in tiles of 8x4 pixels (`line` pixels per row, counted from
-// the range's first pixel): bands of four lines, in a band tiles of eight
-// columns. The last band has the lines that are left, its last tile the
-// columns; a rest of less than a line keeps its order. A permutation of 0..n-1,
-// so no item is lost or padded whatever the width.
-__device__ __forceinline__ unsigned tile_order(unsigned q, unsigned line, unsigned n)
+// Items of `count` pixels in tiles (the tiles' pixels outside the range too).
+__device__ __forceinline__ int64_t tile_items(const FilmTiles& t, int64_t count)
 {
-    const unsigned lines = n / line;
-    const unsigned band = q / (4u * line);
-    const unsigned base = band * 4u * line;
-    const unsigned h = min(4u, lines - min(lines, 4u * band));
-    const unsigned r = q - base;
-    if (r >= h * line)
-        return q;
-    const unsigned x0 = r / (8u * h) * 8u;
-    const unsigned w = min(8u, line - x0);
-    const unsigned k = r - x0 * h;
-    const unsigned y = k / w;
-    return base + y * line + x0 + (k - y * w);
+    return t.columns > 0 ? int64_t(t.columns) * t.rows * 32 : count;
+}
+
+// Whether an item is a pixel of the range, and which (in `i`, from the range's
+// first). Tiles lie on the film's columns, so that a warp's pixels are one
+// tile whatever the width: in a permutation without padding, whose warps
+// straddle two tiles where the width is no multiple of 8, the RAY frame of
+// 1919x1079 pixels took 544 us instead of 502.
+__device__ __forceinline__ bool tile_pixel(const FilmTiles& t, int64_t count, int64_t item, int64_t& i)
+{
+    i = item;
+    if (t.columns > 0)
+    {
+        const int tile = int(item >> 5);
+        const int row = tile / t.columns;
+        const int x = (tile - row * t.columns) * 8 + int(item & 7);
+        const int64_t y = int64_t(row) * 4 + int((item >> 3) & 3);
+        i = y * t.width + x - t.skip;
+        if (x >= t.width)
+            return false;
+    }
+    return i >= 0 && i < count;
 }
 
 __device__ __forceinline__ void load_node(const DevNode* __restrict__ nodes, int i, float4& a, float4& b, float4& c,
