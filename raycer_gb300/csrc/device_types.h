@@ -19,8 +19,8 @@
 //            (same leaves, same triangle order): the four children's boxes as
 //            one float4 per bound (child k in component k), their links, and
 //            the number of children. Read by the path tracer's uncounted nearest-first
-//            kernels (traverse_wide); the binary tree serves every other
-//            query.
+//            kernels and by large nearest-first rc_cast batches; the binary
+//            tree serves every other query.
 // Everything is 16-B aligned and fetched with 128-bit loads.
 #pragma once
 

@@ -1261,40 +1261,54 @@ __global__ void __launch_bounds__(128, 8) k_path_group(PassParams p, unsigned G)
         atomicAdd(finished, 1u);
 }
 
+// Film update, one pixel per thread at a time. A thread waits for the pass's
+// stop bit, its chunk's record, the scene's, and then for the samples and the
+// film; with more blocks than the GPU holds each block waits for the records
+// again, so where a pass has one chunk the resident blocks keep them and go
+// over the pixels: 1080p with one path per pixel 59 -> 29 us (33 MB of results
+// and 66 MB of film).
 __global__ void __launch_bounds__(256) k_accumulate(PassParams p)
 {
     int pix = blockIdx.x * blockDim.x + threadIdx.x;
     if (pix >= p.npixels || pass_stopped(p))
         return;
-    if (p.monitor && threadIdx.x == 0)
-        atomicAdd(&p.ctl->progress, static_cast<unsigned long long>(min(256, p.npixels - pix)));
-    const PathChunk ch = p.chunks[chunk_of_pixel(p, uint32_t(pix))];
-    const PathScene& sc = p.scenes[ch.scene];
-    const uint32_t inChunk = uint32_t(pix) - ch.pixelPassBegin;
-    const int nn = sc.n * sc.n;
-    const float fP = float(sc.P);
-    float4* fp = sc.film + ch.pixelLocalBegin + inChunk;
-    float4 f = *fp;
-    size_t base = size_t(ch.slotBegin) + size_t(inChunk) * size_t(sc.spp);
-    for (int j = 0; j < nn; ++j)
+    PathChunk ch = p.chunks[chunk_of_pixel(p, uint32_t(pix))];
+    const PathScene* sc = p.scenes + ch.scene;
+    float4* film = sc->film;
+    int nn = sc->n * sc->n, P = sc->P, spp = sc->spp;
+    while (true)
     {
-        float sr = 0.0f, sg = 0.0f, sb = 0.0f, w = 0.0f;
-        for (int k = 0; k < sc.P; ++k)
+        if (p.monitor && threadIdx.x == 0)
+            atomicAdd(&p.ctl->progress, static_cast<unsigned long long>(min(256, p.npixels - pix)));
+        const uint32_t inChunk = uint32_t(pix) - ch.pixelPassBegin;
+        const float fP = float(P);
+        float4* fp = film + ch.pixelLocalBegin + inChunk;
+        float4 f = *fp;
+        const size_t base = size_t(ch.slotBegin) + size_t(inChunk) * size_t(spp);
+#pragma unroll 4
+        for (int j = 0; j < nn; ++j)
         {
-            float4 r = p.res[base + size_t(j) * size_t(sc.P) + size_t(k)];
-            sr = __fadd_rn(sr, r.x);
-            sg = __fadd_rn(sg, r.y);
-            sb = __fadd_rn(sb, r.z);
-            w = r.w;
+            float sr = 0.0f, sg = 0.0f, sb = 0.0f, w = 0.0f;
+            for (int k = 0; k < P; ++k)
+            {
+                float4 r = p.res[base + size_t(j) * size_t(P) + size_t(k)];
+                sr = __fadd_rn(sr, r.x);
+                sg = __fadd_rn(sg, r.y);
+                sb = __fadd_rn(sb, r.z);
+                w = r.w;
+            }
+            // PathTracer::trace divides by pathSampleCount (PathTracer.cpp:22);
+            // Film::addSample adds color * weight and weight (Film.cpp:57-58).
+            f.x = __fadd_rn(f.x, __fmul_rn(__fdiv_rn(sr, fP), w));
+            f.y = __fadd_rn(f.y, __fmul_rn(__fdiv_rn(sg, fP), w));
+            f.z = __fadd_rn(f.z, __fmul_rn(__fdiv_rn(sb, fP), w));
+            f.w = __fadd_rn(f.w, w);
         }
-        // PathTracer::trace divides by pathSampleCount (PathTracer.cpp:22);
-        // Film::addSample adds color * weight and weight (Film.cpp:57-58).
-        f.x = __fadd_rn(f.x, __fmul_rn(__fdiv_rn(sr, fP), w));
-        f.y = __fadd_rn(f.y, __fmul_rn(__fdiv_rn(sg, fP), w));
-        f.z = __fadd_rn(f.z, __fmul_rn(__fdiv_rn(sb, fP), w));
-        f.w = __fadd_rn(f.w, w);
+        *fp = f;
+        pix += int(gridDim.x * blockDim.x);
+        if (pix >= p.npixels)
+            return;
     }
-    *fp = f;
 }
 
 // Persistent grid: resident blocks per SM (cached per device) x the
@@ -1617,9 +1631,13 @@ cudaError_t launch_path_segments(const PassParams& p, int order, int counting, c
     return cudaSuccess;
 }
 
-cudaError_t launch_path_accumulate(const PassParams& p, cudaStream_t stream)
+cudaError_t launch_path_accumulate(const PassParams& p, cudaStream_t stream, int numSMs)
 {
-    k_accumulate<<<unsigned((p.npixels + 255) / 256), 256, 0, stream>>>(p);
+    static OccupancyCache occ;
+    unsigned blocks = unsigned((p.npixels + 255) / 256);
+    if (p.numChunks == 1)
+        blocks = std::min(blocks, unsigned(persistent_blocks(k_accumulate, 256, numSMs, occ)));
+    k_accumulate<<<blocks, 256, 0, stream>>>(p);
     return cudaGetLastError();
 }
 
@@ -1629,7 +1647,7 @@ cudaError_t launch_path_pass(const PassParams& p, int order, int counting, const
     cudaError_t e = launch_path_segments(p, order, counting, shape, stream, numSMs, extendEvents);
     if (e != cudaSuccess)
         return e;
-    return launch_path_accumulate(p, stream);
+    return launch_path_accumulate(p, stream, numSMs);
 }
 
 cudaError_t launch_nrc_targets(const PassParams& p, cudaStream_t stream)

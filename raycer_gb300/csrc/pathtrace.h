@@ -144,7 +144,7 @@ cudaError_t launch_path_pass(const PassParams& p, int order, int counting, const
 // update (cache lookups): generate + segments, then accumulate.
 cudaError_t launch_path_segments(const PassParams& p, int order, int counting, const PassShape& shape,
                                  cudaStream_t stream, int numSMs, const cudaEvent_t* extendEvents);
-cudaError_t launch_path_accumulate(const PassParams& p, cudaStream_t stream);
+cudaError_t launch_path_accumulate(const PassParams& p, cudaStream_t stream, int numSMs);
 // Training targets of the pass's training paths (radiance of each vertex's
 // suffix, written over the bounce factors) and the sample index list.
 cudaError_t launch_nrc_targets(const PassParams& p, cudaStream_t stream);

@@ -346,7 +346,7 @@ rc_status render_path(rc_tracer* h, uint64_t pixelStart, uint64_t count, RenderW
         rc_status s = nrc_lookups(h, pp);
         if (s == RC_OK)
         {
-            RC_CUDA_TRY(h, launch_path_accumulate(pp, h->stream), "launch film update");
+            RC_CUDA_TRY(h, launch_path_accumulate(pp, h->stream, h->numSMs), "launch film update");
             s = nrc_train_pass(h, pp);
         }
         if (s != RC_OK)

@@ -399,7 +399,7 @@ __device__ __forceinline__ void wide_cswap(float& da, int& la, float& db, int& l
     la = l;
 }
 
-// Closest hit through the 4-wide BVH (sc.wide; wide_bvh.cpp): one 128-B
+// Closest hit through the 4-wide BVH (sc.wide; wide_build.cu): one 128-B
 // node fetch tests up to four child boxes, the children hit within the
 // current closest distance are sorted by entry distance (a five-exchange
 // network), the nearest is entered and the others pushed farthest first with
