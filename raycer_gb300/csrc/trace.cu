@@ -32,11 +32,19 @@ constexpr int kBlock = 128;
 #ifndef RC_TRACE_MIN_BLOCKS
 #define RC_TRACE_MIN_BLOCKS 10
 #endif
-// The one-kernel RAY frame (primary + shadow walks) at 9 blocks: 56
-// registers, no spills; 0.405 ms per 1080p heightfield frame against 0.417
-// at 10 blocks (48 registers, spills) and 0.420 at 8.
+// The one-kernel RAY frame (primary + shadow walks) of a single-level scene at
+// 7 blocks (it takes 60-64 registers, so 8 are resident): it is bound by issue,
+// and on frames of few tiles per warp by the chain of the longest tile; with
+// registers to spare the compiler orders the fetches better, which the warps
+// of a ninth block (56 registers) do not make up for. 7 / 8 / 9 blocks, 1M
+// triangles: 1080p 392 / 394 / 398 us, 640x360 192 / 199 / 203, in reference
+// order 836 / 875 / 855 and 719 / 753 / 782; 6 and 5 blocks as 7. Two-level
+// frames keep 9.
 #ifndef RC_FUSED_MIN_BLOCKS
-#define RC_FUSED_MIN_BLOCKS 9
+#define RC_FUSED_MIN_BLOCKS 7
+#endif
+#ifndef RC_FUSED_INST_MIN_BLOCKS
+#define RC_FUSED_INST_MIN_BLOCKS 9
 #endif
 #ifndef RC_TRACE_TILES
 #define RC_TRACE_TILES 1
@@ -186,7 +194,10 @@ __device__ __forceinline__ void shadow_of(const DevScene& sc, const RayF& ray, c
 // tiles on a silhouette leave lanes idle. With the caller's rays in host
 // memory the shadow work then overlaps the ray reads over the host link.
 template <int ORDER, bool COUNT, bool PACKET, bool INST, bool FUSED = false, bool SL = false, int SOCT = -1>
-__global__ void __launch_bounds__(kBlock, FUSED ? RC_FUSED_MIN_BLOCKS : RC_TRACE_MIN_BLOCKS) k_raycast_primary(DevScene sc, DevCamera cam, const rc_ray* __restrict__ rays,
+__global__ void __launch_bounds__(kBlock, !FUSED ? RC_TRACE_MIN_BLOCKS
+                                          : INST ? RC_FUSED_INST_MIN_BLOCKS
+                                                 : RC_FUSED_MIN_BLOCKS)
+    k_raycast_primary(DevScene sc, DevCamera cam, const rc_ray* __restrict__ rays,
                                                             uint64_t pixelStart, int64_t count, int64_t width,
                                                             FilmTiles tiles, int castShadow,
                                                             rc_cast_pixel* __restrict__ out, int* __restrict__ queue,
