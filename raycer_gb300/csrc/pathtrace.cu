@@ -1121,7 +1121,8 @@ __global__ void __launch_bounds__(128, RC_INST_MIN_BLOCKS)
             // one decision per warp (lane 0's view of the stop bit)
             if (watched && __shfl_sync(kAll, int(render_stopped(p.ctl)), 0) != 0)
                 break;
-            if (__ballot_sync(kAll, w.cur > kWalkReturn) == 0u)
+            // a lane on its way out of an instance (kWalkReturn) walks on too
+            if (__ballot_sync(kAll, w.cur > kWalkNone) == 0u)
                 break;
             continue;
         }
