@@ -468,8 +468,10 @@ __global__ void __launch_bounds__(kBlock, 8) k_cast_phased(DevScene sc, const rc
                     write_hit(sc, h, hits + i);
                     w.cur = kWalkNone;
                 }
+                // decided after this turn's rays are listed: the 31 of a list
+                // with room and the 32 that may be in flight fit its 64 entries
                 const unsigned idle = __ballot_sync(kAll, w.cur == kWalkNone);
-                if (take)
+                if (!drained && listed < 32)
                 {
                     const unsigned base = warp_fetch(&ctl->head[0], unsigned(__popc(idle)));
                     drained = base + unsigned(__popc(idle)) >= unsigned(n);
