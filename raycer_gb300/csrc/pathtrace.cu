@@ -247,6 +247,41 @@ __device__ __forceinline__ void flush_extend_counts(const PassParams& p, unsigne
         atomicOr(&p.ctl->error, 1);
 }
 
+// Closest hit of a ray put aside from the 4-wide walk (an inverse direction
+// that is not finite) through the binary trees; no triangle accepts a ray with
+// a NaN, whose walk would enter every box.
+template <bool INST>
+static __device__ __noinline__ HitF aside_hit(const PassParams& p, int s, const float4& o, const float4& d)
+{
+    HitF h{ -1, FLT_MAX, 0.0f, 0.0f, -1 };
+    if (!(o.x == o.x && o.y == o.y && o.z == o.z && d.x == d.x && d.y == d.y && d.z == d.z))
+        return h;
+    const DevScene sc = scene_of_slot(p, s);
+    const RayF ray = make_ray(v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), 0.0f, FLT_MAX);
+    TravCount none{ 0, 0 };
+    int err = 0;
+    if (INST)
+        traverse_instanced<false, false>(sc, ray, h, none, err, __float_as_int(o.w), __float_as_int(d.w));
+    else
+        traverse<false, ORDER_NEAREST, false>(sc, ray, h, none, err, __float_as_int(o.w));
+    if (err)
+        atomicOr(&p.ctl->error, 1);
+    return h;
+}
+
+// Queued rays that their lane has put aside, a list through the hit records
+// from slot s on (-1: none): their hits.
+static __device__ __noinline__ void extend_aside(const PassParams& p, int s)
+{
+    while (s >= 0)
+    {
+        const int next = p.hit[s].x;
+        const HitF h = aside_hit<false>(p, s, p.o[s], p.d[s]);
+        p.hit[s] = make_int4(h.slot, __float_as_int(h.t), __float_as_int(h.u), __float_as_int(h.v));
+        s = next;
+    }
+}
+
 template <int ORDER, bool COUNT, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, ((ORDER == ORDER_WIDE ? RC_EXTEND_WIDE_MIN_BLOCKS : RC_EXTEND_MIN_BLOCKS) * 128) /
                                              BLOCK) k_extend(PassParams p, int segment)
@@ -255,6 +290,7 @@ __global__ void __launch_bounds__(BLOCK, ((ORDER == ORDER_WIDE ? RC_EXTEND_WIDE_
     const int* __restrict__ queue = (segment & 1) ? p.qb : p.qa;
     TravCount cnt{ 0, 0 };
     int err = 0;
+    int aside = -1;  // extend_aside's list
     unsigned long long done = 0;
     if (pass_stopped(p))
         return;
@@ -276,13 +312,21 @@ __global__ void __launch_bounds__(BLOCK, ((ORDER == ORDER_WIDE ? RC_EXTEND_WIDE_
             float4 o = p.o[s];
             float4 d = p.d[s];
             RayF ray = make_ray(v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), 0.0f, FLT_MAX);
+            done++;
+            if (ORDER == ORDER_WIDE && !ray.finite)
+            {
+                p.hit[s] = make_int4(aside, 0, 0, 0);
+                aside = s;
+                continue;
+            }
             HitF h{ -1, FLT_MAX, 0.0f, 0.0f, -1 };
             bool found = ORDER == ORDER_WIDE ? traverse_wide(sc, ray, h, err, __float_as_int(o.w))
                                              : traverse<false, ORDER, COUNT>(sc, ray, h, cnt, err, __float_as_int(o.w));
             p.hit[s] = make_int4(found ? h.slot : -1, __float_as_int(h.t), __float_as_int(h.u), __float_as_int(h.v));
-            done++;
         }
     }
+    if (ORDER == ORDER_WIDE)
+        extend_aside(p, aside);
     flush_extend_counts(p, done, cnt, err);
 }
 
@@ -323,6 +367,7 @@ __global__ void __launch_bounds__(BLOCK, (RC_EXTEND_REFILL_MIN_BLOCKS * 128) / B
     const DevNode4* wide = nullptr;
     const DevTri* tris = nullptr;
     bool drained = false;  // warp-uniform
+    int aside = -1;  // extend_aside's list
     const unsigned below = (1u << lane_id()) - 1u;
     if (is_watch_warp(p.monitor, p.budgetNs))
     {
@@ -356,6 +401,13 @@ __global__ void __launch_bounds__(BLOCK, (RC_EXTEND_REFILL_MIN_BLOCKS * 128) / B
                     skip = __float_as_int(o.w);
                     wide = sc.wide;
                     tris = sc.tris;
+                    if (!ray.finite)
+                    {
+                        p.hit[s] = make_int4(aside, 0, 0, 0);
+                        aside = s;
+                        done++;
+                        s = -1;
+                    }
                 }
             }
         }
@@ -372,6 +424,7 @@ __global__ void __launch_bounds__(BLOCK, (RC_EXTEND_REFILL_MIN_BLOCKS * 128) / B
             s = -1;
         }
     }
+    extend_aside(p, aside);
     flush_extend_counts(p, done, TravCount{ 0, 0 }, err);
 }
 
@@ -798,6 +851,18 @@ __global__ void __launch_bounds__(BLOCK) k_shade(PassParams p, int segment)
     }
 }
 
+// A path whose ray has an inverse direction that is not finite is put aside
+// from the 4-wide walk, with its ray and segment: k_finish_aside takes it to
+// its end. (The binary walk in these kernels, or a call for it at the end of
+// their loops, cost every path's walk its registers: 4-40 % slower.)
+__device__ __forceinline__ void put_aside(const PassParams& p, int segment, int s, const float4& o, const float4& d)
+{
+    p.o[s] = o;
+    p.d[s] = d;
+    p.hit[s].x = segment;
+    p.qa[atomicAdd(&p.counts[3], 1u)] = s;
+}
+
 // Extend and shade in one kernel (uncounted nearest-first passes over the
 // 4-wide BVH of a single-level scene, plain or with the radiance cache):
 // each lane walks its slot's ray as k_extend does, then shades the slot at
@@ -850,11 +915,19 @@ __global__ void __launch_bounds__(BLOCK,
             start_slot<NRC, false>(p, unsigned(s), o, d);
             const DevScene sc = scene_of_slot(p, s);
             RayF ray = make_ray(v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), 0.0f, FLT_MAX);
-            HitF h{ -1, FLT_MAX, 0.0f, 0.0f, -1 };
-            const bool found = traverse_wide(sc, ray, h, err, -1);
-            done++;
-            cont = shade_slot<NRC, kRayPassed, true>(p, 0, s, make_int4(found ? h.slot : -1, __float_as_int(h.t), 0, -1),
-                                         o, d, lookup, lrec);
+            if (!ray.finite)
+            {
+                p.thr[s] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
+                put_aside(p, 0, s, o, d);
+            }
+            else
+            {
+                HitF h{ -1, FLT_MAX, 0.0f, 0.0f, -1 };
+                const bool found = traverse_wide(sc, ray, h, err, -1);
+                done++;
+                cont = shade_slot<NRC, kRayPassed, true>(
+                    p, 0, s, make_int4(found ? h.slot : -1, __float_as_int(h.t), 0, -1), o, d, lookup, lrec);
+            }
         }
         enqueue_continuing(cont, s, outCount, p.qb);
         if (NRC)
@@ -996,11 +1069,17 @@ __global__ void __launch_bounds__(BLOCK,
                     tris = sc.tris;
                     w.cur = sc.wideRoot;
                 }
+                if (!ray.finite)
+                {
+                    const int2 path = paths[threadIdx.x];
+                    put_aside(p, path.y, path.x, o, d);
+                    w.cur = kWalkNone;
+                }
             }
             // one decision per warp (lane 0's view of the stop bit)
             if (watched && __shfl_sync(kAll, int(render_stopped(p.ctl)), 0) != 0)
                 break;
-            if (__ballot_sync(kAll, w.cur > kWalkNone) == 0u)
+            if (drained && __ballot_sync(kAll, w.cur > kWalkNone) == 0u)
                 break;
             continue;
         }
@@ -1117,12 +1196,18 @@ __global__ void __launch_bounds__(128, RC_INST_MIN_BLOCKS)
                 h = HitF{ -1, FLT_MAX, 0.0f, 0.0f, -1 };
                 hitInst[threadIdx.x] = -1;
                 w = TwoLevelWalk{ p.scene0.wideTlasRoot, 0, 0, -1 };
+                if (!ray.finite)
+                {
+                    const int2 path = paths[threadIdx.x];
+                    put_aside(p, path.y, path.x, o, d);
+                    w.cur = kWalkNone;
+                }
             }
             // one decision per warp (lane 0's view of the stop bit)
             if (watched && __shfl_sync(kAll, int(render_stopped(p.ctl)), 0) != 0)
                 break;
             // a lane on its way out of an instance (kWalkReturn) walks on too
-            if (__ballot_sync(kAll, w.cur > kWalkNone) == 0u)
+            if (drained && __ballot_sync(kAll, w.cur > kWalkNone) == 0u)
                 break;
             continue;
         }
@@ -1154,6 +1239,13 @@ __global__ void __launch_bounds__(128, RC_INST_MIN_BLOCKS)
                     skips[threadIdx.x] = __float_as_int(d.w) == k ? __float_as_int(o.w) : -1;
                     ray = instance_ray(load_instance(p.scene0.instances, k), ray);
                     w.cur = __ldg(p.scene0.instWide + k);
+                    if (!ray.finite)
+                    {
+                        const int2 path = paths[threadIdx.x];
+                        put_aside(p, path.y, path.x, o, d);
+                        w.abandon();
+                        w.cur = kWalkNone;
+                    }
                 }
             }
         }
@@ -1172,6 +1264,64 @@ __global__ void __launch_bounds__(128, RC_INST_MIN_BLOCKS)
             wide_node_step(w.inst >= 0 ? p.scene0.wide : p.scene0.wideTlas, ray, h, w, stack, err);
     }
     flush_extend_counts(p, lane_id() == 0 ? done : 0u, TravCount{ 0, 0 }, err);
+    if (watched && lane_id() == 0)
+        atomicAdd(finished, 1u);
+}
+
+// The paths that the pass's 4-wide walks put aside, one per lane, to their
+// ends. Usually there are none, and the blocks return at once.
+template <bool NRC, bool INST>
+__global__ void __launch_bounds__(128) k_finish_aside(const __grid_constant__ PassParams p)
+{
+    const unsigned total = *reinterpret_cast<volatile unsigned*>(&p.counts[3]);
+    unsigned* head = &p.counts[p.segments * 4 + 1];
+    unsigned* finished = &p.counts[p.segments * 4 + 2];  // warps that have no more work
+    if (total == 0u || pass_stopped(p))
+        return;
+    if (is_watch_warp(p.monitor, p.budgetNs))
+    {
+        watch_queue(p.monitor, p.budgetNs, p.ctl, head, total, kPublishProgress, 0, finished);
+        return;
+    }
+    const bool watched = monitored(p.monitor, p.budgetNs);
+    unsigned long long done = 0;
+    bool stop = false;  // warp-uniform
+    while (!stop)
+    {
+        const unsigned base = warp_fetch(head, 32u);
+        if (base >= total)
+            break;
+        int s = -1;
+        int segment = 0;
+        float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f), d = o;
+        if (base + lane_id() < total)
+        {
+            s = p.qa[base + lane_id()];
+            segment = p.hit[s].x;
+            o = p.o[s];
+            d = p.d[s];
+        }
+        while (__ballot_sync(0xffffffffu, s >= 0))
+        {
+            // one decision per warp (lane 0's view of the stop bit)
+            stop = watched && __shfl_sync(0xffffffffu, int(render_stopped(p.ctl)), 0) != 0;
+            if (stop)
+                break;
+            bool lookup = false;
+            NrcRecord lrec;
+            if (s >= 0)
+            {
+                const HitF h = aside_hit<INST>(p, s, o, d);
+                done++;
+                if (!shade_slot<NRC, kRayKept>(p, segment++, s, make_int4(h.slot, __float_as_int(h.t), 0, h.inst), o, d,
+                                               lookup, lrec))
+                    s = -1;
+            }
+            if (NRC)
+                enqueue_lookup(lookup, lrec, p);
+        }
+    }
+    flush_extend_counts(p, done, TravCount{ 0, 0 }, 0);
     if (watched && lane_id() == 0)
         atomicAdd(finished, 1u);
 }
@@ -1425,6 +1575,22 @@ cudaError_t bounce_inst(const PassParams& p, int first, cudaStream_t stream, int
     return p.nrc.query ? bounce_inst_b<true>(p, first, stream, numSMs) : bounce_inst_b<false>(p, first, stream, numSMs);
 }
 
+template <bool NRC, bool INST>
+cudaError_t finish_aside_b(const PassParams& p, cudaStream_t stream, int numSMs)
+{
+    auto k = k_finish_aside<NRC, INST>;
+    static OccupancyCache occ;
+    k<<<persistent_blocks(k, 128, numSMs, occ), 128, 0, stream>>>(p);
+    return cudaGetLastError();
+}
+
+cudaError_t finish_aside(const PassParams& p, cudaStream_t stream, int numSMs)
+{
+    if (p.nrc.query)
+        return p.instanced ? finish_aside_b<true, true>(p, stream, numSMs) : finish_aside_b<true, false>(p, stream, numSMs);
+    return p.instanced ? finish_aside_b<false, true>(p, stream, numSMs) : finish_aside_b<false, false>(p, stream, numSMs);
+}
+
 // The block sizes of the kernels it replaces: the autotuned extend block for
 // plain passes, 128 threads for cache passes.
 cudaError_t extend_shade_t(const PassParams& p, int block, cudaStream_t stream, int numSMs)
@@ -1629,7 +1795,8 @@ cudaError_t launch_path_segments(const PassParams& p, int order, int counting, c
         if ((e = shade_t(p, seg, shape.shadeBlock, stream, numSMs)) != cudaSuccess)
             return e;
     }
-    return cudaSuccess;
+    // two-level camera rays walk the binary trees: one segment puts none aside
+    return fused && launches > (p.instanced ? 1 : 0) ? finish_aside(p, stream, numSMs) : cudaSuccess;
 }
 
 cudaError_t launch_path_accumulate(const PassParams& p, cudaStream_t stream, int numSMs)

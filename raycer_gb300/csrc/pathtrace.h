@@ -97,7 +97,7 @@ struct PassParams
     int* qa;
     int* qb;
     int* chunkOf;    // slot -> chunk (written by generate)
-    unsigned* counts;  // per segment: [queue count, extend head, shade head, unused]
+    unsigned* counts;  // per segment: [queue count, extend head, shade head, segment 0: paths put aside]
     DevControl* ctl;
     NrcPass nrc;
     int instanced;   // 1: the pass has two-level scenes (k_extend_instanced)

@@ -393,7 +393,8 @@ __global__ void __launch_bounds__(kBlock, RC_TRACE_MIN_BLOCKS) k_raycast_shadow(
 // lanes wait for, and once kCastLanes walks have ended, those lanes write
 // their hits and take new rays. Nearest-first closest hits walk the 4-wide
 // tree; a hit that lies before its own leaf's entry may have been decided by
-// the order of the walk (see traverse_group) and is walked again alone.
+// the order of the walk (see traverse_group) and is walked again alone, and so
+// is a ray whose walk ends undecided.
 // Reference-order and any-hit queries take the binary tree's boxes and
 // triangles in the reference's order.
 //
@@ -457,7 +458,8 @@ __global__ void __launch_bounds__(kBlock, 8) k_cast_phased(DevScene sc, const rc
                 done += unsigned(__popc(__ballot_sync(kAll, w.cur == kWalkDone)));
                 if constexpr (WIDE)
                 {
-                    const bool odd = w.cur == kWalkDone && h.slot >= 0 && w.hitEntry > h.t;
+                    // no hit: 0 within FLT_MAX; undecided: a NaN
+                    const bool odd = w.cur == kWalkDone && !(w.hitEntry <= h.t);
                     const unsigned m = __ballot_sync(kAll, odd);
                     if (odd)
                         list[listed + __popc(m & below)] = i;

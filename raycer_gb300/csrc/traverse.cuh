@@ -357,7 +357,8 @@ __device__ __forceinline__ bool traverse_stackless(const DevScene& sc, const Ray
 }
 
 // Entry distance of one child box of a wide node, or +inf when the ray misses
-// it or enters it beyond `limit` (the current closest hit); any ray.
+// it or enters it beyond `limit` (the current closest hit); any ray. NaN where
+// slab() hits the box with a NaN entry (see wide_node_step).
 __device__ __forceinline__ float wide_entry(const RayF& ray, float lox, float hix, float loy, float hiy, float loz,
                                             float hiz, float limit)
 {
@@ -406,12 +407,15 @@ __device__ __forceinline__ void wide_cswap(float& da, int& la, float& db, int& l
 // their entry distances, and pops skip entries beyond the current hit. The
 // leaves and their triangle tests are the binary tree's, and the accepted
 // hit (minimum t, ties to the larger slot) does not depend on the order, so
-// it is traverse<false, ORDER_NEAREST>'s. No node or triangle counts: counted
-// frames use the binary traversal.
+// it is traverse<false, ORDER_NEAREST>'s. Rays whose inverse direction is not
+// finite can reach other boxes here than there (see wide_node_step) and walk
+// the binary tree. No node or triangle counts: counted frames use the binary
+// traversal.
 // Where a 4-wide walk stands between steps: the node or leaf link to visit
 // next and the stack depth (the stack arrays are the caller's).
 struct WideWalk
 {
+    static constexpr bool kFinite = true;  // only rays whose inverse direction is finite
     int cur;
     int sp;
     __device__ __forceinline__ void abandon();
@@ -475,6 +479,7 @@ constexpr float kTieCull = 1.01f;
 // hit's leaf and skips boxes only past kTieCull times the hit.
 struct CastWalk
 {
+    static constexpr bool kFinite = false;  // any ray
     int cur;
     int sp;
     float entry;     // of cur
@@ -506,9 +511,26 @@ __device__ __forceinline__ void wide_pop(const HitF& hit, Walk& w, const Stack& 
     w.cur = kWalkDone;
 }
 
+// Whether a CastWalk ended undecided: its ray has to walk the binary tree.
+__device__ __forceinline__ bool walk_undecided(const HitF& hit) { return !(hit.t == hit.t); }
+
 // Node step of the 4-wide walk (w.cur >= 0): enters the nearest child hit
 // within the current closest distance and pushes the others; with none hit,
 // pops. On stack overflow err = 1 and the walk is over.
+//
+// A direction component of zero with the origin on a box's lower plane makes
+// slab()'s product a NaN (0 * inf), and with it, in x, the box's entry: slab()
+// then hits the box wherever its other planes lie. So a box inside a parent
+// that the ray misses can be hit, and which boxes a ray reaches depends on the
+// tree that is walked: the walk ends here, undecided, with the hit's t a NaN.
+// (Taken as entered at 0,
+// such boxes gave 498 other triangles of 32,768 vertical rays at the vertices
+// of a 256x128 heightfield; dropped, 24,677 of its 32,387 hits were lost.)
+// Without a NaN entry the boxes reached are the binary walk's, up to boxes
+// that are flat in a direction the ray has no part of, whose triangles it
+// cannot hit. No triangle accepts a ray that has a NaN itself: it leaves the
+// node. The path tracer's walks keep to finite inverse directions: its kernels
+// ran 6-10 % slower with this branch and what follows from it.
 template <typename Walk, typename Stack>
 __device__ __forceinline__ void wide_node_step(const DevNode4* __restrict__ wide, const RayF& ray, HitF& hit, Walk& w,
                                                Stack& stack, int& err)
@@ -524,7 +546,7 @@ __device__ __forceinline__ void wide_node_step(const DevNode4* __restrict__ wide
     const int nc = __float_as_int(mf.x);
     const float limit = w.limit(hit);
     float d0, d1, d2, d3;
-    if (ray.finite)
+    if (Walk::kFinite || ray.finite)
     {
         const AxisF2 X{ f2(-ray.o.x, -ray.o.x), f2(ray.inv.x, ray.inv.x) };
         const AxisF2 Y{ f2(-ray.o.y, -ray.o.y), f2(ray.inv.y, ray.inv.y) };
@@ -550,6 +572,18 @@ __device__ __forceinline__ void wide_node_step(const DevNode4* __restrict__ wide
         d1 = wide_entry(ray, lox.y, hix.y, loy.y, hiy.y, loz.y, hiz.y, limit);
         d2 = wide_entry(ray, lox.z, hix.z, loy.z, hiy.z, loz.z, hiz.z, limit);
         d3 = wide_entry(ray, lox.w, hix.w, loy.w, hiy.w, loz.w, hiz.w, limit);
+        if (d0 != d0 || d1 != d1 || (nc > 2 && d2 != d2) || (nc > 3 && d3 != d3))
+        {
+            const V3 o = ray.o, d = ray.d;
+            if (o.x != o.x || o.y != o.y || o.z != o.z || d.x != d.x || d.y != d.y || d.z != d.z)
+            {
+                wide_pop(hit, w, stack);
+                return;
+            }
+            hit.t = __int_as_float(0x7fffffff);
+            w.abandon();
+            return;
+        }
     }
     if (nc < 3)
         d2 = kInf;
@@ -650,6 +684,7 @@ constexpr int kWalkReturn = -0x7ffffffe;  // the mesh is done (no leaf code: 13 
 
 struct TwoLevelWalk
 {
+    static constexpr bool kFinite = true;
     int cur;
     int sp;
     int base;
@@ -758,6 +793,7 @@ __device__ __forceinline__ void ref_leaf_step(const DevTri* __restrict__ tris, c
         ref_pop(w, stack);
 }
 
+// The walk of a ray whose inverse direction is finite, to its end.
 __device__ __forceinline__ bool traverse_wide(const DevScene& sc, const RayF& ray, HitF& hit, int& err, int skip)
 {
     int2 entries[kMaxStack];
@@ -1000,6 +1036,13 @@ __device__ __forceinline__ bool traverse_group(const DevScene& sc, const RayF& r
             {
                 h0 = slab(ray, a.x, a.y, a.z, a.w, c.x, c.y, e0);
                 h1 = slab(ray, b.x, b.y, b.z, b.w, c.z, c.w, e1);
+                if (CULL)
+                {
+                    // a NaN entry (see wide_node_step) says nothing of the
+                    // boxes around it, whose entries a walk may have skipped
+                    e0 = fmaxf(e0, __int_as_float(e.y));
+                    e1 = fmaxf(e1, __int_as_float(e.y));
+                }
             }
             if (CULL)
             {
