@@ -243,8 +243,8 @@ void release_scene_data(rc_tracer* h);
 // Collapses the binary device nodes of the handle's single-level scene into
 // the 4-wide BVH on first use (the first PATH or batch render of a scene, or
 // rc_cast of many rays); leaves it out where its stack need exceeds the
-// traversal stack. Failure to allocate is an error. Uploads, RAY frames and
-// small passes and casts do not pay for it.
+// traversal stack or there is no memory for it. Uploads, RAY frames and small
+// passes and casts do not pay for it.
 rc_status ensure_wide(rc_tracer* h);
 // Builds the rope records of the handle's single-level scene on first use
 // (the first RAY frame or rc_cast while the stackless walk is on): one

@@ -1,0 +1,164 @@
+// Host side of the 4-wide trees' construction (kernels: wide_build.cu): which
+// trees a scene gets, when, and their memory.
+//
+// A traversal pushes at most (children - 1) entries per node; a tree whose
+// worst root-to-leaf sum exceeds the stack is left binary, and so is one for
+// which there is no memory (the binary kernels serve every call), and every
+// scene when RC_WIDE_BVH=0 is set in the environment (read once).
+
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstdlib>
+#include <string>
+#include <vector>
+
+#include "host_internal.h"
+#include "wide_collapse.h"
+
+namespace rcx
+{
+namespace
+{
+
+// Collapses the trees of `roots` (inner links into nodes[0, count)) into one
+// array of 4-wide nodes, root i at index i. *out stays null where the stack
+// need (*need) is above `maxNeed`, or where there is no memory.
+rc_status collapse(rc_tracer* h, const DevNode* nodes, size_t count, const std::vector<int32_t>& roots, int levels,
+                   int maxNeed, DevNode4** out, int* need)
+{
+    *out = nullptr;
+    WideItem* items = nullptr;
+    WideCounters* counters = nullptr;
+    WideCounters got{};
+    std::vector<WideItem> first(roots.size());
+    for (size_t i = 0; i < roots.size(); ++i)
+        first[i] = WideItem{ roots[i], 0 };
+    got.nodes = int(roots.size());
+    // a wide node stands for one binary inner node
+    cudaError_t e = cudaMalloc(reinterpret_cast<void**>(out), count * sizeof(DevNode4));
+    if (e == cudaSuccess)
+        e = cudaMalloc(reinterpret_cast<void**>(&items), count * sizeof(WideItem) + sizeof(WideCounters));
+    if (e == cudaSuccess)
+    {
+        counters = reinterpret_cast<WideCounters*>(items + count);
+        e = cudaMemcpyAsync(counters, &got, sizeof(got), cudaMemcpyHostToDevice, h->stream);
+    }
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(items, first.data(), first.size() * sizeof(WideItem), cudaMemcpyHostToDevice, h->stream);
+    levels = std::min(std::max(levels, 1), kMaxStack);
+    for (int level = 0; e == cudaSuccess && level < levels; ++level)
+    {
+        // at most 4^level nodes per root
+        const size_t most = level < 12 ? std::min(count, roots.size() << (2 * level)) : count;
+        e = launch_collapse(nodes, int(count), items, *out, counters, level, most, h->numSMs, h->stream);
+    }
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(&got, counters, sizeof(got), cudaMemcpyDeviceToHost, h->stream);
+    if (e == cudaSuccess)
+        e = cudaStreamSynchronize(h->stream);
+    cudaFree(items);
+    if (e == cudaSuccess && !got.error && got.maxNeed <= maxNeed && got.nodes == got.bound[levels])
+    {
+        *need = got.maxNeed;
+        return RC_OK;
+    }
+    cudaGetLastError();
+    cudaFree(*out);
+    *out = nullptr;
+    if (e != cudaSuccess && e != cudaErrorMemoryAllocation)
+    {
+        h->err = std::string("wide BVH: ") + cudaGetErrorString(e);
+        return RC_CUDA;
+    }
+    if (got.error)
+    {
+        h->err = "wide BVH: malformed binary node links";
+        return RC_DEVICE_ERROR;
+    }
+    return RC_OK;  // stays binary
+}
+
+// The meshes' trees, the top-level one and the instances' mesh roots.
+rc_status ensure_wide_instanced(rc_tracer* h)
+{
+    std::vector<int32_t> roots;  // inner mesh roots, each once
+    for (int32_t r : h->instRoots)
+        if (r >= 0)
+            roots.push_back(r);
+    std::sort(roots.begin(), roots.end());
+    roots.erase(std::unique(roots.begin(), roots.end()), roots.end());
+    std::vector<int32_t> wideRoots;
+    for (int32_t r : h->instRoots)
+        wideRoots.push_back(
+            r < 0 ? r : int32_t(std::lower_bound(roots.begin(), roots.end(), r) - roots.begin()));
+    const int levels = int(std::min<uint64_t>(h->bvhDepth, kMaxStack));
+    int needMesh = 0, needTop = 0;
+    rc_status s = RC_OK;
+    if (!roots.empty() &&
+        ((s = collapse(h, h->dNodes, h->innerCount, roots, levels, kTwoLevelStack, &h->dWide, &needMesh)) != RC_OK ||
+         !h->dWide))
+        return s;
+    h->wideCount = h->dWide ? h->innerCount : 0;
+    h->deviceBytes += h->wideCount * sizeof(DevNode4);
+    h->wideTlasRoot = h->tlasRoot;
+    if (h->tlasRoot >= 0)
+    {
+        s = collapse(h, h->dTlas, h->tlasCount, { h->tlasRoot }, levels, kTwoLevelStack, &h->dWideTlas, &needTop);
+        if (s != RC_OK || !h->dWideTlas)
+            return s;
+        h->wideTlasRoot = 0;
+        h->wideTlasCount = h->tlasCount;
+        h->deviceBytes += h->wideTlasCount * sizeof(DevNode4);
+    }
+    // a leaf of two instances stacks its second one
+    if (needMesh + needTop + 1 > kTwoLevelStack)
+        return RC_OK;  // stays binary
+    cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&h->dInstWide), wideRoots.size() * sizeof(int32_t));
+    if (e == cudaSuccess)
+    {
+        h->deviceBytes += wideRoots.size() * sizeof(int32_t);
+        e = cudaMemcpy(h->dInstWide, wideRoots.data(), wideRoots.size() * sizeof(int32_t), cudaMemcpyHostToDevice);
+    }
+    if (e != cudaSuccess)
+    {
+        cudaGetLastError();
+        if (e == cudaErrorMemoryAllocation)
+            return RC_OK;
+        h->err = std::string("wide BVH: ") + cudaGetErrorString(e);
+        return RC_CUDA;
+    }
+    h->wideInstanced = true;
+    return RC_OK;
+}
+
+}  // namespace
+
+rc_status ensure_wide(rc_tracer* h)
+{
+    if (h->wideTried || !h->sceneReady)
+        return RC_OK;
+    h->wideTried = true;
+    h->wideRoot = h->rootLink;
+    static const bool enabled = [] {
+        const char* v = std::getenv("RC_WIDE_BVH");
+        return !(v && v[0] == '0');
+    }();
+    if (!enabled)
+        return RC_OK;
+    if (h->nInstances > 0)
+        return ensure_wide_instanced(h);
+    if (h->rootLink < 0)
+        return RC_OK;  // a leaf root: nothing to collapse
+    int need = 0;
+    const rc_status s = collapse(h, h->dNodes, h->innerCount, { h->rootLink }, int(h->bvhDepth), kMaxStack, &h->dWide,
+                                 &need);
+    if (s != RC_OK || !h->dWide)
+        return s;
+    h->wideCount = h->innerCount;
+    h->wideRoot = 0;
+    h->deviceBytes += h->wideCount * sizeof(DevNode4);
+    return RC_OK;
+}
+
+}  // namespace rcx
