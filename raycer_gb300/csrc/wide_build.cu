@@ -33,107 +33,13 @@ namespace
 
 constexpr int kBlock = 128;
 
-struct Child
-{
-    int link;
-    float lo[3];
-    float hi[3];
-};
-
-__device__ __forceinline__ void children_of(const DevNode& n, Child& a, Child& b)
-{
-    a = Child{ n.link.x, { n.xy0.x, n.xy0.z, n.z01.x }, { n.xy0.y, n.xy0.w, n.z01.y } };
-    b = Child{ n.link.y, { n.xy1.x, n.xy1.z, n.z01.z }, { n.xy1.y, n.xy1.w, n.z01.w } };
-}
-
-__device__ __forceinline__ float half_area(const Child& c)
-{
-    const float dx = fmaxf(0.0f, c.hi[0] - c.lo[0]);
-    const float dy = fmaxf(0.0f, c.hi[1] - c.lo[1]);
-    const float dz = fmaxf(0.0f, c.hi[2] - c.lo[2]);
-    return dx * dy + dy * dz + dz * dx;
-}
-
 __global__ void __launch_bounds__(kBlock) k_collapse(const DevNode* __restrict__ nodes, int count,
                                                      WideItem* __restrict__ items, DevNode4* __restrict__ wide,
                                                      WideCounters* c, int level)
 {
-    const int end = c->bound[level + 1];
+    const int end = level_end(*c, level, count);
     for (int i = c->bound[level] + int(blockIdx.x) * kBlock + int(threadIdx.x); i < end; i += int(gridDim.x) * kBlock)
-    {
-        const WideItem it = items[i];
-        Child ch[4];
-        int n = 2;
-        children_of(nodes[it.bin], ch[0], ch[1]);
-        bool bad = false;
-        while (n < 4)
-        {
-            int best = -1;
-            float bestA = -1.0f;
-            for (int k = 0; k < n; ++k)
-                if (ch[k].link >= 0 && half_area(ch[k]) > bestA)
-                {
-                    best = k;
-                    bestA = half_area(ch[k]);
-                }
-            if (best < 0)
-                break;
-            if (ch[best].link >= count)
-            {
-                bad = true;
-                break;
-            }
-            Child x, y;
-            children_of(nodes[ch[best].link], x, y);
-            ch[best] = x;
-            ch[n++] = y;
-        }
-        int inner = 0;
-        for (int k = 0; k < n; ++k)
-        {
-            if (ch[k].link >= count)
-                bad = true;
-            if (ch[k].link >= 0)
-                inner++;
-        }
-        int node = bad ? 0 : atomicAdd(&c->nodes, inner);
-        if (bad || node + inner > count)
-        {
-            c->error = 1;  // links that are no tree
-            continue;
-        }
-        const int need = it.need + (n - 1);
-        atomicMax(&c->maxNeed, need);
-        DevNode4 w{};
-        float* lox = &w.lox.x;
-        float* hix = &w.hix.x;
-        float* loy = &w.loy.x;
-        float* hiy = &w.hiy.x;
-        float* loz = &w.loz.x;
-        float* hiz = &w.hiz.x;
-        int* link = &w.link.x;
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-        {
-            if (k >= n)
-                break;
-            lox[k] = ch[k].lo[0];
-            hix[k] = ch[k].hi[0];
-            loy[k] = ch[k].lo[1];
-            hiy[k] = ch[k].hi[1];
-            loz[k] = ch[k].lo[2];
-            hiz[k] = ch[k].hi[2];
-            if (ch[k].link >= 0)
-            {
-                items[node] = WideItem{ ch[k].link, need };
-                link[k] = node++;
-                continue;
-            }
-            link[k] = ch[k].link;
-        }
-        w.meta.x = n;
-        wide[i] = w;
-    }
+        collapse_node(nodes, count, items, wide, c, i);
 }
 
 // Closes the level just taken.

@@ -1,8 +1,12 @@
-// Records and launches of the 4-wide trees' construction: the kernels are in
-// wide_build.cu, the host side in wide_host.cpp.
+// Records, per-node steps and launches of the 4-wide trees' construction: the
+// kernels are in wide_build.cu, the host side in wide_host.cpp. Links that are
+// no tree (an index outside the nodes, more nodes than there are) are found
+// before they are followed, and set `error`.
 #pragma once
 
 #include <cuda_runtime.h>
+
+#include <math.h>
 
 #include "device_types.h"
 
@@ -25,6 +29,124 @@ struct WideItem
     int bin;   // its binary inner node
     int need;  // stack entries pushed above it
 };
+
+struct WideChild
+{
+    int link;
+    float lo[3];
+    float hi[3];
+};
+
+__host__ __device__ inline void children_of(const DevNode& n, WideChild& a, WideChild& b)
+{
+    a = WideChild{ n.link.x, { n.xy0.x, n.xy0.z, n.z01.x }, { n.xy0.y, n.xy0.w, n.z01.y } };
+    b = WideChild{ n.link.y, { n.xy1.x, n.xy1.z, n.z01.z }, { n.xy1.y, n.xy1.w, n.z01.w } };
+}
+
+__host__ __device__ inline float half_area(const WideChild& c)
+{
+    const float dx = fmaxf(0.0f, c.hi[0] - c.lo[0]);
+    const float dy = fmaxf(0.0f, c.hi[1] - c.lo[1]);
+    const float dz = fmaxf(0.0f, c.hi[2] - c.lo[2]);
+    return dx * dy + dy * dz + dz * dx;
+}
+
+// Children of the wide node of binary node `bin`, and how many: 2 to 4, or 0
+// where a link is no index of the `count` nodes.
+__host__ __device__ inline int wide_children(const DevNode* nodes, int count, int bin, WideChild* ch)
+{
+    if (bin < 0 || bin >= count)
+        return 0;
+    int n = 2;
+    children_of(nodes[bin], ch[0], ch[1]);
+    while (n < 4)
+    {
+        int best = -1;
+        float bestA = -1.0f;
+        for (int k = 0; k < n; ++k)
+            if (ch[k].link >= 0 && half_area(ch[k]) > bestA)
+            {
+                best = k;
+                bestA = half_area(ch[k]);
+            }
+        if (best < 0)
+            break;
+        if (ch[best].link >= count)
+            return 0;
+        WideChild x, y;
+        children_of(nodes[ch[best].link], x, y);
+        ch[best] = x;
+        ch[n++] = y;
+    }
+    for (int k = 0; k < n; ++k)
+        if (ch[k].link >= count)
+            return 0;
+    return n;
+}
+
+// The nodes of a level: [bound[level], level_end). None once links are no
+// tree: the count of nodes may then be past the arrays.
+__host__ __device__ inline int level_end(const WideCounters& c, int level, int count)
+{
+    return c.error || c.bound[level + 1] > count ? 0 : c.bound[level + 1];
+}
+
+// Takes wide node i: chooses its children, takes consecutive nodes of the next
+// level for the inner ones (one atomic) and writes it.
+__host__ __device__ inline void collapse_node(const DevNode* nodes, int count, WideItem* items, DevNode4* wide,
+                                              WideCounters* c, int i)
+{
+    const WideItem it = items[i];
+    WideChild ch[4];
+    const int n = wide_children(nodes, count, it.bin, ch);
+    int inner = 0;
+    for (int k = 0; k < n; ++k)
+        inner += ch[k].link >= 0 ? 1 : 0;
+#ifdef __CUDA_ARCH__
+    int node = n > 0 ? atomicAdd(&c->nodes, inner) : 0;
+#else
+    int node = c->nodes;
+    c->nodes += inner;
+#endif
+    if (n == 0 || node + inner > count)
+    {
+        c->error = 1;
+        return;
+    }
+    const int need = it.need + (n - 1);
+#ifdef __CUDA_ARCH__
+    atomicMax(&c->maxNeed, need);
+#else
+    c->maxNeed = need > c->maxNeed ? need : c->maxNeed;
+#endif
+    DevNode4 w{};
+    float* lox = &w.lox.x;
+    float* hix = &w.hix.x;
+    float* loy = &w.loy.x;
+    float* hiy = &w.hiy.x;
+    float* loz = &w.loz.x;
+    float* hiz = &w.hiz.x;
+    int* link = &w.link.x;
+    for (int k = 0; k < 4; ++k)
+    {
+        if (k >= n)
+            break;
+        lox[k] = ch[k].lo[0];
+        hix[k] = ch[k].hi[0];
+        loy[k] = ch[k].lo[1];
+        hiy[k] = ch[k].hi[1];
+        loz[k] = ch[k].lo[2];
+        hiz[k] = ch[k].hi[2];
+        link[k] = ch[k].link;
+        if (ch[k].link >= 0)
+        {
+            items[node] = WideItem{ ch[k].link, need };
+            link[k] = node++;
+        }
+    }
+    w.meta.x = n;
+    wide[i] = w;
+}
 
 // One level of a collapse: closes the level above and takes its nodes, at
 // most `most` of them.

@@ -22,7 +22,7 @@ def _cuda_home() -> Path | None:
 @pytest.mark.skipif(shutil.which("g++") is None or _cuda_home() is None, reason="no C++ compiler or CUDA headers")
 def test_wide_build_on_the_host(tmp_path):
     exe = tmp_path / "wide_build_check"
-    subprocess.run(["g++", "-std=c++17", "-O1", "-g", f"-I{_cuda_home() / 'include'}",
+    subprocess.run(["g++", "-std=c++17", "-O1", "-g", "-fsanitize=address", f"-I{_cuda_home() / 'include'}",
                     str(ROOT / "tests" / "wide_build_check.cpp"), "-o", str(exe)], check=True)
     out = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
     assert out.returncode == 0, out.stdout + out.stderr

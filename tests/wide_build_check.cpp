@@ -1,5 +1,6 @@
 // Host check of wide_host.cpp against a CUDA runtime whose device is host
-// memory: allocations can be made to fail, kernels do nothing.
+// memory: allocations can be made to fail, and a level of nodes is taken one
+// by one, with the kernels' own steps. Built with the address sanitizer.
 
 #include <cuda_runtime.h>
 
@@ -7,6 +8,9 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <random>
+#include <utility>
+#include <vector>
 
 #include "../raycer_gb300/csrc/wide_host.cpp"
 
@@ -63,8 +67,12 @@ extern "C"
 namespace rcx
 {
 
-cudaError_t launch_collapse(const DevNode*, int, WideItem*, DevNode4*, WideCounters*, int, size_t, int, cudaStream_t)
+cudaError_t launch_collapse(const DevNode* nodes, int count, WideItem* items, DevNode4* wide, WideCounters* c,
+                            int level, size_t, int, cudaStream_t)
 {
+    c->bound[level + 1] = c->nodes;
+    for (int i = c->bound[level]; i < level_end(*c, level, count); ++i)
+        collapse_node(nodes, count, items, wide, c, i);
     return cudaSuccess;
 }
 
@@ -84,51 +92,183 @@ int failures = 0;
         }                                                      \
     } while (0)
 
-// A tracer with a scene of `count` inner nodes.
-void scene(rc_tracer& h, size_t count, int instances)
+// A random binary tree of `count` inner nodes in preorder (leaf codes
+// ~(slot << 4 | 1), slots in order), its boxes nested.
+std::vector<rcx::DevNode> random_tree(int count, unsigned seed)
+{
+    std::mt19937 rng(seed);
+    std::vector<rcx::DevNode> nodes(static_cast<size_t>(count));
+    int next = 0, leaf = 0;
+    // inner nodes of the subtree at `node`, its box
+    struct Box
+    {
+        float lo[3], hi[3];
+    };
+    auto grow = [&](auto&& self, int inner, Box box) -> int {
+        const int me = next++;
+        const int left = int(rng() % unsigned(inner));  // of the inner - 1 others
+        const int n[2] = { left, inner - 1 - left };
+        for (int k = 0; k < 2; ++k)
+        {
+            Box b = box;
+            const int axis = int(rng() % 3);
+            (k ? b.lo : b.hi)[axis] = b.lo[axis] + (b.hi[axis] - b.lo[axis]) * (0.3f + 0.4f * float(rng() % 1000) / 1000.0f);
+            (k ? nodes[size_t(me)].xy1 : nodes[size_t(me)].xy0) = make_float4(b.lo[0], b.hi[0], b.lo[1], b.hi[1]);
+            (k ? nodes[size_t(me)].z01.z : nodes[size_t(me)].z01.x) = b.lo[2];
+            (k ? nodes[size_t(me)].z01.w : nodes[size_t(me)].z01.y) = b.hi[2];
+            int link = ~((leaf << rcx::kLeafCountBits) | 1);
+            if (n[k] > 0)
+                link = self(self, n[k], b);
+            else
+                leaf++;
+            (k ? nodes[size_t(me)].link.y : nodes[size_t(me)].link.x) = link;
+        }
+        return me;
+    };
+    grow(grow, count, Box{ { -1.0f, -1.0f, -1.0f }, { 1.0f, 1.0f, 1.0f } });
+    return nodes;
+}
+
+int depth_of(const std::vector<rcx::DevNode>& nodes, int link)
+{
+    if (link < 0)
+        return 1;
+    return 1 + std::max(depth_of(nodes, nodes[size_t(link)].link.x), depth_of(nodes, nodes[size_t(link)].link.y));
+}
+
+// A tracer with a scene of these inner nodes (also the two-level scene's top level).
+void scene(rc_tracer& h, std::vector<rcx::DevNode>& nodes, int levels, int instances)
 {
     h.sceneReady = true;
     h.numSMs = 4;
-    h.innerCount = count;
+    h.innerCount = nodes.size();
     h.rootLink = 0;
-    h.bvhDepth = 12;
-    rcx::DevNode* nodes = static_cast<rcx::DevNode*>(std::calloc(count, sizeof(rcx::DevNode)));
-    h.dNodes = nodes;
+    h.bvhDepth = uint64_t(levels);
+    h.dNodes = nodes.data();
     h.nInstances = instances;
     h.tlasRoot = 0;
-    h.tlasCount = count;
-    h.dTlas = nodes;
+    h.tlasCount = nodes.size();
+    h.dTlas = nodes.data();
     h.instRoots.assign(size_t(instances), 0);
+}
+
+void release(rc_tracer& h)
+{
+    cudaFree(h.dWide);
+    cudaFree(h.dWideTlas);
+    cudaFree(h.dInstWide);
+    CHECK(live.empty());
+}
+
+// Leaf slots below a wide node in preorder of the binary tree, and that every
+// inner node of the binary tree is opened or a wide node's own.
+void leaves(const rcx::DevNode4* wide, int link, std::vector<int>& out)
+{
+    if (link < 0)
+    {
+        out.push_back((~link) >> rcx::kLeafCountBits);
+        return;
+    }
+    const int n = wide[link].meta.x;
+    CHECK(n >= 2 && n <= 4);
+    const int* l = &wide[link].link.x;
+    for (int k = 0; k < n; ++k)
+        leaves(wide, l[k], out);
+}
+
+void valid_trees()
+{
+    for (int count : { 1, 2, 3, 7, 50, 400 })
+        for (unsigned seed = 1; seed <= 5; ++seed)
+        {
+            std::vector<rcx::DevNode> nodes = random_tree(count, seed);
+            const int levels = depth_of(nodes, 0);
+            if (levels > rcx::kMaxStack)
+                continue;
+            rc_tracer h;
+            scene(h, nodes, levels, 0);
+            failAt = 0;
+            CHECK(rcx::ensure_wide(&h) == RC_OK);
+            if (h.dWide)
+            {
+                std::vector<int> slots;
+                leaves(h.dWide, h.wideRoot, slots);
+                std::sort(slots.begin(), slots.end());
+                CHECK(int(slots.size()) == count + 1);
+                for (int i = 0; i < int(slots.size()); ++i)
+                    CHECK(slots[size_t(i)] == i);
+            }
+            CHECK(live_bytes() == h.deviceBytes);
+            release(h);
+        }
+}
+
+// Links that are no tree: reported, and nothing outside the arrays is read or
+// written (the address sanitizer).
+void malformed_links()
+{
+    for (unsigned seed = 1; seed <= 40; ++seed)
+    {
+        std::mt19937 rng(seed);
+        const int count = 2 + int(rng() % 60);
+        std::vector<rcx::DevNode> nodes = random_tree(count, seed);
+        const int levels = rcx::kMaxStack;
+        const size_t at = rng() % nodes.size();
+        int& link = (rng() & 1) ? nodes[at].link.x : nodes[at].link.y;
+        switch (seed % 4)
+        {
+        case 0: link = count; break;                // past the nodes
+        case 1: link = count + 1000000; break;
+        case 2: link = 0; break;                    // a cycle
+        default:                                    // every node twice
+            for (int i = 0; i + 1 < count; ++i)
+                nodes[size_t(i)].link = make_int4(i + 1, i + 1, 0, 0);
+        }
+        rc_tracer h;
+        scene(h, nodes, levels, 0);
+        failAt = 0;
+        const rc_status s = rcx::ensure_wide(&h);
+        CHECK(s == RC_DEVICE_ERROR || (s == RC_OK && !h.dWide));
+        if (seed % 4 < 2)
+            CHECK(s == RC_DEVICE_ERROR);
+        release(h);
+    }
+    // roots outside the nodes
+    for (int root : { 50, 1 << 30 })
+    {
+        std::vector<rcx::DevNode> nodes = random_tree(50, 1);
+        rc_tracer h;
+        scene(h, nodes, rcx::kMaxStack, 2);
+        h.instRoots[1] = root;
+        CHECK(rcx::ensure_wide(&h) == RC_DEVICE_ERROR);
+        release(h);
+    }
 }
 
 // Without memory for a 4-wide tree a scene stays binary: no error, nothing
 // left behind, and the next call neither fails nor tries again.
 void allocation_failures()
 {
+    std::vector<rcx::DevNode> nodes = random_tree(400, 1);
     for (int instances : { 0, 3 })
         for (int at = 1; at <= 6; ++at)
         {
             rc_tracer h;
-            scene(h, 1000, instances);
+            scene(h, nodes, depth_of(nodes, 0), instances);
             allocations = 0;
             failAt = at;
             failWith = cudaErrorMemoryAllocation;
             CHECK(rcx::ensure_wide(&h) == RC_OK);
             CHECK(h.err.empty());
-            if (instances == 0)
-                CHECK(!h.dWide);
-            else
-                CHECK(!h.wideInstanced);
+            if (allocations >= failAt)
+                CHECK(instances == 0 ? !h.dWide : !h.wideInstanced);
             CHECK(live_bytes() == h.deviceBytes);
             CHECK(rcx::ensure_wide(&h) == RC_OK);
-            cudaFree(h.dWide);
-            cudaFree(h.dWideTlas);
-            cudaFree(h.dInstWide);
-            CHECK(live.empty());
+            release(h);
         }
     // another error is reported
     rc_tracer h;
-    scene(h, 1000, 0);
+    scene(h, nodes, depth_of(nodes, 0), 0);
     allocations = 0;
     failAt = 1;
     failWith = cudaErrorUnknown;
@@ -140,6 +280,8 @@ void allocation_failures()
 
 int main()
 {
+    valid_trees();
+    malformed_links();
     allocation_failures();
     if (!failures)
         std::printf("wide build ok\n");
