@@ -43,11 +43,11 @@ __host__ __device__ inline void children_of(const DevNode& n, WideChild& a, Wide
     b = WideChild{ n.link.y, { n.xy1.x, n.xy1.z, n.z01.z }, { n.xy1.y, n.xy1.w, n.z01.w } };
 }
 
-__host__ __device__ inline float half_area(const WideChild& c)
+__host__ __device__ inline double half_area(const WideChild& c)
 {
-    const float dx = fmaxf(0.0f, c.hi[0] - c.lo[0]);
-    const float dy = fmaxf(0.0f, c.hi[1] - c.lo[1]);
-    const float dz = fmaxf(0.0f, c.hi[2] - c.lo[2]);
+    const double dx = fmax(0.0, double(c.hi[0]) - double(c.lo[0]));
+    const double dy = fmax(0.0, double(c.hi[1]) - double(c.lo[1]));
+    const double dz = fmax(0.0, double(c.hi[2]) - double(c.lo[2]));
     return dx * dy + dy * dz + dz * dx;
 }
 
@@ -62,7 +62,7 @@ __host__ __device__ inline int wide_children(const DevNode* nodes, int count, in
     while (n < 4)
     {
         int best = -1;
-        float bestA = -1.0f;
+        double bestA = -1.0;
         for (int k = 0; k < n; ++k)
             if (ch[k].link >= 0 && half_area(ch[k]) > bestA)
             {

@@ -1,6 +1,8 @@
-"""The 4-wide trees' construction (wide_host.cpp) on the host, against a CUDA
-runtime whose device is host memory (wide_build_check.cu): scenes for whose
-trees there is no memory stay binary."""
+"""The 4-wide trees' construction (wide_host.cpp, wide_collapse.h) on the host,
+against a CUDA runtime whose device is host memory (wide_build_check.cpp, with
+the address sanitizer): random trees keep their leaves; the child of largest
+area is opened; links that are no tree are reported and never followed; scenes
+for whose trees there is no memory stay binary."""
 
 from __future__ import annotations
 

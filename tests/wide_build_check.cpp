@@ -203,6 +203,31 @@ void valid_trees()
         }
 }
 
+// A wide node opens its child of largest area, compared in 64 bits: of two
+// boxes of 16 x 16 x 1 and 16 x 16 x (1 + 2^-23), whose areas round to one
+// 32-bit value, the second.
+void largest_area()
+{
+    auto node = [](float h0, int l0, float h1, int l1) {
+        rcx::DevNode n{};
+        n.xy0 = n.xy1 = make_float4(0.0f, 16.0f, 0.0f, 16.0f);
+        n.z01 = make_float4(0.0f, h0, 0.0f, h1);
+        n.link = make_int4(l0, l1, 0, 0);
+        return n;
+    };
+    auto leaf = [](int slot) { return ~((slot << rcx::kLeafCountBits) | 1); };
+    const float more = 1.0f + 1.0f / 8388608.0f;
+    // 0: the large 1 and the box of 2; 1: the box of 3 and a leaf
+    const std::vector<rcx::DevNode> nodes{ node(8.0f, 1, more, 2), node(1.0f, 3, 0.5f, leaf(0)),
+                                           node(0.1f, leaf(1), 0.1f, leaf(2)), node(0.1f, leaf(3), 0.1f, leaf(4)) };
+    rcx::WideChild ch[4];
+    CHECK(rcx::wide_children(nodes.data(), 4, 0, ch) == 4);
+    bool box3 = false;
+    for (const rcx::WideChild& c : ch)
+        box3 |= c.link == 3;
+    CHECK(box3);  // left as it is: the box of 2 is opened
+}
+
 // Links that are no tree: reported, and nothing outside the arrays is read or
 // written (the address sanitizer).
 void malformed_links()
@@ -281,6 +306,7 @@ void allocation_failures()
 int main()
 {
     valid_trees();
+    largest_area();
     malformed_links();
     allocation_failures();
     if (!failures)
