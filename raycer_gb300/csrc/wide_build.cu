@@ -15,10 +15,12 @@
 //
 // One launch per level: thread i takes the i-th wide node of the level,
 // chooses its children and takes consecutive nodes of the next level for the
-// inner ones (one atomic). What bounds it is the chain of levels, two
-// launches each. A scene's first PATH frame, the collapse included (on the
-// host before: nodes downloaded, collapsed, uploaded): 1M triangles
-// 10.6 -> 2.3 ms, 5M triangles 67.8 -> 5.7 ms.
+// inner ones (one atomic). The nodes are written once their number is known,
+// into an array of just that many (111,096 for the 275,270 binary nodes of
+// 1M triangles of terrain). What bounds it is the chain of levels. A scene's
+// first PATH frame, the collapse included (on the host before: nodes
+// downloaded, collapsed, uploaded): 1M triangles 10.6 -> 2.3 ms, 5M triangles
+// 67.8 -> 5.7 ms.
 
 #include <cuda_runtime.h>
 
@@ -33,26 +35,45 @@ namespace
 
 constexpr int kBlock = 128;
 
+// Takes a level's nodes; the last block closes the level they go to.
 __global__ void __launch_bounds__(kBlock) k_collapse(const DevNode* __restrict__ nodes, int count,
-                                                     WideItem* __restrict__ items, DevNode4* __restrict__ wide,
-                                                     WideCounters* c, int level)
+                                                     WideItem* __restrict__ items, WideCounters* c, int level)
 {
     const int end = level_end(*c, level, count);
     for (int i = c->bound[level] + int(blockIdx.x) * kBlock + int(threadIdx.x); i < end; i += int(gridDim.x) * kBlock)
-        collapse_node(nodes, count, items, wide, c, i);
+        collapse_node(nodes, count, items, c, i);
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        __threadfence();
+        if (atomicAdd(&c->blocks[level], 1) == int(gridDim.x) - 1)
+            c->bound[level + 2] = atomicAdd(&c->nodes, 0);
+    }
 }
 
-// Closes the level just taken.
-__global__ void k_collapse_level(WideCounters* c, int level) { c->bound[level + 1] = c->nodes; }
+__global__ void __launch_bounds__(kBlock) k_write_nodes(const DevNode* __restrict__ nodes,
+                                                        const WideItem* __restrict__ items,
+                                                        DevNode4* __restrict__ wide, int taken)
+{
+    const int i = int(blockIdx.x) * kBlock + int(threadIdx.x);
+    if (i < taken)
+        write_node(nodes, items, wide, i);
+}
 
 }  // namespace
 
-cudaError_t launch_collapse(const DevNode* nodes, int count, WideItem* items, DevNode4* wide, WideCounters* c,
-                            int level, size_t most, int numSMs, cudaStream_t stream)
+cudaError_t launch_collapse(const DevNode* nodes, int count, WideItem* items, WideCounters* c, int level, size_t most,
+                            int numSMs, cudaStream_t stream)
 {
-    k_collapse_level<<<1, 1, 0, stream>>>(c, level);
     const unsigned blocks = unsigned(std::min<size_t>((most + kBlock - 1) / kBlock, size_t(numSMs) * 16));
-    k_collapse<<<blocks, kBlock, 0, stream>>>(nodes, count, items, wide, c, level);
+    k_collapse<<<blocks, kBlock, 0, stream>>>(nodes, count, items, c, level);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_write_nodes(const DevNode* nodes, const WideItem* items, DevNode4* wide, int taken,
+                               cudaStream_t stream)
+{
+    k_write_nodes<<<unsigned((taken + kBlock - 1) / kBlock), kBlock, 0, stream>>>(nodes, items, wide, taken);
     return cudaGetLastError();
 }
 

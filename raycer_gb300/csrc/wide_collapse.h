@@ -21,13 +21,16 @@ struct WideCounters
     int maxNeed;  // stack entries pushed on the worst root-to-leaf path
     int error;    // malformed binary links
     int bound[kMaxStack + 2];
+    int blocks[kMaxStack];  // blocks of the level's launch that are done
 };
 
 // What a wide node is made from.
 struct WideItem
 {
-    int bin;   // its binary inner node
-    int need;  // stack entries pushed above it
+    int bin;     // its binary inner node
+    int need;    // stack entries pushed above it
+    int child;   // its first inner child; the others follow
+    int opened;  // the children opened, 4 bits each (index + 1), in order
 };
 
 struct WideChild
@@ -51,10 +54,20 @@ __host__ __device__ inline double half_area(const WideChild& c)
     return dx * dy + dy * dz + dz * dx;
 }
 
-// Children of the wide node of binary node `bin`, and how many: 2 to 4, or 0
-// where a link is no index of the `count` nodes.
-__host__ __device__ inline int wide_children(const DevNode* nodes, int count, int bin, WideChild* ch)
+// Replaces child `k` of n by its own children.
+__host__ __device__ inline void open_child(const DevNode* nodes, WideChild* ch, int& n, int k)
 {
+    WideChild x, y;
+    children_of(nodes[ch[k].link], x, y);
+    ch[k] = x;
+    ch[n++] = y;
+}
+
+// Children of the wide node of binary node `bin`, and how many: 2 to 4, or 0
+// where a link is no index of the `count` nodes; the ones opened in `opened`.
+__host__ __device__ inline int wide_children(const DevNode* nodes, int count, int bin, WideChild* ch, int& opened)
+{
+    opened = 0;
     if (bin < 0 || bin >= count)
         return 0;
     int n = 2;
@@ -73,10 +86,8 @@ __host__ __device__ inline int wide_children(const DevNode* nodes, int count, in
             break;
         if (ch[best].link >= count)
             return 0;
-        WideChild x, y;
-        children_of(nodes[ch[best].link], x, y);
-        ch[best] = x;
-        ch[n++] = y;
+        opened |= (best + 1) << (4 * (n - 2));
+        open_child(nodes, ch, n, best);
     }
     for (int k = 0; k < n; ++k)
         if (ch[k].link >= count)
@@ -91,14 +102,14 @@ __host__ __device__ inline int level_end(const WideCounters& c, int level, int c
     return c.error || c.bound[level + 1] > count ? 0 : c.bound[level + 1];
 }
 
-// Takes wide node i: chooses its children, takes consecutive nodes of the next
-// level for the inner ones (one atomic) and writes it.
-__host__ __device__ inline void collapse_node(const DevNode* nodes, int count, WideItem* items, DevNode4* wide,
-                                              WideCounters* c, int i)
+// Takes wide node i: takes consecutive nodes of the next level for the inner
+// ones of its children (one atomic).
+__host__ __device__ inline void collapse_node(const DevNode* nodes, int count, WideItem* items, WideCounters* c, int i)
 {
     const WideItem it = items[i];
     WideChild ch[4];
-    const int n = wide_children(nodes, count, it.bin, ch);
+    int opened;
+    const int n = wide_children(nodes, count, it.bin, ch, opened);
     int inner = 0;
     for (int k = 0; k < n; ++k)
         inner += ch[k].link >= 0 ? 1 : 0;
@@ -119,6 +130,23 @@ __host__ __device__ inline void collapse_node(const DevNode* nodes, int count, W
 #else
     c->maxNeed = need > c->maxNeed ? need : c->maxNeed;
 #endif
+    items[i].child = node;
+    items[i].opened = opened;
+    for (int k = 0; k < n; ++k)
+        if (ch[k].link >= 0)
+            items[node++] = WideItem{ ch[k].link, need, 0, 0 };
+}
+
+// Writes wide node i of a tree that collapse_node has taken without an error.
+__host__ __device__ inline void write_node(const DevNode* nodes, const WideItem* items, DevNode4* wide, int i)
+{
+    const WideItem it = items[i];
+    WideChild ch[4];
+    int n = 2;
+    children_of(nodes[it.bin], ch[0], ch[1]);
+    for (int o = it.opened; o != 0; o >>= 4)
+        open_child(nodes, ch, n, (o & 15) - 1);
+    int node = it.child;
     DevNode4 w{};
     float* lox = &w.lox.x;
     float* hix = &w.hix.x;
@@ -127,30 +155,25 @@ __host__ __device__ inline void collapse_node(const DevNode* nodes, int count, W
     float* loz = &w.loz.x;
     float* hiz = &w.hiz.x;
     int* link = &w.link.x;
-    for (int k = 0; k < 4; ++k)
+    for (int k = 0; k < n; ++k)
     {
-        if (k >= n)
-            break;
         lox[k] = ch[k].lo[0];
         hix[k] = ch[k].hi[0];
         loy[k] = ch[k].lo[1];
         hiy[k] = ch[k].hi[1];
         loz[k] = ch[k].lo[2];
         hiz[k] = ch[k].hi[2];
-        link[k] = ch[k].link;
-        if (ch[k].link >= 0)
-        {
-            items[node] = WideItem{ ch[k].link, need };
-            link[k] = node++;
-        }
+        link[k] = ch[k].link >= 0 ? node++ : ch[k].link;
     }
     w.meta.x = n;
     wide[i] = w;
 }
 
-// One level of a collapse: closes the level above and takes its nodes, at
-// most `most` of them.
-cudaError_t launch_collapse(const DevNode* nodes, int count, WideItem* items, DevNode4* wide, WideCounters* c,
-                            int level, size_t most, int numSMs, cudaStream_t stream);
+// One level of a collapse: takes its nodes, at most `most`, and closes the next.
+cudaError_t launch_collapse(const DevNode* nodes, int count, WideItem* items, WideCounters* c, int level, size_t most,
+                            int numSMs, cudaStream_t stream);
+// The taken nodes, written.
+cudaError_t launch_write_nodes(const DevNode* nodes, const WideItem* items, DevNode4* wide, int taken,
+                               cudaStream_t stream);
 
 }  // namespace rcx

@@ -21,24 +21,36 @@ namespace rcx
 namespace
 {
 
-// Collapses the trees of `roots` (inner links into nodes[0, count)) into one
-// array of 4-wide nodes, root i at index i. *out stays null where the stack
-// need (*need) is above `maxNeed`, or where there is no memory.
-rc_status collapse(rc_tracer* h, const DevNode* nodes, size_t count, const std::vector<int32_t>& roots, int levels,
-                   int maxNeed, DevNode4** out, int* need)
+// A collapsed tree.
+struct WideTree
 {
-    *out = nullptr;
+    DevNode4* nodes = nullptr;  // null: none, the scene stays binary
+    size_t count = 0;
+    int need = 0;  // stack entries of a walk
+};
+
+void release(WideTree& t)
+{
+    cudaFree(t.nodes);
+    t = WideTree{};
+}
+
+// Collapses the trees of `roots` (inner links into nodes[0, count)) into one
+// array of 4-wide nodes, root i at index i. None where the stack need is above
+// `maxNeed`, or where there is no memory.
+rc_status collapse(rc_tracer* h, const DevNode* nodes, size_t count, const std::vector<int32_t>& roots, int levels,
+                   int maxNeed, WideTree& out)
+{
     WideItem* items = nullptr;
     WideCounters* counters = nullptr;
     WideCounters got{};
     std::vector<WideItem> first(roots.size());
     for (size_t i = 0; i < roots.size(); ++i)
-        first[i] = WideItem{ roots[i], 0 };
-    got.nodes = int(roots.size());
+        first[i] = WideItem{ roots[i], 0, 0, 0 };
+    got.nodes = got.bound[1] = int(roots.size());
     // a wide node stands for one binary inner node
-    cudaError_t e = cudaMalloc(reinterpret_cast<void**>(out), count * sizeof(DevNode4));
-    if (e == cudaSuccess)
-        e = cudaMalloc(reinterpret_cast<void**>(&items), count * sizeof(WideItem) + sizeof(WideCounters));
+    cudaError_t e =
+        cudaMalloc(reinterpret_cast<void**>(&items), count * sizeof(WideItem) + sizeof(WideCounters));
     if (e == cudaSuccess)
     {
         counters = reinterpret_cast<WideCounters*>(items + count);
@@ -51,21 +63,28 @@ rc_status collapse(rc_tracer* h, const DevNode* nodes, size_t count, const std::
     {
         // at most 4^level nodes per root
         const size_t most = level < 12 ? std::min(count, roots.size() << (2 * level)) : count;
-        e = launch_collapse(nodes, int(count), items, *out, counters, level, most, h->numSMs, h->stream);
+        e = launch_collapse(nodes, int(count), items, counters, level, most, h->numSMs, h->stream);
     }
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(&got, counters, sizeof(got), cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(h->stream);
-    cudaFree(items);
-    if (e == cudaSuccess && !got.error && got.maxNeed <= maxNeed && got.nodes == got.bound[levels])
+    const bool fits = e == cudaSuccess && !got.error && got.maxNeed <= maxNeed && got.nodes == got.bound[levels];
+    if (fits)
     {
-        *need = got.maxNeed;
-        return RC_OK;
+        out.count = size_t(got.nodes);
+        out.need = got.maxNeed;
+        e = cudaMalloc(reinterpret_cast<void**>(&out.nodes), out.count * sizeof(DevNode4));
+        if (e == cudaSuccess)
+            e = launch_write_nodes(nodes, items, out.nodes, got.nodes, h->stream);
+        if (e == cudaSuccess)
+            e = cudaStreamSynchronize(h->stream);
     }
+    cudaFree(items);
+    if (fits && e == cudaSuccess)
+        return RC_OK;
     cudaGetLastError();
-    cudaFree(*out);
-    *out = nullptr;
+    release(out);
     if (e != cudaSuccess && e != cudaErrorMemoryAllocation)
     {
         h->err = std::string("wide BVH: ") + cudaGetErrorString(e);
@@ -79,7 +98,8 @@ rc_status collapse(rc_tracer* h, const DevNode* nodes, size_t count, const std::
     return RC_OK;  // stays binary
 }
 
-// The meshes' trees, the top-level one and the instances' mesh roots.
+// The meshes' trees, the top-level one and the instances' mesh roots: all of
+// them, or none.
 rc_status ensure_wide_instanced(rc_tracer* h)
 {
     std::vector<int32_t> roots;  // inner mesh roots, each once
@@ -93,43 +113,49 @@ rc_status ensure_wide_instanced(rc_tracer* h)
         wideRoots.push_back(
             r < 0 ? r : int32_t(std::lower_bound(roots.begin(), roots.end(), r) - roots.begin()));
     const int levels = int(std::min<uint64_t>(h->bvhDepth, kMaxStack));
-    int needMesh = 0, needTop = 0;
+    WideTree mesh, top;
+    int32_t* instWide = nullptr;
     rc_status s = RC_OK;
-    if (!roots.empty() &&
-        ((s = collapse(h, h->dNodes, h->innerCount, roots, levels, kTwoLevelStack, &h->dWide, &needMesh)) != RC_OK ||
-         !h->dWide))
-        return s;
-    h->wideCount = h->dWide ? h->innerCount : 0;
-    h->deviceBytes += h->wideCount * sizeof(DevNode4);
-    h->wideTlasRoot = h->tlasRoot;
-    if (h->tlasRoot >= 0)
+    bool whole = true;
+    if (!roots.empty())
     {
-        s = collapse(h, h->dTlas, h->tlasCount, { h->tlasRoot }, levels, kTwoLevelStack, &h->dWideTlas, &needTop);
-        if (s != RC_OK || !h->dWideTlas)
-            return s;
-        h->wideTlasRoot = 0;
-        h->wideTlasCount = h->tlasCount;
-        h->deviceBytes += h->wideTlasCount * sizeof(DevNode4);
+        s = collapse(h, h->dNodes, h->innerCount, roots, levels, kTwoLevelStack, mesh);
+        whole = s == RC_OK && mesh.nodes;
+    }
+    if (whole && h->tlasRoot >= 0)
+    {
+        s = collapse(h, h->dTlas, h->tlasCount, { h->tlasRoot }, levels, kTwoLevelStack, top);
+        whole = s == RC_OK && top.nodes;
     }
     // a leaf of two instances stacks its second one
-    if (needMesh + needTop + 1 > kTwoLevelStack)
-        return RC_OK;  // stays binary
-    cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&h->dInstWide), wideRoots.size() * sizeof(int32_t));
-    if (e == cudaSuccess)
+    if (whole && mesh.need + top.need + 1 <= kTwoLevelStack)
     {
-        h->deviceBytes += wideRoots.size() * sizeof(int32_t);
-        e = cudaMemcpy(h->dInstWide, wideRoots.data(), wideRoots.size() * sizeof(int32_t), cudaMemcpyHostToDevice);
-    }
-    if (e != cudaSuccess)
-    {
-        cudaGetLastError();
-        if (e == cudaErrorMemoryAllocation)
+        cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&instWide), wideRoots.size() * sizeof(int32_t));
+        if (e == cudaSuccess)
+            e = cudaMemcpy(instWide, wideRoots.data(), wideRoots.size() * sizeof(int32_t), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess)
+        {
+            h->dWide = mesh.nodes;
+            h->wideCount = mesh.count;
+            h->dWideTlas = top.nodes;
+            h->wideTlasCount = top.count;
+            h->wideTlasRoot = h->tlasRoot >= 0 ? 0 : h->tlasRoot;
+            h->dInstWide = instWide;
+            h->deviceBytes += (mesh.count + top.count) * sizeof(DevNode4) + wideRoots.size() * sizeof(int32_t);
+            h->wideInstanced = true;
             return RC_OK;
-        h->err = std::string("wide BVH: ") + cudaGetErrorString(e);
-        return RC_CUDA;
+        }
+        cudaGetLastError();
+        if (e != cudaErrorMemoryAllocation)
+        {
+            h->err = std::string("wide BVH: ") + cudaGetErrorString(e);
+            s = RC_CUDA;
+        }
     }
-    h->wideInstanced = true;
-    return RC_OK;
+    cudaFree(instWide);
+    release(top);
+    release(mesh);
+    return s;
 }
 
 }  // namespace
@@ -150,12 +176,12 @@ rc_status ensure_wide(rc_tracer* h)
         return ensure_wide_instanced(h);
     if (h->rootLink < 0)
         return RC_OK;  // a leaf root: nothing to collapse
-    int need = 0;
-    const rc_status s = collapse(h, h->dNodes, h->innerCount, { h->rootLink }, int(h->bvhDepth), kMaxStack, &h->dWide,
-                                 &need);
-    if (s != RC_OK || !h->dWide)
+    WideTree tree;
+    const rc_status s = collapse(h, h->dNodes, h->innerCount, { h->rootLink }, int(h->bvhDepth), kMaxStack, tree);
+    if (s != RC_OK || !tree.nodes)
         return s;
-    h->wideCount = h->innerCount;
+    h->dWide = tree.nodes;
+    h->wideCount = tree.count;
     h->wideRoot = 0;
     h->deviceBytes += h->wideCount * sizeof(DevNode4);
     return RC_OK;

@@ -67,12 +67,21 @@ extern "C"
 namespace rcx
 {
 
-cudaError_t launch_collapse(const DevNode* nodes, int count, WideItem* items, DevNode4* wide, WideCounters* c,
-                            int level, size_t, int, cudaStream_t)
+cudaError_t launch_collapse(const DevNode* nodes, int count, WideItem* items, WideCounters* c, int level, size_t, int,
+                            cudaStream_t)
 {
-    c->bound[level + 1] = c->nodes;
-    for (int i = c->bound[level]; i < level_end(*c, level, count); ++i)
-        collapse_node(nodes, count, items, wide, c, i);
+    const int end = level_end(*c, level, count);
+    for (int i = c->bound[level]; i < end; ++i)
+        collapse_node(nodes, count, items, c, i);
+    c->bound[level + 2] = c->nodes;
+    return cudaSuccess;
+}
+
+cudaError_t launch_write_nodes(const DevNode* nodes, const WideItem* items, DevNode4* wide, int taken,
+                               cudaStream_t)
+{
+    for (int i = 0; i < taken; ++i)
+        write_node(nodes, items, wide, i);
     return cudaSuccess;
 }
 
@@ -160,20 +169,20 @@ void release(rc_tracer& h)
     CHECK(live.empty());
 }
 
-// Leaf slots below a wide node in preorder of the binary tree, and that every
-// inner node of the binary tree is opened or a wide node's own.
-void leaves(const rcx::DevNode4* wide, int link, std::vector<int>& out)
+// Leaf slots below a wide node, and the wide nodes (`used`).
+void leaves(const rcx::DevNode4* wide, int link, std::vector<int>& out, size_t& used)
 {
     if (link < 0)
     {
         out.push_back((~link) >> rcx::kLeafCountBits);
         return;
     }
+    used++;
     const int n = wide[link].meta.x;
     CHECK(n >= 2 && n <= 4);
     const int* l = &wide[link].link.x;
     for (int k = 0; k < n; ++k)
-        leaves(wide, l[k], out);
+        leaves(wide, l[k], out, used);
 }
 
 void valid_trees()
@@ -192,7 +201,9 @@ void valid_trees()
             if (h.dWide)
             {
                 std::vector<int> slots;
-                leaves(h.dWide, h.wideRoot, slots);
+                size_t used = 0;
+                leaves(h.dWide, h.wideRoot, slots, used);
+                CHECK(live[h.dWide] == used * sizeof(rcx::DevNode4));  // no more than the tree's nodes
                 std::sort(slots.begin(), slots.end());
                 CHECK(int(slots.size()) == count + 1);
                 for (int i = 0; i < int(slots.size()); ++i)
@@ -221,7 +232,8 @@ void largest_area()
     const std::vector<rcx::DevNode> nodes{ node(8.0f, 1, more, 2), node(1.0f, 3, 0.5f, leaf(0)),
                                            node(0.1f, leaf(1), 0.1f, leaf(2)), node(0.1f, leaf(3), 0.1f, leaf(4)) };
     rcx::WideChild ch[4];
-    CHECK(rcx::wide_children(nodes.data(), 4, 0, ch) == 4);
+    int opened;
+    CHECK(rcx::wide_children(nodes.data(), 4, 0, ch, opened) == 4);
     bool box3 = false;
     for (const rcx::WideChild& c : ch)
         box3 |= c.link == 3;
