@@ -869,7 +869,7 @@ bool stackless_walk()
 
 bool cast_walks_wide(const LaunchInfo& li, const DevScene& sc, int64_t n, int anyHit, int order)
 {
-    if (anyHit || order != ORDER_NEAREST || li.counting || sc.numInstances > 0)
+    if (anyHit || order != ORDER_NEAREST || li.counting || sc.numInstances > 0 || (sc.ropes && stackless_walk()))
         return false;
     static OccupancyCache occ;
     return group_lanes(sc, n, persistent_blocks(k_cast_group<false, ORDER_NEAREST>, li.numSMs, occ), 4) == 0u;
