@@ -97,9 +97,9 @@ int blocks_per_sm(K kernel, int block, size_t smem, OccupancyCache& cache)
 // use while this is on).
 bool stackless_walk();
 
-// Whether launch_cast of this call walks the scene's 4-wide tree where there
-// is one (the host builds it on first use).
-bool cast_walks_wide(const LaunchInfo& li, const DevScene& sc, int64_t n, int anyHit, int order);
+// Rays of this launch_cast that the scene's 4-wide tree, where there is one,
+// makes cheaper: those above the line up to which groups of lanes walk a ray.
+int64_t cast_wide_rays(const LaunchInfo& li, const DevScene& sc, int64_t n, int anyHit, int order);
 
 // Generic ray queries (rc_ray -> rc_hit).
 cudaError_t launch_cast(const LaunchInfo& li, const DevScene& sc, const rc_ray* rays, int64_t n, int anyHit,

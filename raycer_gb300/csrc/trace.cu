@@ -867,12 +867,14 @@ bool stackless_walk()
     return on;
 }
 
-bool cast_walks_wide(const LaunchInfo& li, const DevScene& sc, int64_t n, int anyHit, int order)
+int64_t cast_wide_rays(const LaunchInfo& li, const DevScene& sc, int64_t n, int anyHit, int order)
 {
     if (anyHit || order != ORDER_NEAREST || li.counting || sc.numInstances > 0 || (sc.ropes && stackless_walk()))
-        return false;
+        return 0;
     static OccupancyCache occ;
-    return group_lanes(sc, n, persistent_blocks(k_cast_group<false, ORDER_NEAREST>, li.numSMs, occ), 4) == 0u;
+    const int blocks = persistent_blocks(k_cast_group<false, ORDER_NEAREST>, li.numSMs, occ);
+    const int64_t line = int64_t(blocks) * kBlock * 2;  // most rays that groups of 4 lanes walk (group_lanes)
+    return std::max<int64_t>(0, n - line);
 }
 
 cudaError_t launch_cast(const LaunchInfo& li, const DevScene& sc, const rc_ray* rays, int64_t n, int anyHit,

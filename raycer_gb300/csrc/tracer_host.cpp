@@ -122,6 +122,7 @@ void release_scene(rc_tracer* h)
     h->wideInstanced = false;
     h->wideRoot = 0;
     h->wideTried = false;
+    h->castRays = 0;
     dev_free(h, &h->dRopes, h->ropeCount);
     h->ropeCount = 0;
     h->ropesTried = false;
@@ -1063,8 +1064,8 @@ rc_status rc_cast_device(rc_tracer* h, const rc_ray* d_rays, int64_t n, int32_t 
         return fail(h, RC_INVALID_ARG, "cast: invalid traversal order");
     cudaSetDevice(h->device);
     rc_status s = stackless_walk() ? ensure_ropes(h) : RC_OK;
-    if (s == RC_OK && cast_walks_wide(launch_info(h), dev_scene(h), n, any_hit, order))
-        s = ensure_wide(h);
+    if (s == RC_OK)
+        s = ensure_wide_for_casts(h, cast_wide_rays(launch_info(h), dev_scene(h), n, any_hit, order));
     if (s != RC_OK)
         return s;
     s = begin_launch(h);

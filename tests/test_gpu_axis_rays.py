@@ -20,6 +20,7 @@ from raycer_gb300.tracer import RAY_DTYPE, CudaTracer
 
 from helpers import small_room
 from test_gpu_cast import _edge_rays
+from test_gpu_cast_tree import grow_tree
 
 pytestmark = pytest.mark.gpu
 
@@ -30,6 +31,7 @@ FAR = np.float32(3.0e38)
 def _compare(sc, rays, order, any_hit=False):
     with CudaTracer(0) as t:
         t.initializeBuffers(sc)
+        assert grow_tree(t) > 0
         hits = t.cast(rays, any_hit=any_hit, order=order)
     prim, tt, u, v, _ = oracle.Oracle(sc).cast32(rays, any_hit=any_hit, order=order)
     assert np.array_equal(hits["prim"], prim), int((hits["prim"] != prim).sum())

@@ -14,6 +14,8 @@ from raycer_gb300 import _native as N
 from raycer_gb300 import scenes
 from raycer_gb300.tracer import RAY_DTYPE, CudaTracer
 
+from test_gpu_cast_tree import grow_tree
+
 pytestmark = pytest.mark.gpu
 
 
@@ -40,6 +42,7 @@ def test_parallel_rays_onto_a_sheet(height, spread):
     rays["t_max"] = 3.0e38
     with CudaTracer(0) as t:
         t.initializeBuffers(sc)
+        assert grow_tree(t) > 0
         hits = t.cast(rays, order=N.RC_ORDER_NEAREST)
     prim, tt, u, v, _ = oracle.Oracle(sc).cast32(rays, any_hit=False, order=1)
     assert (prim >= 0).all()

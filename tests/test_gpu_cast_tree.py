@@ -1,5 +1,7 @@
 """When rc_cast builds the scene's 4-wide tree, seen in the handle's device
-memory: never where its kernels would not walk it (the stackless switch)."""
+memory: once the rays pay for it, and never where its kernels would not walk it
+(the stackless switch). Casts through a tree that is there equal the float32
+oracle's at the sizes where the kernels change."""
 
 from __future__ import annotations
 
@@ -8,11 +10,69 @@ import subprocess
 import sys
 from pathlib import Path
 
+import numpy as np
 import pytest
+
+import oracle
+from raycer_gb300 import _native as N
+from raycer_gb300.tracer import RAY_DTYPE, CudaTracer
+
+from helpers import small_heightfield, small_room
+from test_gpu_degenerate import scene as degenerate_scene
+from test_gpu_ray_groups import _rays
 
 pytestmark = pytest.mark.gpu
 
 TESTS = Path(__file__).resolve().parent
+
+
+def grow_tree(t):
+    """Has the tracer's scene build its 4-wide tree: a cast of many empty rays."""
+    rays = np.zeros(4_000_000, RAY_DTYPE)
+    rays["direction"][:, 2] = 1.0
+    rays["t_max"] = -1.0
+    t.cast(rays, any_hit=True)  # the call's buffers
+    before = t.stats()["device_bytes"]
+    t.cast(rays)
+    return t.stats()["device_bytes"] - before
+
+
+def test_casts_build_the_tree_once_they_pay_for_it():
+    sc = small_heightfield()
+    rays = _rays(1_500_000, 3)
+    with CudaTracer(0) as t:
+        for _ in range(2):  # the second upload starts anew
+            t.initializeBuffers(sc)
+            t.cast(rays, any_hit=True)
+            before = t.stats()["device_bytes"]
+            grown = []
+            first = t.cast(rays)
+            for _ in range(3):
+                grown.append(t.stats()["device_bytes"] - before)
+                assert np.array_equal(t.cast(rays), first)
+            t.cast(rays[:300_000])
+            t.cast(rays, order=N.RC_ORDER_REFERENCE)
+            assert grown[0] == grown[1] == 0 and grown[2] > 0
+            assert grown[2] == t.stats()["device_bytes"] - before
+        t.initializeBuffers(sc)
+        assert grow_tree(t) == grown[2]
+
+
+@pytest.mark.parametrize("n", [311_299, 311_400, 400_000])
+@pytest.mark.parametrize("name", ["room", "terrain", "coplanar", "duplicates"])
+def test_casts_through_the_tree(name, n):
+    sc = {"room": lambda: small_room(clutter=1000), "terrain": small_heightfield,
+          "coplanar": lambda: degenerate_scene("coplanar", 4), "duplicates": lambda: degenerate_scene("duplicates", 1)}[name]()
+    rays = _rays(n, n)
+    with CudaTracer(0) as t:
+        t.initializeBuffers(sc)
+        assert grow_tree(t) > 0
+        hits = t.cast(rays)
+    prim, tt, u, v, _ = oracle.Oracle(sc).cast32(rays, any_hit=False, order=N.RC_ORDER_NEAREST)
+    assert np.array_equal(hits["prim"], prim)
+    for k, ref in (("t", tt), ("u", u), ("v", v)):
+        assert np.array_equal(hits[k], ref)
+
 
 _STACKLESS = """
 import sys
