@@ -112,6 +112,7 @@ struct rc_tracer
     rcx::DevInstance* dInstances = nullptr;
     int64_t nInstances = 0;
     int32_t tlasRoot = 0;
+    uint32_t tlasDepth = 0;  // of bvhDepth, which is both levels'
     std::vector<rcx::InstancedMesh> instMeshes;  // two-level scene: its meshes
     std::vector<rc_instance> instDescs;          //   and instances, for rc_save_scene
     // 4-wide BVH of a single-level scene (wide_build.cu), or none.
@@ -128,6 +129,7 @@ struct rc_tracer
     bool wideInstanced = false;  // the three above and dWide are built
     bool wideTried = false;  // ensure_wide ran for the current scene
     int64_t castRays = 0;    // cast_wide_rays of the scene's casts while it has no such tree
+    int64_t bounceRounds = 0;  // bounce segments of the two-level scene's passes, likewise
     // Rope records of a single-level scene for the stackless walk (wide_bvh.cpp), or none.
     rcx::DevRope* dRopes = nullptr;
     size_t ropeCount = 0;
@@ -243,13 +245,17 @@ rc_status upload_host_scene(rc_tracer* h, HostScene&& hs);
 void release_scene_data(rc_tracer* h);
 // Collapses the binary device nodes of the handle's single-level scene into
 // the 4-wide BVH on first use (the first PATH or batch render of a scene, or
-// rc_cast once the rays pay for it); leaves it out where its stack need exceeds the
+// rc_cast once the rays pay for it), or a two-level scene's meshes and the tree
+// over its instances (PATH renders, once their bounces pay for it); leaves it out where its stack need exceeds the
 // traversal stack or there is no memory for it. Uploads, RAY frames and small
 // passes and casts do not pay for it.
 rc_status ensure_wide(rc_tracer* h);
 // ensure_wide for a cast of `rays` (cast_wide_rays), once the scene's casts
 // have had enough of them.
 rc_status ensure_wide_for_casts(rc_tracer* h, int64_t rays);
+// ensure_wide of a two-level scene for passes of `rounds` bounce segments
+// together, once its passes have had enough of them.
+rc_status ensure_wide_for_bounces(rc_tracer* h, int64_t rounds);
 // Builds the rope records of the handle's single-level scene on first use
 // (the first RAY frame or rc_cast while the stackless walk is on): one
 // download of the binary nodes, one upload of the records.

@@ -484,6 +484,7 @@ rc_status upload_instanced_scenes(rc_tracer* h, std::vector<HostScene>&& meshSce
     for (uint32_t d : meshDepth)
         depth = std::max(depth, d);
     h->bvhDepth = depth + tb.depth;
+    h->tlasDepth = tb.depth;
     h->bvhInner = nodes.size() + tn.size();
     h->deviceBytes += nodes.size() * sizeof(DevNode) + tris.size() * (sizeof(DevTri) + sizeof(DevShade)) +
                       mats.size() * sizeof(DevMat) + tn.size() * sizeof(DevNode) + ordered.size() * sizeof(DevInstance);

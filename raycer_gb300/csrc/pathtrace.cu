@@ -1717,9 +1717,16 @@ cudaError_t path_group_b(const PassParams& p, unsigned G, cudaStream_t stream, i
 
 }  // namespace
 
-bool path_walks_wide(const PassParams& p, int order, int counting, int numSMs)
+bool path_is_small(const PassParams& p, int order, int counting, int numSMs)
 {
-    return path_group_lanes(p, order, counting, numSMs) == 0u;
+    return path_group_lanes(p, order, counting, numSMs) != 0u;
+}
+
+bool path_walks_wide(const PassParams& p, int order, int counting)
+{
+    if (p.instanced)
+        return one_kernel_pass(order, counting) && p.segments > 1;  // the bounces
+    return order == ORDER_NEAREST && !counting && p.segments > 0;
 }
 
 int path_extend_launches(const PassParams& p, int order, int counting)

@@ -102,7 +102,7 @@ struct PassParams
     NrcPass nrc;
     int instanced;   // 1: the pass has two-level scenes (k_extend_instanced)
     int wide;        // 1: every scene of the pass has its 4-wide BVH (uncounted nearest-first extend uses it)
-    int small = 0;        // 1: the render's largest pass is walked by groups of lanes (path_walks_wide false)
+    int small = 0;        // 1: the render's largest pass is walked by groups of lanes (path_is_small)
     int singleScene = 0;  // 1: every slot of the pass is scene0's (a one-scene render), so the
                           // extend kernels read the scene record from the parameters, not the table
     DevScene scene0;
@@ -128,9 +128,11 @@ struct PassShape
     int shadeBlock = 128;
 };
 
-// Whether a pass (nslots, scene0 and the like set) walks the 4-wide trees
-// where there are any; a small one does not.
-bool path_walks_wide(const PassParams& p, int order, int counting, int numSMs);
+// Whether a pass (nslots, scene0 and the like set) is walked by groups of
+// lanes, through the binary tree.
+bool path_is_small(const PassParams& p, int order, int counting, int numSMs);
+// Whether a pass that is not small walks the 4-wide trees where there are any.
+bool path_walks_wide(const PassParams& p, int order, int counting);
 // Extend launches of a pass: one per segment, or, where extend and shade run
 // as one kernel, one for the camera rays and one for all later segments (a
 // render of small passes: one).

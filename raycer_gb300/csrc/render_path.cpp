@@ -232,8 +232,10 @@ rc_status render_path(rc_tracer* h, uint64_t pixelStart, uint64_t count, RenderW
         probe.instanced = h->nInstances > 0 ? 1 : 0;
         probe.singleScene = 1;
         probe.scene0 = path_scene(h, pixelStart).sc;
-        small = !path_walks_wide(probe, h->order, h->counting, h->numSMs);
-        const rc_status ws = small ? RC_OK : ensure_wide(h);
+        small = path_is_small(probe, h->order, h->counting, h->numSMs);
+        rc_status ws = RC_OK;
+        if (!small && path_walks_wide(probe, h->order, h->counting))
+            ws = h->nInstances > 0 ? ensure_wide_for_bounces(h, int64_t(passes) * (g.max_path_length - 1)) : ensure_wide(h);
         if (ws != RC_OK)
             return ws;
     }

@@ -123,6 +123,7 @@ void release_scene(rc_tracer* h)
     h->wideRoot = 0;
     h->wideTried = false;
     h->castRays = 0;
+    h->bounceRounds = 0;
     dev_free(h, &h->dRopes, h->ropeCount);
     h->ropeCount = 0;
     h->ropesTried = false;

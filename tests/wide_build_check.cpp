@@ -152,7 +152,8 @@ void scene(rc_tracer& h, std::vector<rcx::DevNode>& nodes, int levels, int insta
     h.numSMs = 4;
     h.innerCount = nodes.size();
     h.rootLink = 0;
-    h.bvhDepth = uint64_t(levels);
+    h.bvhDepth = uint64_t(instances > 0 ? 2 * levels : levels);
+    h.tlasDepth = uint32_t(instances > 0 ? levels : 0);
     h.dNodes = nodes.data();
     h.nInstances = instances;
     h.tlasRoot = 0;
