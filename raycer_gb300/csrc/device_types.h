@@ -137,16 +137,22 @@ struct FilmTiles
 };
 
 // Tiles of `count` pixels from pixelStart on of a film `width` wide; none where
-// the range has no four lines or a line no tile.
+// the range has no four lines or a line no tile, or where the tiles' pixels
+// and what the warps take past them leave a queue head's 32 bits.
 inline FilmTiles film_tiles(uint64_t pixelStart, int64_t count, int64_t width)
 {
     FilmTiles t;
-    if (width < 8 || count / width < 4 || count >= (int64_t(1) << 30))
+    if (width < 8 || count / width < 4)
+        return t;
+    const int64_t skip = int64_t(pixelStart % uint64_t(width));
+    const int64_t columns = (width + 7) / 8;
+    const int64_t rows = ((skip + count + width - 1) / width + 3) / 4;
+    if (columns * rows >= (int64_t(1) << 27) - (int64_t(1) << 19))
         return t;
     t.width = width;
-    t.skip = int64_t(pixelStart % uint64_t(width));
-    t.columns = int((width + 7) / 8);
-    t.rows = int(((t.skip + count + width - 1) / width + 3) / 4);
+    t.skip = skip;
+    t.columns = int(columns);
+    t.rows = int(rows);
     return t;
 }
 
