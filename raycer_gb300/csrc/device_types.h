@@ -156,6 +156,18 @@ inline FilmTiles film_tiles(uint64_t pixelStart, int64_t count, int64_t width)
     return t;
 }
 
+// Pixels of the range's `count` in its first `tile` tiles.
+__host__ __device__ inline int64_t tile_pixels_before(const FilmTiles& t, int64_t count, int64_t tile)
+{
+    const int64_t row = tile / t.columns;
+    const int64_t left = (tile - row * t.columns) * 8 < t.width ? (tile - row * t.columns) * 8 : t.width;
+    const auto clip = [count](int64_t i) { return i < 0 ? int64_t(0) : i < count ? i : count; };
+    int64_t n = clip(row * 4 * t.width - t.skip);
+    for (int64_t y = row * 4; y < row * 4 + 4; ++y)
+        n += clip(y * t.width - t.skip + left) - clip(y * t.width - t.skip);
+    return n;
+}
+
 // Device scene handed to every kernel by value. Two-level scenes
 // (numInstances > 0) keep every mesh's BVH in `nodes` / `tris` / `shade`
 // (links already offset into the pools) and a top-level BVH over the

@@ -96,14 +96,16 @@ static __device__ __noinline__ int poll_render(RenderMonitor* mon, unsigned long
 // had reached `items` at a poll (every item taken), a stop, or kWatchPolls
 // polls (then it just stops watching). The other warps' work loop carries no poll at all.
 // publish: kPublishNone, kPublishProgress, or kPublishEstimate (the pixels of
-// the items taken before those the other warps may hold, at most `pixels`).
+// the items taken before those the other warps may hold: of `pixels` in order,
+// or in `tiles`).
 // finished: where an item is long (a whole path), the count of warps that
 // have left the kernel's loop; the watch then goes on until all have.
 constexpr unsigned kWatchPolls = 1u << 24;
 
 static __device__ __forceinline__ void watch_queue(RenderMonitor* mon, unsigned long long budgetNs, DevControl* ctl,
                                          unsigned* head, unsigned long long items, unsigned long long publish,
-                                         unsigned long long pixels, const unsigned* finished = nullptr)
+                                         unsigned long long pixels, const unsigned* finished = nullptr,
+                                         const FilmTiles& tiles = FilmTiles{})
 {
     if ((threadIdx.x & 31u) != 0u)
         return;
@@ -115,8 +117,10 @@ static __device__ __forceinline__ void watch_queue(RenderMonitor* mon, unsigned 
         if (publish == kPublishEstimate)
         {
             const unsigned long long item = h >> 5;
-            pub = item > workers ? (item - workers) * 32ull : 0ull;
-            pub = pub < pixels ? pub : pixels;
+            const unsigned long long whole = item > workers ? item - workers : 0ull;
+            pub = tiles.columns > 0
+                      ? static_cast<unsigned long long>(tile_pixels_before(tiles, int64_t(pixels), int64_t(whole)))
+                      : (whole * 32ull < pixels ? whole * 32ull : pixels);
         }
         // polled once before the head is looked at: a kernel whose items
         // were all taken at once is still checked (a budget of 0 stops it)

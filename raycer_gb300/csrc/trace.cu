@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(kBlock, !FUSED ? RC_TRACE_MIN_BLOCKS
     if (is_watch_warp(sc.monitor, sc.budgetNs))
     {
         watch_queue(sc.monitor, sc.budgetNs, ctl, &ctl->head[0], static_cast<unsigned long long>(items),
-                    FUSED ? kPublishEstimate : kPublishNone, static_cast<unsigned long long>(count));
+                    FUSED ? kPublishEstimate : kPublishNone, static_cast<unsigned long long>(count), nullptr, tiles);
         return;
     }
     while (true)
@@ -584,7 +584,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_raycast_group(DevScene sc, DevCam
     if (is_watch_warp(sc.monitor, sc.budgetNs))
     {
         watch_queue(sc.monitor, sc.budgetNs, ctl, &ctl->head[0], static_cast<unsigned long long>(items),
-                    kPublishEstimate, static_cast<unsigned long long>(count));
+                    kPublishEstimate, static_cast<unsigned long long>(count), nullptr, tiles);
         return;
     }
     while (true)

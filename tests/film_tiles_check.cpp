@@ -1,4 +1,4 @@
-// Host check of film_tiles (device_types.h).
+// Host check of film_tiles and tile_pixels_before (device_types.h).
 
 #include "../raycer_gb300/csrc/device_types.h"
 
@@ -39,11 +39,40 @@ void largest_films()
     CHECK(rcx::film_tiles(0, (int64_t(1) << 30) * 2 - 2, 9).columns == 2);
 }
 
+// tile_pixels_before against the tiles' pixels counted one by one.
+void pixels_before()
+{
+    const int64_t widths[] = { 8, 9, 15, 16, 37 };
+    const int64_t starts[] = { 0, 1, 8, 30 };
+    const int64_t counts[] = { 37 * 4, 301, 555 };
+    for (int64_t width : widths)
+        for (int64_t start : starts)
+            for (int64_t count : counts)
+            {
+                const rcx::FilmTiles t = rcx::film_tiles(uint64_t(start), count, width);
+                CHECK(t.columns > 0);
+                int64_t n = 0;
+                for (int64_t tile = 0; tile < int64_t(t.columns) * t.rows; ++tile)
+                {
+                    CHECK(rcx::tile_pixels_before(t, count, tile) == n);
+                    for (int64_t k = 0; k < 32; ++k)
+                    {
+                        const int64_t x = tile % t.columns * 8 + k % 8, y = tile / t.columns * 4 + k / 8;
+                        const int64_t i = y * width + x - t.skip;
+                        n += x < width && i >= 0 && i < count ? 1 : 0;
+                    }
+                }
+                CHECK(n == count);
+                CHECK(rcx::tile_pixels_before(t, count, int64_t(t.columns) * t.rows) == count);
+            }
+}
+
 }  // namespace
 
 int main()
 {
     largest_films();
+    pixels_before();
     if (!failures)
         std::printf("film tiles ok\n");
     return failures ? 1 : 0;

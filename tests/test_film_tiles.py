@@ -1,6 +1,6 @@
 """The tiles in which pixel ranges are taken (film_tiles), checked on the host
 (film_tiles_check.cpp): films of 2^30 pixels and more are taken in tiles as
-smaller ones are."""
+smaller ones are; the pixels of a number of tiles."""
 
 from __future__ import annotations
 
