@@ -247,8 +247,7 @@ __device__ __forceinline__ void flush_extend_counts(const PassParams& p, unsigne
         atomicOr(&p.ctl->error, 1);
 }
 
-// Closest hit of a ray put aside from the 4-wide walk (an inverse direction
-// that is not finite) through the binary trees; no triangle accepts a ray with
+// Closest hit of a ray put aside from the 4-wide walk through the binary trees; no triangle accepts a ray with
 // a NaN, whose walk would enter every box.
 template <bool INST>
 static __device__ __noinline__ HitF aside_hit(const PassParams& p, int s, const float4& o, const float4& d)
@@ -851,9 +850,9 @@ __global__ void __launch_bounds__(BLOCK) k_shade(PassParams p, int segment)
     }
 }
 
-// A path whose ray has an inverse direction that is not finite is put aside
-// from the 4-wide walk, with its ray and segment: k_finish_aside takes it to
-// its end. (The binary walk in these kernels, or a call for it at the end of
+// A path whose ray has an inverse direction that is not finite, or whose walk
+// is undecided, is put aside from the 4-wide walk, with its ray and segment:
+// k_finish_aside takes it to its end. (The binary walk in these kernels, or a call for it at the end of
 // their loops, cost every path's walk its registers: 4-40 % slower.)
 __device__ __forceinline__ void put_aside(const PassParams& p, int segment, int s, const float4& o, const float4& d)
 {
@@ -1256,7 +1255,14 @@ __global__ void __launch_bounds__(128, RC_INST_MIN_BLOCKS)
                 const float t0 = h.t;
                 const int s0 = h.slot;
                 wide_leaf_step(p.scene0.tris, ray, h, w, stack, skips[threadIdx.x]);
-                if (h.t != t0 || h.slot != s0)
+                if (walk_undecided(h))
+                {
+                    const int2 path = paths[threadIdx.x];
+                    put_aside(p, path.y, path.x, worldO[threadIdx.x], worldD[threadIdx.x]);
+                    w.abandon();
+                    w.cur = kWalkNone;
+                }
+                else if (h.t != t0 || h.slot != s0)
                     hitInst[threadIdx.x] = w.inst;
             }
         }

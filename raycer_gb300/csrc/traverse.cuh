@@ -416,6 +416,7 @@ __device__ __forceinline__ void wide_cswap(float& da, int& la, float& db, int& l
 struct WideWalk
 {
     static constexpr bool kFinite = true;  // only rays whose inverse direction is finite
+    static constexpr bool kTies = false;
     int cur;
     int sp;
     __device__ __forceinline__ void abandon();
@@ -480,6 +481,7 @@ constexpr float kTieCull = 1.01f;
 struct CastWalk
 {
     static constexpr bool kFinite = false;  // any ray
+    static constexpr bool kTies = false;
     int cur;
     int sp;
     float entry;     // of cur
@@ -511,7 +513,7 @@ __device__ __forceinline__ void wide_pop(const HitF& hit, Walk& w, const Stack& 
     w.cur = kWalkDone;
 }
 
-// Whether a CastWalk ended undecided: its ray has to walk the binary tree.
+// Whether a walk ended undecided: its ray has to walk the binary trees.
 __device__ __forceinline__ bool walk_undecided(const HitF& hit) { return !(hit.t == hit.t); }
 
 // Node step of the 4-wide walk (w.cur >= 0): enters the nearest child hit
@@ -630,7 +632,10 @@ __device__ __forceinline__ void wide_node_step(const DevNode4* __restrict__ wide
     wide_pop(hit, w, stack);
 }
 
-// The closest-hit test of one leaf triangle in the 4-wide walk.
+// The closest-hit test of one leaf triangle in the 4-wide walk. kTies: the
+// same triangle at the same distance again is another instance's, and the one
+// met first is the hit: the order of the walk decides, and the hit's t is set
+// to a NaN (walk_undecided).
 template <typename Walk>
 __device__ __forceinline__ void wide_leaf_test(const RayF& ray, HitF& hit, Walk& w, int slot, int skip,
                                                const float4& ta, const float4& tb, const float4& tc)
@@ -638,8 +643,9 @@ __device__ __forceinline__ void wide_leaf_test(const RayF& ray, HitF& hit, Walk&
     if (slot == skip)
         return;
     float t, u, v;
-    if (tri_hit(ray, v3(ta.x, ta.y, ta.z), v3(ta.w, tb.x, tb.y), v3(tb.z, tb.w, tc.x), t, u, v) &&
-        (t < hit.t || (t == hit.t && slot > hit.slot)))
+    if (!tri_hit(ray, v3(ta.x, ta.y, ta.z), v3(ta.w, tb.x, tb.y), v3(tb.z, tb.w, tc.x), t, u, v))
+        return;
+    if (t < hit.t || (t == hit.t && slot > hit.slot))
     {
         hit.slot = slot;
         hit.t = t;
@@ -647,6 +653,8 @@ __device__ __forceinline__ void wide_leaf_test(const RayF& ray, HitF& hit, Walk&
         hit.v = v;
         w.accepted();
     }
+    else if (Walk::kTies && t == hit.t && slot == hit.slot)
+        hit.t = __int_as_float(0x7fffffff);
 }
 
 // Leaf step (w.cur < 0): two of the leaf's triangles, both fetched before
@@ -679,12 +687,14 @@ __device__ __forceinline__ void wide_leaf_step(const DevTri* __restrict__ tris, 
 
 // A walk of a two-level scene: the top-level tree over the instances (inst =
 // -1) or an instance's mesh, whose entries lie above `base` of one stack. At
-// the top level a leaf code names instances.
+// the top level a leaf code names instances. Coincident instances of a mesh
+// are decided by the order of the binary walk (wide_leaf_test).
 constexpr int kWalkReturn = -0x7ffffffe;  // the mesh is done (no leaf code: 13 triangles would start at the last slot)
 
 struct TwoLevelWalk
 {
     static constexpr bool kFinite = true;
+    static constexpr bool kTies = true;
     int cur;
     int sp;
     int base;
