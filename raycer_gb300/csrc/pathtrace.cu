@@ -1135,7 +1135,7 @@ __global__ void __launch_bounds__(128, RC_INST_MIN_BLOCKS)
     __shared__ float4 worldD[BLOCK];
     __shared__ int skips[BLOCK];      // the triangle the walk skips in its instance
     __shared__ int hitInst[BLOCK];    // the closest hit's instance
-    __shared__ int2 nearEntries[kNearEntries][BLOCK];
+    __shared__ int2 nearEntries[kNearEntries + 1][BLOCK];
     int2 farEntries[kTwoLevelStack - kNearEntries];
     SharedStack<kNearEntries, BLOCK, kTwoLevelStack> stack{ &nearEntries[0][threadIdx.x], farEntries };
     unsigned done = 0;           // warp-uniform
@@ -1143,7 +1143,7 @@ __global__ void __launch_bounds__(128, RC_INST_MIN_BLOCKS)
     int err = 0;
     RayF ray = make_ray(v3(0.0f, 0.0f, 0.0f), v3(1.0f, 1.0f, 1.0f), 0.0f, FLT_MAX);
     HitF h{ -1, FLT_MAX, 0.0f, 0.0f, -1 };
-    TwoLevelWalk w{ kWalkNone, 0, 0, -1 };
+    TwoLevelWalk w{ kWalkNone, 0, 0, -1, 0.0f };
     while (true)
     {
         const unsigned atNode = __ballot_sync(kAll, w.cur >= 0);
@@ -1194,7 +1194,7 @@ __global__ void __launch_bounds__(128, RC_INST_MIN_BLOCKS)
                 ray = make_ray(v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), 0.0f, FLT_MAX);
                 h = HitF{ -1, FLT_MAX, 0.0f, 0.0f, -1 };
                 hitInst[threadIdx.x] = -1;
-                w = TwoLevelWalk{ p.scene0.wideTlasRoot, 0, 0, -1 };
+                w = TwoLevelWalk{ p.scene0.wideTlasRoot, 0, 0, -1, 0.0f };
                 if (!ray.finite)
                 {
                     const int2 path = paths[threadIdx.x];
@@ -1232,9 +1232,10 @@ __global__ void __launch_bounds__(128, RC_INST_MIN_BLOCKS)
                     const int k = code >> kLeafCountBits;
                     const int count = code & ((1 << kLeafCountBits) - 1);
                     if (count > 1)
-                        stack.put(w.sp++, make_int2(~(((k + 1) << kLeafCountBits) | (count - 1)), 0));
+                        stack.put(w.sp++, make_int2(~(((k + 1) << kLeafCountBits) | (count - 1)), __float_as_int(w.entry)));
                     w.base = w.sp;
                     w.inst = k;
+                    stack.extra().y = __float_as_int(w.entry);
                     skips[threadIdx.x] = __float_as_int(d.w) == k ? __float_as_int(o.w) : -1;
                     ray = instance_ray(load_instance(p.scene0.instances, k), ray);
                     w.cur = __ldg(p.scene0.instWide + k);

@@ -416,7 +416,6 @@ __device__ __forceinline__ void wide_cswap(float& da, int& la, float& db, int& l
 struct WideWalk
 {
     static constexpr bool kFinite = true;  // only rays whose inverse direction is finite
-    static constexpr bool kTies = false;
     int cur;
     int sp;
     __device__ __forceinline__ void abandon();
@@ -464,6 +463,8 @@ struct SharedStack
             far[i - D] = v;
     }
     __device__ __forceinline__ Entry get(int i) const { return i < D ? near[i * THREADS] : far[i - D]; }
+    // an entry apart from the stack, where the near entries have a row more
+    __device__ __forceinline__ Entry& extra() const { return near[D * THREADS]; }
 };
 
 __device__ __forceinline__ void WideWalk::abandon()
@@ -481,7 +482,6 @@ constexpr float kTieCull = 1.01f;
 struct CastWalk
 {
     static constexpr bool kFinite = false;  // any ray
-    static constexpr bool kTies = false;
     int cur;
     int sp;
     float entry;     // of cur
@@ -632,20 +632,16 @@ __device__ __forceinline__ void wide_node_step(const DevNode4* __restrict__ wide
     wide_pop(hit, w, stack);
 }
 
-// The closest-hit test of one leaf triangle in the 4-wide walk. kTies: the
-// same triangle at the same distance again is another instance's, and the one
-// met first is the hit: the order of the walk decides, and the hit's t is set
-// to a NaN (walk_undecided).
-template <typename Walk>
-__device__ __forceinline__ void wide_leaf_test(const RayF& ray, HitF& hit, Walk& w, int slot, int skip,
+// The closest-hit test of one leaf triangle in the 4-wide walk.
+template <typename Walk, typename Stack>
+__device__ __forceinline__ void wide_leaf_test(const RayF& ray, HitF& hit, Walk& w, const Stack&, int slot, int skip,
                                                const float4& ta, const float4& tb, const float4& tc)
 {
     if (slot == skip)
         return;
     float t, u, v;
-    if (!tri_hit(ray, v3(ta.x, ta.y, ta.z), v3(ta.w, tb.x, tb.y), v3(tb.z, tb.w, tc.x), t, u, v))
-        return;
-    if (t < hit.t || (t == hit.t && slot > hit.slot))
+    if (tri_hit(ray, v3(ta.x, ta.y, ta.z), v3(ta.w, tb.x, tb.y), v3(tb.z, tb.w, tc.x), t, u, v) &&
+        (t < hit.t || (t == hit.t && slot > hit.slot)))
     {
         hit.slot = slot;
         hit.t = t;
@@ -653,8 +649,6 @@ __device__ __forceinline__ void wide_leaf_test(const RayF& ray, HitF& hit, Walk&
         hit.v = v;
         w.accepted();
     }
-    else if (Walk::kTies && t == hit.t && slot == hit.slot)
-        hit.t = __int_as_float(0x7fffffff);
 }
 
 // Leaf step (w.cur < 0): two of the leaf's triangles, both fetched before
@@ -676,9 +670,9 @@ __device__ __forceinline__ void wide_leaf_step(const DevTri* __restrict__ tris, 
     const float4* p1 = reinterpret_cast<const float4*>(tris + s1);
     const float4 a0 = __ldg(p0 + 0), b0 = __ldg(p0 + 1), c0 = __ldg(p0 + 2);
     const float4 a1 = __ldg(p1 + 0), b1 = __ldg(p1 + 1), c1 = __ldg(p1 + 2);
-    wide_leaf_test(ray, hit, w, s0, skip, a0, b0, c0);
+    wide_leaf_test(ray, hit, w, stack, s0, skip, a0, b0, c0);
     if (count > 1)
-        wide_leaf_test(ray, hit, w, s1, skip, a1, b1, c1);
+        wide_leaf_test(ray, hit, w, stack, s1, skip, a1, b1, c1);
     if (count > 2)
         w.cur = ~(((s0 + 2) << kLeafCountBits) | (count - 2));
     else
@@ -687,28 +681,62 @@ __device__ __forceinline__ void wide_leaf_step(const DevTri* __restrict__ tris, 
 
 // A walk of a two-level scene: the top-level tree over the instances (inst =
 // -1) or an instance's mesh, whose entries lie above `base` of one stack. At
-// the top level a leaf code names instances. Coincident instances of a mesh
-// are decided by the order of the binary walk (wide_leaf_test).
+// the top level a leaf code names instances.
+//
+// The hit is that of the binary walk (traverse_instanced) unless its order
+// decides, and then the walk ends undecided:
+//   the same triangle at the same distance in two instances: the one met
+//   first is the hit;
+//   a hit before the entry of a box around it (see traverse_group), and
+//   another one nearer than that entry: met first, it hides the box.
+// To meet such hits the walk skips boxes only past kTieCull times the hit.
 constexpr int kWalkReturn = -0x7ffffffe;  // the mesh is done (no leaf code: 13 triangles would start at the last slot)
 
 struct TwoLevelWalk
 {
     static constexpr bool kFinite = true;
-    static constexpr bool kTies = true;
     int cur;
     int sp;
     int base;
     int inst;
+    float entry;  // of cur
     __device__ __forceinline__ void abandon()
     {
         sp = base = 0;
         inst = -1;
         cur = kWalkDone;
     }
-    __device__ __forceinline__ float limit(const HitF& hit) const { return hit.t; }
-    __device__ __forceinline__ void entered(float) {}
-    __device__ __forceinline__ void accepted() {}
+    __device__ __forceinline__ float limit(const HitF& hit) const { return hit.t * kTieCull; }
+    __device__ __forceinline__ void entered(float e) { entry = e; }
 };
+
+// The leaf test of a two-level walk. The stack's extra entry holds the entries
+// of the boxes around the hit (x) and of the instance (y).
+template <typename Stack>
+__device__ __forceinline__ void wide_leaf_test(const RayF& ray, HitF& hit, TwoLevelWalk& w, const Stack& stack, int slot,
+                                               int skip, const float4& ta, const float4& tb, const float4& tc)
+{
+    if (slot == skip)
+        return;
+    float t, u, v;
+    if (!tri_hit(ray, v3(ta.x, ta.y, ta.z), v3(ta.w, tb.x, tb.y), v3(tb.z, tb.w, tc.x), t, u, v))
+        return;
+    bool undecided;
+    if (t < hit.t || (t == hit.t && slot > hit.slot))
+    {
+        const float e = fmaxf(w.entry, __int_as_float(stack.extra().y));
+        undecided = hit.t < e;
+        stack.extra().x = __float_as_int(e);
+        hit.slot = slot;
+        hit.t = t;
+        hit.u = u;
+        hit.v = v;
+    }
+    else
+        undecided = (t == hit.t && slot == hit.slot) || t < __int_as_float(stack.extra().x);
+    if (undecided)
+        hit.t = __int_as_float(0x7fffffff);
+}
 
 template <typename Stack>
 __device__ __forceinline__ void wide_pop(const HitF& hit, TwoLevelWalk& w, const Stack& stack)
@@ -717,8 +745,11 @@ __device__ __forceinline__ void wide_pop(const HitF& hit, TwoLevelWalk& w, const
     {
         const int2 e = stack.get(--w.sp);
         w.cur = e.x;
-        if (!(__int_as_float(e.y) > hit.t))
+        if (!(__int_as_float(e.y) > w.limit(hit)))
+        {
+            w.entered(__int_as_float(e.y));
             return;
+        }
     }
     w.cur = w.inst >= 0 ? kWalkReturn : kWalkDone;
 }
