@@ -711,20 +711,32 @@ int trace_packets()
     return mode;
 }
 
+// Whether a pixel range is whole lines from the film's first on.
+bool whole_lines(uint64_t pixelStart, int64_t count, int64_t width)
+{
+    return pixelStart == 0 && (count / width) * width == count;
+}
+
 // The tiles of a frame (device_types.h), or none: camera rays of any pixel
 // range, or one caller ray per pixel of a whole image (other ray lists are
 // walked in order: nothing says that a ray's neighbour in the next line is
-// near it). In order, a range's warps were 32 pixels of a row, walked one ray
-// per lane; device time of ranges of 1237x701 and 1921x1081 films, in order ->
-// tiles: 1M triangles, nearest-first 37 % / 90 % / 50 % of the film 162 / 362 /
-// 257 -> 148 / 333 / 204 us, reference order 219 / 812 / 419 -> 190 / 667 /
-// 277; 90k triangles 100 / 248 / 162 -> 79 / 201 / 131 and 113 / 446 / 214 ->
-// 92 / 272 / 146.
+// near it).
 FilmTiles frame_tiles(const rc_ray* rays, uint64_t pixelStart, int64_t count, int64_t width)
 {
-    if (!RC_TRACE_TILES || width <= 0 || (rays && (pixelStart != 0 || (count / width) * width != count)))
+    if (!RC_TRACE_TILES || width <= 0 || (rays && !whole_lines(pixelStart, count, width)))
         return FilmTiles{};
     return film_tiles(pixelStart, count, width);
+}
+
+// Whether an uncounted frame of tiles is walked by packets: whole lines, and
+// any range in reference order, where a packet meets each ray's triangles in
+// the ray's order. Nearest-first, a packet's order can decide between hits
+// that rounding puts before their boxes (33 of 480,000 pixels in a room of
+// overlapping coplanar triangles): a range keeps its rays' own walks, and so
+// its records do not depend on where it ends.
+bool packet_frame(uint64_t pixelStart, int64_t count, int64_t width, int order)
+{
+    return order == ORDER_REF || whole_lines(pixelStart, count, width);
 }
 
 // Sign octant of the shadow rays' direction L for slab_oct (bit k: component
@@ -767,8 +779,7 @@ cudaError_t raycast_t(const LaunchInfo& li, const DevScene& sc, const DevCamera&
                       rc_cast_pixel* out, int* queue, DevControl* ctl, cudaEvent_t between, float4* origins,
                       int& kernels)
 {
-    // Tile a whole frame (pixel range = the full image; camera rays or one
-    // caller ray per pixel): only the order the warps take the pixels in.
+    // only the order the warps take the pixels in
     const FilmTiles tiles = frame_tiles(rays, pixelStart, count, width);
     if (FUSED && castShadow)
     {
@@ -947,7 +958,8 @@ cudaError_t launch_raycast(const LaunchInfo& li, const DevScene& sc, const DevCa
         }
     }
     const int packets = trace_packets();
-    const bool packet = frame_tiles(rays, pixelStart, count, width).columns > 0 && (packets == 2 || (packets == 1 && !rays));
+    const bool packet = frame_tiles(rays, pixelStart, count, width).columns > 0 &&
+                        packet_frame(pixelStart, count, width, order) && (packets == 2 || (packets == 1 && !rays));
     if (stackless_walk() && sc.ropes)
     {
         if (packet)
