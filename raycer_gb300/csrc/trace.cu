@@ -739,6 +739,24 @@ bool packet_frame(uint64_t pixelStart, int64_t count, int64_t width, int order)
     return order == ORDER_REF || whole_lines(pixelStart, count, width);
 }
 
+// The tiles of a frame walked by more than groups of lanes. Ranges walked one
+// ray per lane take them from four tiles per resident warp on: with fewer the
+// longest tile's chain of walks is longer than the longest row's. In order ->
+// tiles, device time of ranges of 192k, 240k, 320k, 433k, 607k, 780k and 1.87M
+// pixels, 1M triangles: 115 / 125 / 125 / 145 / 191 / 265 / 470 -> 134 / 148 /
+// 133 / 157 / 192 / 228 / 387 us. Packets in reference order: 222 / 268 / 226 /
+// 294 / 535 / 737 / 1,310 -> 224 / 281 / 184 / 238 / 387 / 600 / 803. Two-level
+// scenes gain at all sizes but one: 1M + 200 blobs of 20,480 triangles, 60k, 192k,
+// 240k, 320k, 433k, 607k and 1.87M pixels 613 / 416 / 541 / 423 / 648 / 866 /
+// 2,092 -> 525 / 403 / 602 / 359 / 570 / 780 / 1,646.
+FilmTiles walk_tiles(const LaunchInfo& li, const rc_ray* rays, uint64_t pixelStart, int64_t count, int64_t width,
+                     int order, bool instanced)
+{
+    if (!instanced && width > 0 && !packet_frame(pixelStart, count, width, order) && count < int64_t(li.numSMs) * 4 * 32 * 32)
+        return FilmTiles{};
+    return frame_tiles(rays, pixelStart, count, width);
+}
+
 // Sign octant of the shadow rays' direction L for slab_oct (bit k: component
 // k negative), or -1 where a component is zero, not finite or too small for
 // its reciprocal to be finite (the general box test then applies).
@@ -780,7 +798,7 @@ cudaError_t raycast_t(const LaunchInfo& li, const DevScene& sc, const DevCamera&
                       int& kernels)
 {
     // only the order the warps take the pixels in
-    const FilmTiles tiles = frame_tiles(rays, pixelStart, count, width);
+    const FilmTiles tiles = walk_tiles(li, rays, pixelStart, count, width, ORDER, INST);
     if (FUSED && castShadow)
     {
         kernels = 1;
