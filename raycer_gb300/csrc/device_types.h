@@ -18,9 +18,9 @@
 //   DevNode4 128 B per node of the 4-wide BVH collapsed from the DevNode tree
 //            (same leaves, same triangle order): the four children's boxes as
 //            one float4 per bound (child k in component k), their links, and
-//            the number of children. Read by the path tracer's uncounted nearest-first
-//            kernels and by large nearest-first rc_cast batches; the binary
-//            tree serves every other query.
+//            the number of children. Read by the path tracer's uncounted
+//            nearest-first kernels and by large nearest-first rc_cast batches;
+//            the binary tree serves every other query.
 // Everything is 16-B aligned and fetched with 128-bit loads.
 #pragma once
 

@@ -115,7 +115,8 @@ struct rc_tracer
     uint32_t tlasDepth = 0;  // of bvhDepth, which is both levels'
     std::vector<rcx::InstancedMesh> instMeshes;  // two-level scene: its meshes
     std::vector<rc_instance> instDescs;          //   and instances, for rc_save_scene
-    // 4-wide BVH of a single-level scene (wide_build.cu), or none.
+    // 4-wide BVH of a single-level scene, or of a two-level scene's meshes
+    // (wide_host.cpp), or none.
     rcx::DevNode4* dWide = nullptr;
     size_t wideCount = 0;              // allocated nodes
     int32_t wideRoot = 0;
@@ -243,12 +244,12 @@ void build_host_scene(const double* v, const uint32_t* matIdx, int64_t n, const 
                       std::vector<BuildNode>&& nodes, std::vector<uint32_t>&& order, uint32_t depth, HostScene& hs);
 rc_status upload_host_scene(rc_tracer* h, HostScene&& hs);
 void release_scene_data(rc_tracer* h);
-// Collapses the binary device nodes of the handle's single-level scene into
-// the 4-wide BVH on first use (the first PATH or batch render of a scene, or
-// rc_cast once the rays pay for it), or a two-level scene's meshes and the tree
-// over its instances (PATH renders, once their bounces pay for it); leaves it out where its stack need exceeds the
-// traversal stack or there is no memory for it. Uploads, RAY frames and small
-// passes and casts do not pay for it.
+// Builds the scene's 4-wide BVHs on the first call: the tree of a single-level
+// scene, or those of a two-level scene's meshes and the one over its instances.
+// A scene stays binary where a stack need exceeds the traversal stack or there
+// is no memory. PATH renders and batches of single-level scenes call it at once,
+// casts and two-level renders when they pay for it (below); uploads, RAY frames
+// and small passes and casts do not.
 rc_status ensure_wide(rc_tracer* h);
 // ensure_wide for a cast of `rays` (cast_wide_rays), once the scene's casts
 // have had enough of them.

@@ -12,7 +12,8 @@
 //   thr        path throughput (rgb)
 //   res        radiance result (rgb) + the camera sample's filter weight (w)
 //   hit        closest hit of the last extend (slot, t, u, v)
-// Stages (one launch each, per segment):
+// Stages (in their general form one launch each, extend and shade once per
+// segment; what runs fused is below):
 //   generate   camera rays for every slot; queue 0 = all slots (where one
 //              kernel traces and shades the camera rays, it makes them itself)
 //   extend     closest hit for every queued slot              (persistent)
@@ -23,10 +24,11 @@
 //   accumulate per pixel, in sample order: c_j = (sum_k L_jk) / P,
 //              film.rgb += w_j * c_j, film.w += w_j (Film::addSample,
 //              Film.cpp:54-59). One thread owns one pixel: deterministic.
-// Uncounted nearest-first passes over the 4-wide BVH run extend and shade of
-// a segment as one kernel (k_extend_shade); the hit record is then never
-// written. All segments after the first run as one kernel (k_bounce_paths,
-// k_bounce_instanced); small passes run whole in one (k_path_group).
+// Uncounted nearest-first passes over 4-wide BVHs trace and shade the camera
+// rays in one kernel (k_extend_shade; two-level scenes in two) and all later
+// segments in another (k_bounce_paths, k_bounce_instanced); the hit record is
+// then written only for the paths they put aside, which k_finish_aside takes to
+// their ends. Small passes run whole in one kernel (k_path_group).
 // Queue counts live on the device, so a pass is a fixed launch sequence the
 // host never waits on (and can be captured in a CUDA graph).
 

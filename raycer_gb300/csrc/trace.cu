@@ -634,27 +634,60 @@ int persistent_blocks(K kernel, int numSMs, OccupancyCache& cache)
     return blocks_per_sm(kernel, kBlock, 0, cache) * numSMs;
 }
 
-// Lanes per ray of an uncounted call with n rays on a single-level scene, or 0
-// for one ray per lane: the largest group (32, 16, 8, 4) whose `rounds` rounds
-// of one ray per group cover the rays (twice as many rounds for groups of 4,
-// whose alternative is one ray per lane). Each larger group shortens a ray's
-// chain of fetches but gives the warp fewer rays, so the lines lie where a
-// call stops being bound by latency. Measured (device times; 1M-triangle
-// terrain for casts, 260k for frames; group of 32 / 16 / 8 / 4 / none):
-//   25,000 random rays    80 /  66 /  67 /  91 / 159 us   (lines for 4 rounds)
-//   100,000                - /   - / 146 / 170 / 214 us
-//   400,000                - /   - /   - / 458 / 360 us
-//   160x90 frame          86 /  58 /  60 /   - / 226 us   (2 rounds: a tile's
-//   320x180                - / 150 / 101 / 103 / 199 us    neighbouring rays share
-//   480x270                - /   - / 186 / 153 / 194 us    fetches in a full warp)
-//   640x360                - /   - /   - / 225 / 186 us
-// A tree too deep for the group's stack is walked one ray per lane.
-unsigned group_lanes(const DevScene& sc, int64_t n, int blocks, int rounds)
+// Whether a group of G lanes has the stack for the scene's tree; a deeper tree
+// is walked one ray per lane.
+bool group_fits(const DevScene& sc, unsigned G) { return int(G) * kGroupEntries / 32 >= sc.depth + 2 * int(G); }
+
+// Lanes per ray of an uncounted cast of n rays on a single-level scene, or 0
+// for one ray per lane: the largest group (32, 16, 8, 4) whose four rounds of
+// one ray per group cover the rays (eight for groups of 4, whose alternative
+// is one ray per lane). Each larger group shortens a ray's chain of fetches
+// but gives the warp fewer rays, so the lines lie where a call stops being
+// bound by latency. Random rays in 1M triangles, device time with a group of
+// 32 / 16 / 8 / 4 / none:
+//   25,000 rays    80 /  66 /  67 /  91 / 159 us
+//   100,000         - /   - / 146 / 170 / 214 us
+//   400,000         - /   - /   - / 458 / 360 us
+unsigned cast_group_lanes(const DevScene& sc, int64_t n, int blocks)
 {
     const int64_t lanes = int64_t(blocks) * kBlock;
     for (unsigned G = 32u; G >= 4u; G /= 2u)
-        if (n * int64_t(G) <= lanes * rounds * (G == 4u ? 2 : 1))
-            return int(G) * kGroupEntries / 32 >= sc.depth + 2 * int(G) ? G : 0u;
+        if (n * int64_t(G) <= lanes * (G == 4u ? 8 : 4))
+            return group_fits(sc, G) ? G : 0u;
+    return 0u;
+}
+
+// The same for a frame of n rays. A tile's neighbouring rays share their
+// fetches in a full warp, so a frame gains by groups only while it is bound by
+// the latency of one warp's walk, which grows with the scene, and a group's
+// time grows with the rays that hit. The line is where frames whose rays all
+// hit (a terrain seen from above or in a wide strip) take as long either way;
+// it is lanes x (6 log2(triangles) - 39) / 40 rays x lanes. Groups above 4 only
+// within one ray per group at a time. Whole frames from above, device time with
+// a group of 32 / 16 / 8 / 4 / none:
+//   1,482 triangles, 160x90    74 /  45 /  36 /  32 /  34 us
+//                    320x180    - /   - /  73 /  45 /  33
+//   8,930            120x68    56 /  39 /  37 /  34 /  57
+//                    240x135    - /   - /  57 /  41 /  52
+//                    320x180    - /   - /   - /  56 /  49
+//   34,776           160x90    95 /  58 /  46 /  45 /  87
+//                    320x180    - /   - /  97 /  70 /  76
+//                    400x225    - /   - /   - /  92 /  74
+//   1M               160x90   113 /  70 /  59 /  68 / 278
+//                    400x225    - /   - / 184 / 141 / 228
+//                    520x290    - /   - /   - / 194 / 207
+// A strip of 603x150 pixels: 8,930 triangles 79 / 50 (4 / none), 34,776 94 / 63,
+// 260,610 121 / 105, 1M 142 / 174.
+unsigned frame_group_lanes(const DevScene& sc, int64_t n, int blocks)
+{
+    const int64_t lanes = int64_t(blocks) * kBlock;
+    int bits = 0;
+    while ((sc.numTris >> bits) > 1)
+        bits++;
+    const int64_t most = lanes * (6 * bits - 39) / 40;
+    for (unsigned G = 32u; G >= 4u; G /= 2u)
+        if (n * int64_t(G) <= (G == 4u ? most : std::min(most, lanes)))
+            return group_fits(sc, G) ? G : 0u;
     return 0u;
 }
 
@@ -675,7 +708,7 @@ cudaError_t cast_group(const LaunchInfo& li, const DevScene& sc, const rc_ray* r
     auto k = k_cast_group<ANY, ORDER>;
     static OccupancyCache occ;
     const int blocks = persistent_blocks(k, li.numSMs, occ);
-    const unsigned G = group_lanes(sc, n, blocks, 4);
+    const unsigned G = cast_group_lanes(sc, n, blocks);
     taken = G != 0u;
     if (!taken)
         return cudaSuccess;
@@ -857,7 +890,7 @@ cudaError_t raycast_group(const LaunchInfo& li, const DevScene& sc, const DevCam
     auto k = k_raycast_group<ORDER>;
     static OccupancyCache occ;
     const int blocks = persistent_blocks(k, li.numSMs, occ);
-    const unsigned G = group_lanes(sc, count, blocks, 2);
+    const unsigned G = frame_group_lanes(sc, count, blocks);
     taken = G != 0u;
     if (!taken)
         return cudaSuccess;
@@ -902,7 +935,7 @@ int64_t cast_wide_rays(const LaunchInfo& li, const DevScene& sc, int64_t n, int 
         return 0;
     static OccupancyCache occ;
     const int blocks = persistent_blocks(k_cast_group<false, ORDER_NEAREST>, li.numSMs, occ);
-    const int64_t line = int64_t(blocks) * kBlock * 2;  // most rays that groups of 4 lanes walk (group_lanes)
+    const int64_t line = int64_t(blocks) * kBlock * 2;  // most rays that groups of 4 lanes walk
     return std::max<int64_t>(0, n - line);
 }
 

@@ -407,7 +407,12 @@ __device__ __forceinline__ void wide_cswap(float& da, int& la, float& db, int& l
 // their entry distances, and pops skip entries beyond the current hit. The
 // leaves and their triangle tests are the binary tree's, and the accepted
 // hit (minimum t, ties to the larger slot) does not depend on the order, so
-// it is traverse<false, ORDER_NEAREST>'s. Rays whose inverse direction is not
+// it is traverse<false, ORDER_NEAREST>'s, but for overlapping coplanar
+// triangles where rounding puts hits before their boxes (see traverse_group):
+// casts walk such rays again, two-level bounces put them aside, and the paths
+// of one-level scenes keep this walk's hit (at 500x400, 475-7,495 pixels of
+// scenes made of such sheets differ from the counted render's film, none of
+// others). Rays whose inverse direction is not
 // finite can reach other boxes here than there (see wide_node_step) and walk
 // the binary tree. No node or triangle counts: counted frames use the binary
 // traversal.
@@ -474,7 +479,12 @@ __device__ __forceinline__ void WideWalk::abandon()
 }
 
 // How far past the current closest hit a walk goes that must meet every box
-// which could decide a tie (see traverse_group).
+// which could decide a tie (see traverse_group). A margin that was measured, not
+// a bound: over 16M rays at coplanar triangles (axis-aligned and tilted planes,
+// scales of 0.1-100 at offsets up to 1,000, origins from 1e-7 of the scale above
+// the plane on, grazing to 0.1 %) no hit lies more than 0.015 % before the entry
+// of its leaf. Axis-aligned planes subtract exactly; the box of a tilted
+// triangle is thick where its rounding is large.
 constexpr float kTieCull = 1.01f;
 
 // A walk whose hit is reported (rc_cast): it keeps the entry distance of the
@@ -869,7 +879,8 @@ struct PacketEntry
 //                  lanes find nearer; each lane culls boxes whose entry
 //                  distance lies beyond its own current hit. The accepted hit
 //                  (minimum t, ties to the larger slot) does not depend on
-//                  the order.
+//                  the order, but where rounding puts hits on overlapping
+//                  coplanar triangles before their boxes (see traverse_group).
 // It pays for coherent rays (the primary rays of a pixel tile); any-hit
 // shadow rays, which stop at different depths, ran slower this way than one
 // traversal per lane. Node and triangle counts are not kept: counted frames

@@ -8,10 +8,10 @@
 // same order), so a triangle test of the wide traversal is the binary
 // traversal's. A child box of the binary tree lies inside its parent's box
 // (also in float: both were rounded to nearest from nested boxes, or are
-// float unions), and the slab test is monotone in the box, so every ray that
-// reaches a grandchild through the binary tree reaches it through the wide
-// node too: the nearest-first closest hit, which does not depend on the
-// visiting order, is the same.
+// float unions), and the slab test is monotone in the box where it meets no
+// NaN, so every ray that reaches a grandchild through the binary tree reaches it
+// through the wide node too, and no other: the nearest-first closest hit is the
+// same (traverse.cuh says for which rays it is not, and what they do).
 //
 // One launch per level: thread i takes the i-th wide node of the level,
 // chooses its children and takes consecutive nodes of the next level for the
