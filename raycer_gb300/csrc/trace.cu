@@ -772,20 +772,24 @@ bool packet_frame(uint64_t pixelStart, int64_t count, int64_t width, int order)
     return order == ORDER_REF || whole_lines(pixelStart, count, width);
 }
 
-// The tiles of a frame walked by more than groups of lanes. Ranges walked one
-// ray per lane take them from four tiles per resident warp on: with fewer the
+// The tiles of a frame that groups of lanes do not walk. Ranges walked one ray
+// per lane take them from four tiles per resident warp on: with fewer the
 // longest tile's chain of walks is longer than the longest row's. In order ->
 // tiles, device time of ranges of 192k, 240k, 320k, 433k, 607k, 780k and 1.87M
 // pixels, 1M triangles: 115 / 125 / 125 / 145 / 191 / 265 / 470 -> 134 / 148 /
-// 133 / 157 / 192 / 228 / 387 us. Packets in reference order: 222 / 268 / 226 /
-// 294 / 535 / 737 / 1,310 -> 224 / 281 / 184 / 238 / 387 / 600 / 803. Two-level
+// 133 / 157 / 192 / 228 / 387 us. Packets in reference order, from one tile per
+// warp on: 78k / 90k / 138k pixels 302 / 313 / 323 -> 401 / 381 / 366 us, the
+// others 222 / 268 / 226 / 294 / 535 / 737 / 1,310 -> 224 / 281 / 184 / 238 / 387
+// / 600 / 803. Two-level
 // scenes gain at all sizes but one: 1M + 200 blobs of 20,480 triangles, 60k, 192k,
 // 240k, 320k, 433k, 607k and 1.87M pixels 613 / 416 / 541 / 423 / 648 / 866 /
 // 2,092 -> 525 / 403 / 602 / 359 / 570 / 780 / 1,646.
 FilmTiles walk_tiles(const LaunchInfo& li, const rc_ray* rays, uint64_t pixelStart, int64_t count, int64_t width,
                      int order, bool instanced)
 {
-    if (!instanced && width > 0 && !packet_frame(pixelStart, count, width, order) && count < int64_t(li.numSMs) * 4 * 32 * 32)
+    const int64_t warps = int64_t(li.numSMs) * 32;
+    if (!instanced && width > 0 && !whole_lines(pixelStart, count, width) &&
+        count < warps * 32 * (order == ORDER_REF ? 1 : 4))
         return FilmTiles{};
     return frame_tiles(rays, pixelStart, count, width);
 }
@@ -1009,7 +1013,7 @@ cudaError_t launch_raycast(const LaunchInfo& li, const DevScene& sc, const DevCa
         }
     }
     const int packets = trace_packets();
-    const bool packet = frame_tiles(rays, pixelStart, count, width).columns > 0 &&
+    const bool packet = walk_tiles(li, rays, pixelStart, count, width, order, false).columns > 0 &&
                         packet_frame(pixelStart, count, width, order) && (packets == 2 || (packets == 1 && !rays));
     if (stackless_walk() && sc.ropes)
     {
