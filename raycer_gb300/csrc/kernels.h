@@ -97,8 +97,17 @@ int blocks_per_sm(K kernel, int block, size_t smem, OccupancyCache& cache)
 // use while this is on).
 bool stackless_walk();
 
+// log2 of the scene's triangles, rounded down.
+inline int scene_bits(const DevScene& sc)
+{
+    int bits = 0;
+    while ((sc.numTris >> bits) > 1)
+        bits++;
+    return bits;
+}
+
 // Rays of this launch_cast that the scene's 4-wide tree, where there is one,
-// makes cheaper: those above the line up to which groups of lanes walk a ray.
+// makes cheaper: those above the line from which on casts walk it.
 int64_t cast_wide_rays(const LaunchInfo& li, const DevScene& sc, int64_t n, int anyHit, int order);
 
 // Generic ray queries (rc_ray -> rc_hit).

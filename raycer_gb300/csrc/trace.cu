@@ -639,20 +639,57 @@ int persistent_blocks(K kernel, int numSMs, OccupancyCache& cache)
 bool group_fits(const DevScene& sc, unsigned G) { return int(G) * kGroupEntries / 32 >= sc.depth + 2 * int(G); }
 
 // Lanes per ray of an uncounted cast of n rays on a single-level scene, or 0
-// for one ray per lane: the largest group (32, 16, 8, 4) whose four rounds of
-// one ray per group cover the rays (eight for groups of 4, whose alternative
-// is one ray per lane). Each larger group shortens a ray's chain of fetches
-// but gives the warp fewer rays, so the lines lie where a call stops being
-// bound by latency. Random rays in 1M triangles, device time with a group of
-// 32 / 16 / 8 / 4 / none:
-//   25,000 rays    80 /  66 /  67 /  91 / 159 us
-//   100,000         - /   - / 146 / 170 / 214 us
-//   400,000         - /   - /   - / 458 / 360 us
+// for one ray per lane. Each larger group shortens a ray's chain of fetches but
+// gives the warp fewer rays, so a group wins where a call is bound by latency,
+// which grows with the scene: n x G may be `most` lanes for groups of 32, 16
+// and 8, and `most4` for groups of 4. The lines lie where random rays and rays
+// of a frame from above, whichever is earlier, take as long one ray per lane.
+// Device time with a group of 32 / 16 / 8 / 4 / none, nearest-first:
+//   1,482 triangles  10,000 random   34 /  27 /  26 /  30 /  49 us
+//                    10,000 frame    37 /  26 /  22 /  21 /  27
+//                    40,000 frame     - /   - /  37 /  27 /  26
+//   8,930            40,000 random    - /   - /  51 /  45 /  57
+//                    80,000 frame     - /   - /  66 /  45 /  42
+//   1M               20,000 random   68 /  53 /  47 /  57 /  76
+//                    80,000 random    - /   - / 105 / 102 /  97
+//                   120,000 frame     - /   - / 148 / 112 / 113
+// any hit:
+//   8,930            40,000 random    - /   - /  54 /  57 /  64
+//   1M               40,000 random    - /  86 /  89 / 103 /  88
+//                    40,000 frame     - /  79 /  72 /  96 / 119
+// reference order:
+//   8,930            80,000 frame     - /   - /  61 /  44 /  46
+//   70,668          160,000 frame     - /   - /   - /  95 / 117
+//                   148,200 strip     - /   - /   - /  93 /  84
+//   1M              311,000 random    - /   - /   - / 402 / 499
+template <bool ANY, int ORDER>
 unsigned cast_group_lanes(const DevScene& sc, int64_t n, int blocks)
 {
     const int64_t lanes = int64_t(blocks) * kBlock;
+    const int bits = scene_bits(sc);
+    int64_t most, most4;
+    if (bits < 13)
+    {
+        most = lanes / 2;
+        most4 = bits < 10 ? lanes * 2 / 3 : lanes;
+    }
+    else if (ANY)
+    {
+        most = lanes * 2;
+        most4 = 0;
+    }
+    else if (ORDER == ORDER_NEAREST)
+    {
+        most = lanes;
+        most4 = lanes * 7 / 4;
+    }
+    else
+    {
+        most = lanes * 2;
+        most4 = bits < 16 ? lanes * 2 : bits < 17 ? lanes * 3 : lanes * 8;
+    }
     for (unsigned G = 32u; G >= 4u; G /= 2u)
-        if (n * int64_t(G) <= lanes * (G == 4u ? 8 : 4))
+        if (n * int64_t(G) <= (G == 4u ? most4 : most))
             return group_fits(sc, G) ? G : 0u;
     return 0u;
 }
@@ -681,10 +718,7 @@ unsigned cast_group_lanes(const DevScene& sc, int64_t n, int blocks)
 unsigned frame_group_lanes(const DevScene& sc, int64_t n, int blocks)
 {
     const int64_t lanes = int64_t(blocks) * kBlock;
-    int bits = 0;
-    while ((sc.numTris >> bits) > 1)
-        bits++;
-    const int64_t most = lanes * (6 * bits - 39) / 40;
+    const int64_t most = lanes * (6 * scene_bits(sc) - 39) / 40;
     for (unsigned G = 32u; G >= 4u; G /= 2u)
         if (n * int64_t(G) <= (G == 4u ? most : std::min(most, lanes)))
             return group_fits(sc, G) ? G : 0u;
@@ -708,7 +742,7 @@ cudaError_t cast_group(const LaunchInfo& li, const DevScene& sc, const rc_ray* r
     auto k = k_cast_group<ANY, ORDER>;
     static OccupancyCache occ;
     const int blocks = persistent_blocks(k, li.numSMs, occ);
-    const unsigned G = cast_group_lanes(sc, n, blocks);
+    const unsigned G = cast_group_lanes<ANY, ORDER>(sc, n, blocks);
     taken = G != 0u;
     if (!taken)
         return cudaSuccess;
@@ -933,14 +967,20 @@ bool stackless_walk()
     return on;
 }
 
+namespace
+{
+
+// Rays from which on nearest-first casts walk the 4-wide tree in phases: two
+// per lane of 32 resident warps per SM.
+int64_t phased_line(const LaunchInfo& li) { return int64_t(li.numSMs) * 32 * 32 * 2; }
+
+}  // namespace
+
 int64_t cast_wide_rays(const LaunchInfo& li, const DevScene& sc, int64_t n, int anyHit, int order)
 {
     if (anyHit || order != ORDER_NEAREST || li.counting || sc.numInstances > 0 || (sc.ropes && stackless_walk()))
         return 0;
-    static OccupancyCache occ;
-    const int blocks = persistent_blocks(k_cast_group<false, ORDER_NEAREST>, li.numSMs, occ);
-    const int64_t line = int64_t(blocks) * kBlock * 2;  // most rays that groups of 4 lanes walk
-    return std::max<int64_t>(0, n - line);
+    return std::max<int64_t>(0, n - phased_line(li));
 }
 
 cudaError_t launch_cast(const LaunchInfo& li, const DevScene& sc, const rc_ray* rays, int64_t n, int anyHit,
@@ -958,11 +998,11 @@ cudaError_t launch_cast(const LaunchInfo& li, const DevScene& sc, const rc_ray* 
                                      : cast_group<false, ORDER_REF>(li, sc, rays, n, hits, ctl, taken);
         if (taken)
             return e;
-        if (anyHit)
+        if (anyHit && scene_bits(sc) >= 13)
             return cast_phased<true, ORDER_REF>(li, sc, rays, n, hits, ctl);
-        if (order == ORDER_REF)
+        if (!anyHit && order == ORDER_REF)
             return cast_phased<false, ORDER_REF>(li, sc, rays, n, hits, ctl);
-        if (sc.wide)
+        if (!anyHit && sc.wide && n > phased_line(li))
             return cast_phased<false, ORDER_NEAREST>(li, sc, rays, n, hits, ctl);
     }
     if (anyHit)

@@ -159,7 +159,7 @@ rc_status ensure_wide_instanced(rc_tracer* h)
     return s;
 }
 
-// Rays above the group line (cast_wide_rays) after which a scene's casts build
+// Rays above the line for the 4-wide walk (cast_wide_rays) after which a scene's casts build
 // its tree: what they gain by it then makes up for the construction. Measured
 // with random rays (construction; k_cast -> k_cast_phased with 4M rays; rays
 // for which the gain is the construction):

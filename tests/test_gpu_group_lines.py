@@ -10,7 +10,7 @@ import pytest
 import oracle
 from raycer_gb300 import _native as N
 from raycer_gb300 import scenes
-from raycer_gb300.tracer import CudaTracer, TracerState, camera_record
+from raycer_gb300.tracer import RAY_DTYPE, CudaTracer, TracerState, camera_record
 
 from helpers import camera_floats
 
@@ -39,3 +39,24 @@ def test_frames(nx, nz, share, order):
         cam = camera_floats(camera_record(sc))
     ref, _ = oracle.Oracle(sc).raycast32(cam, width, n, -np.array(sc.light_direction, np.float32), order=order)
     assert np.array_equal(got, ref), f"{(got != ref).any(axis=1).sum()} pixels differ"
+
+
+@pytest.mark.parametrize("nx,nz", [(2, 2), (12, 8), (30, 26), (96, 48), (150, 120), (300, 151)])
+@pytest.mark.parametrize("n", [1, 2_400, 2_500, 9_700, 9_800, 25_900, 26_000, 38_900, 39_000, 68_000, 68_200, 77_900, 155_700])
+def test_casts(nx, nz, n):
+    sc = scenes.heightfield_scene(nx=nx, nz=nz)
+    rng = np.random.default_rng(n)
+    v = sc.vertices.reshape(-1, 3)
+    rays = np.zeros(n, RAY_DTYPE)
+    rays["origin"] = rng.uniform(v.min(0) - 0.1, v.max(0) + 0.1, size=(n, 3))
+    rays["direction"] = rng.normal(size=(n, 3))
+    rays["t_max"] = np.where(rng.random(n) < 0.5, np.float32(3.0e38), np.float32(2.0))
+    orc = oracle.Oracle(sc)
+    with CudaTracer(0) as t:
+        t.initializeBuffers(sc)
+        for any_hit, order in ((False, N.RC_ORDER_NEAREST), (False, N.RC_ORDER_REFERENCE), (True, N.RC_ORDER_NEAREST)):
+            hits = t.cast(rays, any_hit=any_hit, order=order)
+            prim, tt, u, v_, _ = orc.cast32(rays, any_hit=any_hit, order=order)
+            assert np.array_equal(hits["prim"], prim)
+            for k, ref in (("t", tt), ("u", u), ("v", v_)):
+                assert np.array_equal(hits[k], ref, equal_nan=True)
