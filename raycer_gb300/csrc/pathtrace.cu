@@ -1696,21 +1696,35 @@ bool one_kernel_pass(int order, int counting)
 
 bool fused_pass(const PassParams& p, int order, int counting) { return one_kernel_pass(order, counting) && p.wide; }
 
-// Lanes per path of a one-scene pass, or 0 for one path per lane: the largest
-// group whose two rounds of one path per group (four for groups of 4) cover
-// the pass. Measured on the room above (group of 32 / 16 / 8 / 4 / none):
-// 128x96 169 / 126 / 137 / - / 308 us, 192x144 309 / 208 / 181 / 216 / 360,
-// 320x240 - / - / 363 / 342 / 473, 480x360 - / - / - / 641 / 585. A tree too
-// deep for the group's stack is walked one path per lane.
+// Lanes per path of a one-scene pass, or 0 for one path per lane. As for casts
+// and frames (trace.cu), a group wins where the pass is bound by the latency of
+// its walks, which grows with the scene; the lines lie where passes whose camera
+// rays all hit (a terrain seen from above) take as long either way. Device time
+// of one path per pixel with a group of 32 / 16 / 8 / 4 / none:
+//   1,482 triangles, depth 1  8,160     56 /  49 /  43 /  44 /  41 us
+//                    depth 2  8,160     87 /  70 /  71 /  70 /  81
+//                            44,240      - /   - / 116 /  92 /  87
+//   8,930            depth 1 32,400      - /   - /  62 /  54 /  54
+//                    depth 4 44,240      - /   - / 181 / 160 / 162
+//   70,668           depth 4 57,600      - /   - / 281 / 251 / 253
+//   1M               depth 4  8,160    155 / 132 / 142 / 190 / 219
+//                            57,600      - /   - / 336 / 310 / 310
+//   room of 2,012    depth 4  8,160    123 / 101 / 118 / 168 / 279
+//                            57,600      - /   - / 294 / 290 / 421
+// A tree too deep for the group's stack is walked one path per lane.
 unsigned path_group_lanes(const PassParams& p, int order, int counting, int numSMs)
 {
-    constexpr int rounds = 2;
     if (!p.singleScene || p.instanced || !one_kernel_pass(order, counting) || p.segments < 1 || p.scene0.rootLink < 0)
         return 0u;
     static OccupancyCache occ;
     const int64_t lanes = int64_t(persistent_blocks(k_path_group<true>, 128, numSMs, occ)) * 128;
+    const int bits = scene_bits(p.scene0);
+    if (bits < 13 && p.segments == 1)
+        return 0u;
+    const int64_t most = bits < 13 ? lanes / 2 : lanes;
+    const int64_t most4 = bits >= 15 ? lanes * 4 / 3 : p.segments > 1 ? lanes : lanes * 2 / 3;
     for (unsigned G = 32u; G >= 4u; G /= 2u)
-        if (int64_t(p.nslots) * int64_t(G) <= lanes * rounds * (G == 4u ? 2 : 1))
+        if (int64_t(p.nslots) * int64_t(G) <= (G == 4u ? most4 : most))
             return int(G) * kGroupEntries / 32 >= p.scene0.depth + 2 * int(G) ? G : 0u;
     return 0u;
 }

@@ -60,3 +60,21 @@ def test_casts(nx, nz, n):
             assert np.array_equal(hits["prim"], prim)
             for k, ref in (("t", tt), ("u", u), ("v", v_)):
                 assert np.array_equal(hits[k], ref, equal_nan=True)
+
+
+@pytest.mark.parametrize("nx,nz", [(12, 8), (96, 48), (240, 120)])
+@pytest.mark.parametrize("share", [0.015, 0.06, 0.12, 0.24, 0.26, 0.66, 0.68, 0.97, 1.03, 1.32, 1.35])
+@pytest.mark.parametrize("depth", [1, 3])
+def test_passes(nx, nz, share, depth):
+    width = 211
+    height = max(2, int(share * LANES) // width)
+    sc = scenes.heightfield_path_scene(nx=nx, nz=nz, width=width, height=height, max_path_length=depth)
+    n = width * height
+    with CudaTracer(0) as t:
+        t.initializeBuffers(sc, seed=21)
+        t.initializeImageBuffers(width, height)
+        t.run(TracerState(scene=sc, filmWidth=width, filmHeight=height, pixelCount=n))
+        film = t.read_film()
+        cam = camera_floats(camera_record(sc))
+    ref, _ = oracle.Oracle(sc).render_path32(cam, width, n, 1, 1, 4, (0.5, 0.5), 1e-5, depth, 0, 1, 21, 0)
+    assert np.array_equal(film, ref), f"{(film != ref).any(axis=1).sum()} pixels differ"
