@@ -99,10 +99,30 @@ __device__ __forceinline__ int caller_index(const DevScene& sc, int slot)
     return __float_as_int(__ldg(&sc.tris[slot].c.z));
 }
 
+// Large casts are launched twice, straight (k_cast) and in phases
+// (k_cast_phased), and the samples of k_cast_samples decide on the device which
+// of the two does the work: `run` is the answer a kernel waits for, or kAnyRays.
+enum CastRun
+{
+    kApart = 0,
+    kTogether = 1,
+    kAnyRays = 2
+};
+constexpr int kCastSamples = 32;
+
+__device__ __forceinline__ bool cast_runs(const DevControl* ctl, int run)
+{
+    return run == kAnyRays ||
+           run == (*reinterpret_cast<const volatile unsigned*>(&ctl->head[1]) * 2u >= unsigned(kCastSamples) ? kTogether
+                                                                                                          : kApart);
+}
+
 template <bool ANY, int ORDER, bool COUNT, bool SL>
 __global__ void __launch_bounds__(kBlock, RC_TRACE_MIN_BLOCKS) k_cast(DevScene sc, const rc_ray* __restrict__ rays, int n,
-                                                 rc_hit* __restrict__ hits, DevControl* ctl)
+                                                 rc_hit* __restrict__ hits, DevControl* ctl, int run)
 {
+    if (!cast_runs(ctl, run))
+        return;
     TravCount cnt{ 0, 0 };
     int err = 0;
     unsigned long long done = 0;
@@ -420,10 +440,38 @@ __device__ __forceinline__ void write_hit(const DevScene& sc, const HitF& h, rc_
         make_int4(found ? caller_index(sc, h.slot) : -1, __float_as_int(found ? h.t : -1.0f),
                   __float_as_int(found ? h.u : 0.0f), __float_as_int(found ? h.v : 0.0f));
 }
+
+// How many of 32 samples of 32 consecutive rays, spread over the batch, would
+// walk together: directions within `spread` of the first one's (of its largest
+// component), origins within a 32nd of the scene. Camera rays in the order of a
+// frame do. One block.
+__global__ void __launch_bounds__(kCastSamples * 32) k_cast_samples(DevScene sc, const rc_ray* __restrict__ rays, int n,
+                                                                    float spread, DevControl* ctl)
+{
+    constexpr unsigned kAll = 0xffffffffu;
+    const int64_t last = n / 32 - 1;  // of the batch's whole groups of 32
+    const int64_t group = last * int64_t(threadIdx.x >> 5) / (kCastSamples - 1);
+    const RayF r = load_ray(rays + group * 32 + lane_id());
+    float4 a, b, c;
+    int4 l;
+    load_node(sc.nodes, sc.rootLink, a, b, c, l);
+    const float extent = fmaxf(fmaxf(fmaxf(a.y, b.y) - fminf(a.x, b.x), fmaxf(a.w, b.w) - fminf(a.z, b.z)),
+                               fmaxf(c.y, c.w) - fminf(c.x, c.z));
+    const V3 o = v3(__shfl_sync(kAll, r.o.x, 0), __shfl_sync(kAll, r.o.y, 0), __shfl_sync(kAll, r.o.z, 0));
+    const V3 d = v3(__shfl_sync(kAll, r.d.x, 0), __shfl_sync(kAll, r.d.y, 0), __shfl_sync(kAll, r.d.z, 0));
+    const float away = fmaxf(fmaxf(fabsf(r.o.x - o.x), fabsf(r.o.y - o.y)), fabsf(r.o.z - o.z));
+    const float turn = fmaxf(fmaxf(fabsf(r.d.x - d.x), fabsf(r.d.y - d.y)), fabsf(r.d.z - d.z));
+    const float size = fmaxf(fmaxf(fabsf(d.x), fabsf(d.y)), fabsf(d.z));
+    if (__all_sync(kAll, away <= extent * (1.0f / 32.0f) && turn <= spread * size) && lane_id() == 0)
+        atomicAdd(&ctl->head[1], 1u);
+}
+
 template <bool ANY, int ORDER>
 __global__ void __launch_bounds__(kBlock, 8) k_cast_phased(DevScene sc, const rc_ray* __restrict__ rays, int n,
-                                                           rc_hit* __restrict__ hits, DevControl* ctl)
+                                                           rc_hit* __restrict__ hits, DevControl* ctl, int run)
 {
+    if (!cast_runs(ctl, run))
+        return;
     constexpr unsigned kAll = 0xffffffffu;
     constexpr bool WIDE = !ANY && ORDER == ORDER_NEAREST;
     constexpr int kNear = WIDE ? 12 : 16;  // stack entries in shared memory
@@ -727,11 +775,11 @@ unsigned frame_group_lanes(const DevScene& sc, int64_t n, int blocks)
 
 template <bool ANY, int ORDER>
 cudaError_t cast_phased(const LaunchInfo& li, const DevScene& sc, const rc_ray* rays, int64_t n, rc_hit* hits,
-                        DevControl* ctl)
+                        DevControl* ctl, int run = kAnyRays)
 {
     auto k = k_cast_phased<ANY, ORDER>;
     static OccupancyCache occ;
-    k<<<persistent_blocks(k, li.numSMs, occ), kBlock, 0, li.stream>>>(sc, rays, int(n), hits, ctl);
+    k<<<persistent_blocks(k, li.numSMs, occ), kBlock, 0, li.stream>>>(sc, rays, int(n), hits, ctl, run);
     return cudaGetLastError();
 }
 
@@ -752,12 +800,34 @@ cudaError_t cast_group(const LaunchInfo& li, const DevScene& sc, const rc_ray* r
 
 template <bool ANY, int ORDER, bool COUNT, bool SL = false>
 cudaError_t cast_t(const LaunchInfo& li, const DevScene& sc, const rc_ray* rays, int64_t n, rc_hit* hits,
-                   DevControl* ctl)
+                   DevControl* ctl, int run = kAnyRays)
 {
     auto k = k_cast<ANY, ORDER, COUNT, SL>;
     static OccupancyCache occ;
-    k<<<persistent_blocks(k, li.numSMs, occ), kBlock, 0, li.stream>>>(sc, rays, int(n), hits, ctl);
+    k<<<persistent_blocks(k, li.numSMs, occ), kBlock, 0, li.stream>>>(sc, rays, int(n), hits, ctl, run);
     return cudaGetLastError();
+}
+
+// A large cast: straight where its rays walk together, else in phases. In
+// phases warps lose the coherence that camera rays have, and random rays gain
+// lanes: straight -> phases, 4M rays, 8,930 triangles: a frame's rays 240 ->
+// 357 us (nearest-first), 214 -> 305 (any hit), 305 -> 393 (reference order),
+// random rays 891 -> 709, 853 -> 616, 2,044 -> 1,016; 1M triangles: 667 -> 885,
+// 628 -> 761, 1,160 -> 1,203, and 1,436 -> 1,045, 1,322 -> 901, 4,516 -> 2,086.
+// The spreads are about those of 32 pixels of a row at the sizes where a frame's
+// rays take as long either way (400k-600k pixels; 1M in reference order).
+template <bool ANY, int ORDER>
+cudaError_t cast_large(const LaunchInfo& li, const DevScene& sc, const rc_ray* rays, int64_t n, rc_hit* hits,
+                       DevControl* ctl)
+{
+    if (sc.rootLink < 0)
+        return cast_phased<ANY, ORDER>(li, sc, rays, n, hits, ctl);
+    constexpr float spread = !ANY && ORDER == ORDER_REF ? 1.0f / 40.0f : 1.0f / 24.0f;
+    k_cast_samples<<<1, kCastSamples * 32, 0, li.stream>>>(sc, rays, int(n), spread, ctl);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess)
+        e = cast_t<ANY, ORDER, false>(li, sc, rays, n, hits, ctl, kTogether);
+    return e == cudaSuccess ? cast_phased<ANY, ORDER>(li, sc, rays, n, hits, ctl, kApart) : e;
 }
 
 // Warp-wide traversal of the primary rays of uncounted RAY frames walked in
@@ -970,9 +1040,16 @@ bool stackless_walk()
 namespace
 {
 
-// Rays from which on nearest-first casts walk the 4-wide tree in phases: two
-// per lane of 32 resident warps per SM.
-int64_t phased_line(const LaunchInfo& li) { return int64_t(li.numSMs) * 32 * 32 * 2; }
+// Rays above which a cast looks at its rays first (cast_large), and nearest-first
+// casts walk the 4-wide tree: four per lane of 32 resident warps per SM, eight
+// for scenes below 2^15 triangles and in reference order. Below, the gain of
+// phases is within what looking costs (10 us for two more launches), or what a
+// frame's rays would lose: 400k of them from above, 8,930 triangles: 57 -> 66 us
+// nearest-first, 59 -> 66 any hit (from 2^15 triangles on 89 -> 89).
+int64_t large_line(const LaunchInfo& li, const DevScene& sc, bool reference)
+{
+    return int64_t(li.numSMs) * 32 * 32 * (reference || scene_bits(sc) < 15 ? 8 : 4);
+}
 
 }  // namespace
 
@@ -980,7 +1057,7 @@ int64_t cast_wide_rays(const LaunchInfo& li, const DevScene& sc, int64_t n, int 
 {
     if (anyHit || order != ORDER_NEAREST || li.counting || sc.numInstances > 0 || (sc.ropes && stackless_walk()))
         return 0;
-    return std::max<int64_t>(0, n - phased_line(li));
+    return std::max<int64_t>(0, n - large_line(li, sc, false));
 }
 
 cudaError_t launch_cast(const LaunchInfo& li, const DevScene& sc, const rc_ray* rays, int64_t n, int anyHit,
@@ -998,12 +1075,15 @@ cudaError_t launch_cast(const LaunchInfo& li, const DevScene& sc, const rc_ray* 
                                      : cast_group<false, ORDER_REF>(li, sc, rays, n, hits, ctl, taken);
         if (taken)
             return e;
-        if (anyHit && scene_bits(sc) >= 13)
-            return cast_phased<true, ORDER_REF>(li, sc, rays, n, hits, ctl);
+        const bool large = n > large_line(li, sc, !anyHit && order == ORDER_REF);
+        if (anyHit && (large || scene_bits(sc) >= 15))
+            return large ? cast_large<true, ORDER_REF>(li, sc, rays, n, hits, ctl)
+                         : cast_phased<true, ORDER_REF>(li, sc, rays, n, hits, ctl);
         if (!anyHit && order == ORDER_REF)
-            return cast_phased<false, ORDER_REF>(li, sc, rays, n, hits, ctl);
-        if (!anyHit && sc.wide && n > phased_line(li))
-            return cast_phased<false, ORDER_NEAREST>(li, sc, rays, n, hits, ctl);
+            return large ? cast_large<false, ORDER_REF>(li, sc, rays, n, hits, ctl)
+                         : cast_phased<false, ORDER_REF>(li, sc, rays, n, hits, ctl);
+        if (!anyHit && sc.wide && large)
+            return cast_large<false, ORDER_NEAREST>(li, sc, rays, n, hits, ctl);
     }
     if (anyHit)
         return li.counting ? cast_t<true, ORDER_REF, true>(li, sc, rays, n, hits, ctl)

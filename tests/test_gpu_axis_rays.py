@@ -40,7 +40,7 @@ def _compare(sc, rays, order, any_hit=False):
     return prim
 
 
-@pytest.mark.parametrize("n", [777, 32_768, 400_000])
+@pytest.mark.parametrize("n", [777, 32_768, 400_000, 1_300_000])
 @pytest.mark.parametrize("direction", [(0.0, -1.0, 0.0), (-0.0, -1.0, -0.0), (0.0, 1.0, 0.0), (0.0, -1.0, 0.3)])
 @pytest.mark.parametrize("order", ORDERS)
 def test_rays_at_grid_vertices(n, direction, order):
@@ -71,7 +71,7 @@ def _cubes(leaf):
                             scenes.CameraDesc(position=(0.0, 0.0, 4.0), fov=50.0), 64, 48, max_leaf_size=leaf)
 
 
-@pytest.mark.parametrize("n", [5_000, 100_000, 400_000])
+@pytest.mark.parametrize("n", [5_000, 100_000, 400_000, 1_300_000])
 @pytest.mark.parametrize("leaf", [1, 4])
 @pytest.mark.parametrize("order,any_hit", [(N.RC_ORDER_REFERENCE, False), (N.RC_ORDER_NEAREST, False),
                                            (N.RC_ORDER_NEAREST, True)])
@@ -89,7 +89,7 @@ def test_axis_rays_among_cubes(n, leaf, order, any_hit):
 @pytest.mark.parametrize("order,any_hit", [(N.RC_ORDER_REFERENCE, False), (N.RC_ORDER_NEAREST, False),
                                            (N.RC_ORDER_NEAREST, True)])
 def test_many_edge_rays(order, any_hit):
-    rays = np.resize(_edge_rays(), 400_000)
+    rays = np.resize(_edge_rays(), 1_300_000)
     _compare(small_room(clutter=500), rays, order, any_hit)
 
 

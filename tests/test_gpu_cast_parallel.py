@@ -33,7 +33,7 @@ def _sheet():
 def test_parallel_rays_onto_a_sheet(height, spread):
     sc = _sheet()
     rng = np.random.default_rng(17)
-    n = 350_000
+    n = 1_300_000
     rays = np.zeros(n, RAY_DTYPE)
     d = np.array((0.05, 0.02, -1.0)) + spread * rng.normal(size=(n, 3))
     rays["direction"] = d / np.linalg.norm(d, axis=1, keepdims=True)

@@ -15,9 +15,9 @@ import pytest
 
 import oracle
 from raycer_gb300 import _native as N
-from raycer_gb300.tracer import RAY_DTYPE, CudaTracer
+from raycer_gb300.tracer import RAY_DTYPE, CudaTracer, camera_record
 
-from helpers import small_heightfield, small_room
+from helpers import camera_floats, small_heightfield, small_room
 from test_gpu_degenerate import scene as degenerate_scene
 from test_gpu_ray_groups import _rays
 
@@ -34,12 +34,13 @@ def grow_tree(t):
     t.cast(rays, any_hit=True)  # the call's buffers
     before = t.stats()["device_bytes"]
     t.cast(rays)
+    t.cast(rays)
     return t.stats()["device_bytes"] - before
 
 
 def test_casts_build_the_tree_once_they_pay_for_it():
     sc = small_heightfield()
-    rays = _rays(1_500_000, 3)
+    rays = _rays(2_100_000, 3)
     with CudaTracer(0) as t:
         for _ in range(2):  # the second upload starts anew
             t.initializeBuffers(sc)
@@ -47,18 +48,18 @@ def test_casts_build_the_tree_once_they_pay_for_it():
             before = t.stats()["device_bytes"]
             grown = []
             first = t.cast(rays)
-            for _ in range(3):
+            for _ in range(4):
                 grown.append(t.stats()["device_bytes"] - before)
                 assert np.array_equal(t.cast(rays), first)
             t.cast(rays[:300_000])
             t.cast(rays, order=N.RC_ORDER_REFERENCE)
-            assert grown[0] == grown[1] == 0 and grown[2] > 0
-            assert grown[2] == t.stats()["device_bytes"] - before
+            assert grown[0] == grown[1] == grown[2] == 0 and grown[3] > 0
+            assert grown[3] == t.stats()["device_bytes"] - before
         t.initializeBuffers(sc)
-        assert grow_tree(t) == grown[2]
+        assert grow_tree(t) == grown[3]
 
 
-@pytest.mark.parametrize("n", [311_299, 311_400, 400_000])
+@pytest.mark.parametrize("n", [1_245_184, 1_245_185, 1_300_000])
 @pytest.mark.parametrize("name", ["room", "terrain", "coplanar", "duplicates"])
 def test_casts_through_the_tree(name, n):
     sc = {"room": lambda: small_room(clutter=1000), "terrain": small_heightfield,
@@ -72,6 +73,29 @@ def test_casts_through_the_tree(name, n):
     assert np.array_equal(hits["prim"], prim)
     for k, ref in (("t", tt), ("u", u), ("v", v)):
         assert np.array_equal(hits[k], ref)
+
+
+@pytest.mark.parametrize("frame", [1.0, 0.55, 0.45])
+def test_large_casts_of_a_frames_rays(frame):
+    """Rays that walk together, and batches of which about half do."""
+    width, height = 1400, 1000
+    sc = small_heightfield(width=width, height=height)
+    n = width * height
+    rays = _rays(n, 9)
+    cam = np.ascontiguousarray(oracle.camera_rays32(camera_floats(camera_record(sc)), width, n))
+    first = int(frame * n)
+    rays[:first] = cam.view(rays.dtype).reshape(-1)[:first]
+    orc = oracle.Oracle(sc)
+    with CudaTracer(0) as t:
+        t.initializeBuffers(sc)
+        assert grow_tree(t) > 0
+        for any_hit, order in ((False, N.RC_ORDER_NEAREST), (False, N.RC_ORDER_REFERENCE), (True, N.RC_ORDER_NEAREST)):
+            hits = t.cast(rays, any_hit=any_hit, order=order)
+            prim, tt, u, v, _ = orc.cast32(rays, any_hit=any_hit, order=order)
+            assert np.array_equal(hits["prim"], prim)
+            for k, ref in (("t", tt), ("u", u), ("v", v)):
+                assert np.array_equal(hits[k], ref)
+            assert t.stats()["rays_traced"] == n
 
 
 _STACKLESS = """
