@@ -1105,7 +1105,7 @@ __global__ void __launch_bounds__(BLOCK,
 // traverse_instanced, held a warp in step instance by instance: a segment's
 // launch took 600 us however few paths it had. 1080p, heightfield + 200
 // blobs of 20,480 triangles, 30 % glass, depth 12: 11.1 -> 5.8 ms of device
-// time. Bound by ALU (58 %) and issue (63 %) at 14.6 lanes per instruction.
+// time (2 % more since hits that a walk's order decides are put aside). Bound by ALU (58 %) and issue (63 %) at 14.6 lanes per instruction.
 // The camera rays stay with k_extend_instanced and k_shade, whose coherent
 // warps lose nothing to the nesting (1.10 ms; 1.34 in phases). 6, 7 and 8
 // blocks per SM: 6.10 / 5.85 / 6.37 (72 registers; 8 blocks spill).
